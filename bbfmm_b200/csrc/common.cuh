@@ -106,6 +106,13 @@ struct Tables {
   const double *tkz_d, *cw_d, *kw_d;
   const float *tkz_f, *cw_f, *kw_f;
 };
+// Leaves above `cap` particles of a pass's rows (device lists, launch_heavy): P2M and L2P run one
+// warp per leaf, and these as chunks of at most cap particles, one warp each.
+struct HeavyLeaves {
+  int cap = 0x7fffffff, nitems = 0, nheavy = 0;
+  int4 *items = nullptr, *heavy = nullptr;  // (row, p0, p1, cell); (row, first item, items, cell)
+  void *part = nullptr;                     // nitems x n^3 partial P2M sums
+};
 // Row remapping of the projection GEMMs between Morton and cpg order.
 enum { MAP_NONE = 0, MAP_IN_CPG = 1, MAP_OUT_CPG = 2 };
 }  // namespace bbfmm

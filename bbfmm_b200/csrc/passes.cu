@@ -19,28 +19,9 @@ namespace bbfmm {
 int launch_m2m_dmma(const double *Sc, double *Sp, const double *cw, int64_t first, int64_t count, cudaStream_t s);
 int launch_l2l_dmma(const double *Fp, double *Fc, const double *cw, int64_t first, int64_t count, cudaStream_t s);
 
-// Lane t < 3 NN of a warp: S(x_m, c) for axis t / NN (c = x, y, z) and node m = t % NN by
-// the Clenshaw recurrence of ComputeSn2 (bbfmm.c:1682-1690), S = 1/2 T_0(x_m) + sum_k
-// T_k(x_m) T_k(c) with Tkz[m n + k] = T_k(x_m); other lanes return 0. The warp shares the
-// 3 NN values by shuffles instead of every lane evaluating all of them.
-template <typename T, int NN>
-__device__ __forceinline__ T sn_lane(const T *__restrict__ tkz, int lane, T x, T y, T z) {
-  if (lane >= 3 * NN) return (T)0;
-  const int a = lane / NN, m = lane % NN;
-  const T c = a == 0 ? x : (a == 1 ? y : z);
-  T d1 = 0, d2 = 0;
-#pragma unroll
-  for (int j = NN - 1; j > 0; --j) {
-    const T d0 = 2 * c * d1 - d2 + tkz[m * NN + j];
-    d2 = d1;
-    d1 = d0;
-  }
-  return c * d1 - d2 + (T)0.5 * tkz[m * NN];
-}
-
-// S(x_m, c) for axis idx / NN (c = x, y, z) and node m = idx % NN, idx < 3 NN: the value
-// lane idx of sn_lane returns, from the transposed table tkzT[j n + m] = T_j(x_m) (lanes of
-// consecutive nodes read consecutive words).
+// S(x_m, c) for axis idx / NN (c = x, y, z) and node m = idx % NN, idx < 3 NN, by the Clenshaw
+// recurrence of ComputeSn2 (bbfmm.c:1682-1690), S = 1/2 T_0(x_m) + sum_k T_k(x_m) T_k(c), from the
+// transposed table tkzT[j n + m] = T_j(x_m) (lanes of consecutive nodes read consecutive words).
 template <typename T, int NN>
 __device__ __forceinline__ T sn_value(const T *__restrict__ tkzT, int idx, T x, T y, T z) {
   const int a = idx / NN, m = idx % NN;
@@ -70,63 +51,179 @@ template <> __device__ __forceinline__ const float *tab_cw<float>(const Tables &
 // S_leaf[m * n3 + l], Morton order at maxlev. With Ssplit (mixed mode) the kernel also writes
 // the [hi | lo] BF16 split of the same rows (hi plane count x n3, then the lo plane), as
 // split_rows_kernel would from S, for the tensor-core up projection.
+//
+// Four particles a pass: their 3 n S values each are spread over the lanes (independent Clenshaw
+// chains, three a lane at n = 8) into shared memory, then every lane adds its n^3 / 32 products,
+// with q Sz Sy formed once per (particle, l2). Bound by FP64 issue in full leaves and by the
+// latency of the chains in small ones; a leaf of thousands of particles would be one warp's serial
+// work, so leaves above `cap` are left to the item form (below) and only skipped here.
+//
+// With `items` the kernel instead takes one (row, p0, p1, cell) chunk of a heavy leaf per warp and
+// writes its plain sums to part[item n3 ...]; p2m_join_kernel adds a leaf's chunks in order.
+template <typename T, int NN>
+struct P2MSum {
+  static constexpr int N3 = NN * NN * NN, PER = N3 / 32, G = 4;
+  // acc[k] += sum over particles [p0, p1) of q Sx Sy Sz at node lane + 32 k; sS: G x 3 NN values and
+  // sq: G charges of this warp
+  static __device__ __forceinline__ void run(const T *__restrict__ pos4, int p0, int p1, T cx, T cy, T cz, T ihalf,
+                                             const T *s_tkzT, T *sS, T *sq, int lane, T *acc);
+};
+
+template <typename T, int NN>
+__device__ __forceinline__ void P2MSum<T, NN>::run(const T *__restrict__ pos4, int p0, int p1, T cx, T cy, T cz, T ihalf,
+                                                   const T *s_tkzT, T *sS, T *sq, int lane, T *acc) {
+  for (int p = p0; p < p1; p += G) {
+    const int n = p1 - p < G ? p1 - p : G;
+#pragma unroll
+    for (int e = 0; e < (G * 3 * NN + 31) / 32; ++e) {
+      const int v = lane + 32 * e, j = v / (3 * NN);
+      if (j < n) {  // NN = 4: 48 values, the second round is half full (j = 4 there is past every n)
+        const T *me = pos4 + 4 * (int64_t)(p + j);
+        sS[v] = sn_value<T, NN>(s_tkzT, v % (3 * NN), ihalf * (me[0] - cx), ihalf * (me[1] - cy), ihalf * (me[2] - cz));
+      }
+    }
+    if (lane < n) sq[lane] = pos4[4 * (int64_t)(p + lane) + 3];
+    __syncwarp();
+#pragma unroll
+    for (int j = 0; j < G; ++j) {
+      if (j < n) {
+        const T *S = sS + j * 3 * NN;
+        const T qz = sq[j] * S[2 * NN + (lane & (NN - 1))];
+        if constexpr (NN == 8) {  // node lane + 32 k: l1 = k / 2, l2 = lane / 8 + 4 (k mod 2), l3 = lane mod 8
+          const T w0 = qz * S[NN + (lane >> 3)], w1 = qz * S[NN + 4 + (lane >> 3)];
+#pragma unroll
+          for (int k = 0; k < 8; ++k) {
+            const T sx = S[k];
+            acc[2 * k] += sx * w0;
+            acc[2 * k + 1] += sx * w1;
+          }
+        } else {  // n = 4: l1 = lane / 16 + 2 k, l2 = (lane / 4) mod 4, l3 = lane mod 4
+          const T w = qz * S[NN + ((lane >> 2) & 3)];
+          acc[0] += S[lane >> 4] * w;
+          acc[1] += S[2 + (lane >> 4)] * w;
+        }
+      }
+    }
+    __syncwarp();  // sS and sq are rewritten for the next four
+  }
+}
+
+// S row (and its BF16 split) from a lane's sums.
+template <typename T, int NN>
+__device__ __forceinline__ void p2m_store(const T *acc, T pre3, int lane, int64_t row, int64_t count, T *__restrict__ S,
+                                          __nv_bfloat16 *__restrict__ Ssplit) {
+  constexpr int N3 = NN * NN * NN, PER = N3 / 32;
+  T *out = S + row * N3;
+#pragma unroll
+  for (int k = 0; k < PER; ++k) out[lane + 32 * k] = pre3 * acc[k];
+  if (Ssplit) {
+    __nv_bfloat16 *hi = Ssplit + row * N3, *lo = Ssplit + (count + row) * N3;
+#pragma unroll
+    for (int k = 0; k < PER; ++k) {
+      const double x = (double)(pre3 * acc[k]);
+      const __nv_bfloat16 h = __double2bfloat16(x);
+      hi[lane + 32 * k] = h;
+      lo[lane + 32 * k] = __double2bfloat16(x - (double)__bfloat162float(h));
+    }
+  }
+}
+
 template <typename T, int NN>
 __global__ void __launch_bounds__(128) p2m_kernel(const T *__restrict__ pos4, const int *__restrict__ leaf_start,
                                                   int maxlev, T L, Tables tabs, T *__restrict__ S, int64_t m0,
                                                   int64_t count, __nv_bfloat16 *__restrict__ Ssplit,
-                                                  const int64_t *__restrict__ rows) {
-  constexpr int N3 = NN * NN * NN;
-  constexpr int PER = (N3 + 31) / 32;
-  __shared__ T s_tkz[NN * NN];
+                                                  const int64_t *__restrict__ rows, int cap,
+                                                  const int4 *__restrict__ items, int nitems, T *__restrict__ part) {
+  using Sum = P2MSum<T, NN>;
+  __shared__ T s_tkzT[NN * NN];  // transposed: s_tkzT[j n + m] = T_j(x_m)
+  __shared__ T s_S[4][Sum::G * 3 * NN], s_q[4][Sum::G];
   const T *tkz = tab_tkz<T>(tabs);
-  for (int i = threadIdx.x; i < NN * NN; i += blockDim.x) s_tkz[i] = tkz[i];
+  for (int i = threadIdx.x; i < NN * NN; i += blockDim.x) s_tkzT[(i % NN) * NN + i / NN] = tkz[i];
   __syncthreads();
-  const int lane = threadIdx.x & 31;
+  const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
   const T len = cell_length<T>(maxlev, L);
   const T ihalf = (T)1 / (len / (T)2);
   const T prefac = (T)2 / (T)NN;
   const T pre3 = prefac * prefac * prefac;
   const int64_t warp = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
   const int64_t nwarps = ((int64_t)gridDim.x * blockDim.x) >> 5;
-  for (int64_t mm = warp; mm < count; mm += nwarps) {
-    const int64_t m = pass_cell(rows, m0, mm);  // leaf; S holds the pass's leaves in order
+  const int64_t todo = items ? nitems : count;
+  for (int64_t mm = warp; mm < todo; mm += nwarps) {
+    int64_t m;  // leaf; S holds the pass's leaves in order
+    int p0, p1;
+    if (items) {
+      const int4 it = items[mm];
+      if (it.x < m0 || it.x >= m0 + count) continue;  // a leaf of another slab
+      m = it.w;
+      p0 = it.y;
+      p1 = it.z;
+    } else {
+      m = pass_cell(rows, m0, mm);
+      p0 = leaf_start[m];
+      p1 = leaf_start[m + 1];
+      if (p1 - p0 > cap) continue;
+    }
     int ix, iy, iz;
     morton_to_grid(m, maxlev, ix, iy, iz);  // the set index above bit 3 maxlev is ignored
     const T cx = cell_center_1d<T>(ix, maxlev, L), cy = cell_center_1d<T>(iy, maxlev, L),
             cz = cell_center_1d<T>(iz, maxlev, L);
-    T acc[PER];
+    T acc[Sum::PER];
 #pragma unroll
-    for (int k = 0; k < PER; ++k) acc[k] = 0;
-    const int p0 = leaf_start[m], p1 = leaf_start[m + 1];
-    for (int p = p0; p < p1; ++p) {
-      const T x = ihalf * (pos4[4 * (int64_t)p] - cx);
-      const T y = ihalf * (pos4[4 * (int64_t)p + 1] - cy);
-      const T z = ihalf * (pos4[4 * (int64_t)p + 2] - cz);
-      const T q = pos4[4 * (int64_t)p + 3];
-      const T val = sn_lane<T, NN>(s_tkz, lane, x, y, z);
-      const T szl = wshfl(val, 2 * NN + lane % NN);  // l3 = lane % NN for every k (32 % NN == 0)
+    for (int k = 0; k < Sum::PER; ++k) acc[k] = 0;
+    Sum::run(pos4, p0, p1, cx, cy, cz, ihalf, s_tkzT, s_S[wib], s_q[wib], lane, acc);
+    if (items) {
 #pragma unroll
-      for (int k = 0; k < PER; ++k) {  // N3 is a multiple of 32: every lane has PER outputs
-        const int l = lane + 32 * k;
-        const int l1 = l / (NN * NN), l2 = (l / NN) % NN;
-        const T w = q * wshfl(val, l1) * wshfl(val, NN + l2);
-        acc[k] += w * szl;
-      }
-    }
-    T *out = S + mm * N3;
-#pragma unroll
-    for (int k = 0; k < PER; ++k) out[lane + 32 * k] = pre3 * acc[k];
-    if (Ssplit) {
-      __nv_bfloat16 *hi = Ssplit + mm * N3, *lo = Ssplit + (count + mm) * N3;
-#pragma unroll
-      for (int k = 0; k < PER; ++k) {
-        const double x = (double)(pre3 * acc[k]);
-        const __nv_bfloat16 h = __double2bfloat16(x);
-        hi[lane + 32 * k] = h;
-        lo[lane + 32 * k] = __double2bfloat16(x - (double)__bfloat162float(h));
-      }
+      for (int k = 0; k < Sum::PER; ++k) part[mm * Sum::N3 + lane + 32 * k] = acc[k];
+    } else {
+      p2m_store<T, NN>(acc, pre3, lane, mm, count, S, Ssplit);
     }
   }
+}
+
+// One warp per heavy leaf (row, first item, items, -): its chunks' sums in order.
+template <typename T, int NN>
+__global__ void __launch_bounds__(128) p2m_join_kernel(const int4 *__restrict__ heavy, int nheavy,
+                                                       const T *__restrict__ part, T *__restrict__ S, int64_t m0,
+                                                       int64_t count, __nv_bfloat16 *__restrict__ Ssplit) {
+  constexpr int N3 = NN * NN * NN, PER = N3 / 32;
+  const int w = blockIdx.x * 4 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+  if (w >= nheavy) return;
+  const int4 h = heavy[w];
+  if (h.x < m0 || h.x >= m0 + count) return;
+  const T prefac = (T)2 / (T)NN;
+  T acc[PER];
+#pragma unroll
+  for (int k = 0; k < PER; ++k) acc[k] = 0;
+  for (int i = 0; i < h.z; ++i)
+#pragma unroll
+    for (int k = 0; k < PER; ++k) acc[k] += part[(int64_t)(h.y + i) * N3 + lane + 32 * k];
+  p2m_store<T, NN>(acc, prefac * prefac * prefac, lane, h.x - m0, count, S, Ssplit);
+}
+
+// The leaves (rows of a pass: cells, or the cells of a row list) above `cap` particles: with items
+// null only counts (counts[0] items of at most cap particles, counts[1] leaves), else writes
+// items (row, p0, p1, cell) and heavy (row, first item, items, cell), in no particular order of leaves.
+__global__ void heavy_kernel(const int *__restrict__ leaf_start, const int64_t *__restrict__ rows, int64_t count, int cap,
+                             int *counts, int4 *items, int4 *heavy) {
+  for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < count; t += (int64_t)gridDim.x * blockDim.x) {
+    const int64_t m = pass_cell(rows, 0, t);
+    const int p0 = leaf_start[m], p1 = leaf_start[m + 1];
+    if (p1 - p0 <= cap) continue;
+    const int n = (p1 - p0 + cap - 1) / cap;
+    const int i0 = atomicAdd(&counts[0], n), h = atomicAdd(&counts[1], 1);
+    if (!items) continue;
+    heavy[h] = make_int4((int)t, i0, n, (int)m);
+    for (int i = 0; i < n; ++i)
+      items[i0 + i] = make_int4((int)t, p0 + i * cap, min(p1, p0 + (i + 1) * cap), (int)m);
+  }
+}
+
+int launch_heavy(const int *leaf_start, const int64_t *rows, int64_t count, int cap, int *counts, int4 *items, int4 *heavy,
+                 cudaStream_t s) {
+  if (count <= 0) return BBFMM_OK;
+  const int64_t g = (count + 255) / 256;
+  heavy_kernel<<<(unsigned)(g < 148 * 16 ? g : 148 * 16), 256, 0, s>>>(leaf_start, rows, count, cap, counts, items, heavy);
+  return bbfmm_set_cuda_error(cudaGetLastError(), "heavy leaves", __FILE__, __LINE__);
 }
 
 // ----------------------------------------------------------------------------- M2M
@@ -309,13 +406,15 @@ __device__ __forceinline__ uint32_t pass_smem_u32(const void *p) { return (uint3
 // chunk ahead (and whose centres they compute, one leaf per lane), so no leaf waits for its own
 // offset loads. Empty leaves take no copy (the slot's barrier is arrived at without bytes).
 // body(p0, p1, the slot -- the leaf's n^3 values, then the positions of particles
-// p0 .. p0 + L2P_PCAP - 1 --, leaf centre) does the arithmetic. A wait that gives up records
+// p0 .. p0 + L2P_PCAP - 1 --, leaf centre) does the arithmetic. Leaves above `cap` particles are
+// skipped; a second launch takes them as `items` (row, p0, p1, cell), chunks of at most `cap`. A wait that gives up records
 // PASS_WAIT_CODE in g_pass_status and ends the warp's work.
 template <typename T, int NN, typename Body>
 __device__ __forceinline__ void l2p_pipeline(const int *__restrict__ leaf_start, const T *__restrict__ F,
                                              const T *__restrict__ pos4, int maxlev, T L, int64_t m0, int64_t count,
-                                             const int64_t *__restrict__ rows, T *ring_all, uint64_t *bars_all,
-                                             int2 *offs_all, Body body) {
+                                             const int64_t *__restrict__ rows, int cap,
+                                             const int4 *__restrict__ items, int nitems, T *ring_all,
+                                             uint64_t *bars_all, int2 *offs_all, Body body) {
   constexpr int N3 = NN * NN * NN, D = L2P_DEPTH, SLOT = l2p_slot_elems<T, NN>();
   static_assert(D < 32, "the slots run at most one offset chunk ahead");
   constexpr uint32_t BYTES = N3 * sizeof(T);
@@ -323,7 +422,8 @@ __device__ __forceinline__ void l2p_pipeline(const int *__restrict__ leaf_start,
   const int64_t warp = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
   const int64_t nwarps = ((int64_t)gridDim.x * blockDim.x) >> 5;
   // leaves of this warp: index i is local row warp + i nwarps
-  const int64_t nmine = warp < count ? (count - warp + nwarps - 1) / nwarps : 0;
+  const int64_t todo = items ? nitems : count;
+  const int64_t nmine = warp < todo ? (todo - warp + nwarps - 1) / nwarps : 0;
   T *ring = ring_all + (size_t)wib * D * SLOT;
   uint64_t *bars = bars_all + wib * D;
   int2 *offs = offs_all + wib * D;
@@ -335,14 +435,24 @@ __device__ __forceinline__ void l2p_pipeline(const int *__restrict__ leaf_start,
   __syncwarp();
   // chunk c of 32 leaves: lane j holds leaf 32 c + j's cell and offsets (loaded one chunk
   // ahead) and, for the current chunk, its centre
-  auto load_chunk = [&](int64_t c, int64_t &m, int &p0, int &p1) {
+  auto load_chunk = [&](int64_t c, int64_t &m, int &p0, int &p1, int64_t &fr) {
     const int64_t i = 32 * c + lane;
-    m = 0;
+    m = fr = 0;
     p0 = p1 = 0;
     if (i < nmine) {
-      m = pass_cell(rows, m0, warp + i * nwarps);
-      p0 = leaf_start[m];
-      p1 = leaf_start[m + 1];
+      fr = warp + i * nwarps;
+      if (items) {  // a chunk of a heavy leaf; chunks of other slabs' leaves count as empty
+        const int4 it = items[fr];
+        m = it.w;
+        p0 = it.y;
+        p1 = it.x >= m0 && it.x < m0 + count ? it.z : p0;
+        fr = it.x - m0;
+      } else {
+        m = pass_cell(rows, m0, fr);
+        p0 = leaf_start[m];
+        p1 = leaf_start[m + 1];
+        if (p1 - p0 > cap) p1 = p0;  // heavy: left to its items
+      }
     }
   };
   T ccx, ccy, ccz;  // centre of this lane's leaf of the current chunk
@@ -353,13 +463,13 @@ __device__ __forceinline__ void l2p_pipeline(const int *__restrict__ leaf_start,
     ccy = cell_center_1d<T>(iy, maxlev, L);
     ccz = cell_center_1d<T>(iz, maxlev, L);
   };
-  int64_t cm, nm;  // cells of the current chunk and the next one
+  int64_t cm, nm, cf, nf;  // cells and F rows of the current chunk and the next one
   int c0, c1, n0, n1;
-  load_chunk(0, cm, c0, c1);
-  load_chunk(1, nm, n0, n1);
+  load_chunk(0, cm, c0, c1, cf);
+  load_chunk(1, nm, n0, n1, nf);
   centre(cm);
   // lane 0: slot (i % D) <- leaf i, whose offsets are (p0, p1)
-  auto issue = [&](int64_t i, int p0, int p1) {
+  auto issue = [&](int64_t i, int p0, int p1, int64_t fr) {
     const int d = (int)(i % D);
     offs[d] = make_int2(p0, p1);
     const uint32_t bar = pass_smem_u32(bars + d);
@@ -373,7 +483,7 @@ __device__ __forceinline__ void l2p_pipeline(const int *__restrict__ leaf_start,
       asm volatile(
           "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
               pass_smem_u32(slot)),
-          "l"(F + (warp + i * nwarps) * N3), "r"(BYTES), "r"(bar)
+          "l"(F + fr * N3), "r"(BYTES), "r"(bar)
           : "memory");
       asm volatile(
           "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
@@ -383,18 +493,21 @@ __device__ __forceinline__ void l2p_pipeline(const int *__restrict__ leaf_start,
     }
   };
   // offsets of leaf j (in the current chunk of leaf i or the next one), from its lane
-  auto offsets_of = [&](int64_t j, int64_t i, int &p0, int &p1) {
+  auto offsets_of = [&](int64_t j, int64_t i, int &p0, int &p1, int64_t &fr) {
     const bool here = (j >> 5) == (i >> 5);
     const int a0 = __shfl_sync(0xffffffffu, c0, (int)(j & 31)), a1 = __shfl_sync(0xffffffffu, c1, (int)(j & 31));
     const int b0 = __shfl_sync(0xffffffffu, n0, (int)(j & 31)), b1 = __shfl_sync(0xffffffffu, n1, (int)(j & 31));
+    const int64_t f0 = __shfl_sync(0xffffffffu, cf, (int)(j & 31)), f1 = __shfl_sync(0xffffffffu, nf, (int)(j & 31));
     p0 = here ? a0 : b0;
     p1 = here ? a1 : b1;
+    fr = here ? f0 : f1;
   };
   int64_t nxt = 0;  // next leaf to issue
   for (; nxt < D && nxt < nmine; ++nxt) {
     int p0, p1;
-    offsets_of(nxt, 0, p0, p1);
-    if (lane == 0) issue(nxt, p0, p1);
+    int64_t fr;
+    offsets_of(nxt, 0, p0, p1, fr);
+    if (lane == 0) issue(nxt, p0, p1, fr);
   }
   auto wait_slot = [&](int64_t i) -> bool {  // bounded wait for leaf i's slot
     const uint32_t bar = pass_smem_u32(bars + (int)(i % D));
@@ -416,7 +529,8 @@ __device__ __forceinline__ void l2p_pipeline(const int *__restrict__ leaf_start,
       cm = nm;
       c0 = n0;
       c1 = n1;
-      load_chunk((i >> 5) + 1, nm, n0, n1);
+      cf = nf;
+      load_chunk((i >> 5) + 1, nm, n0, n1, nf);
       centre(cm);
     }
     if (!wait_slot(i)) {
@@ -433,8 +547,9 @@ __device__ __forceinline__ void l2p_pipeline(const int *__restrict__ leaf_start,
     __syncwarp();  // every lane has used the slot's values
     if (nxt < nmine) {
       int p0, p1;
-      offsets_of(nxt, i, p0, p1);
-      if (lane == 0) issue(nxt, p0, p1);
+      int64_t fr;
+      offsets_of(nxt, i, p0, p1, fr);
+      if (lane == 0) issue(nxt, p0, p1, fr);
       ++nxt;
     }
   }
@@ -453,7 +568,8 @@ template <typename T, int NN>
 __global__ void __launch_bounds__(128, 4) l2p_kernel(const T *__restrict__ pos4, const int *__restrict__ leaf_start,
                                                   int maxlev, T L, Tables tabs, const T *__restrict__ F,
                                                   T *__restrict__ phi, int64_t m0, int64_t count,
-                                                  const int64_t *__restrict__ rows) {
+                                                  const int64_t *__restrict__ rows, int cap,
+                                                  const int4 *__restrict__ items, int nitems) {
   __shared__ T s_tkzT[NN * NN];  // transposed: s_tkzT[j n + m] = T_j(x_m)
   const T *tkz = tab_tkz<T>(tabs);
   for (int i = threadIdx.x; i < NN * NN; i += blockDim.x) s_tkzT[(i % NN) * NN + i / NN] = tkz[i];
@@ -474,8 +590,8 @@ __global__ void __launch_bounds__(128, 4) l2p_kernel(const T *__restrict__ pos4,
   __shared__ T s_S[L2P_WARPS][2][3 * NN];
   const int h = lane >> 4, s = lane & 15;
   T *sS = s_S[threadIdx.x >> 5][h];
-  l2p_pipeline<T, NN>(leaf_start, F, pos4, maxlev, L, m0, count, rows, reinterpret_cast<T *>(l2p_ring), l2p_bars,
-                      l2p_offs, [&](int p0, int p1, const T *slot, T cx, T cy, T cz) {
+  l2p_pipeline<T, NN>(leaf_start, F, pos4, maxlev, L, m0, count, rows, cap, items, nitems,
+                      reinterpret_cast<T *>(l2p_ring), l2p_bars, l2p_offs, [&](int p0, int p1, const T *slot, T cx, T cy, T cz) {
     const T *spos = slot + NN * NN * NN;
     const T *sF = slot + s;  // this lane's values s + 16 k are sF[16 k]
     for (int pb = p0; pb < p1; pb += 2) {
@@ -656,15 +772,25 @@ int pass_status(int clear) {
   return v;
 }
 
+template <typename T, int NN>
+static void p2m_launches(const T *pos4, const int *leaf_start, int maxlev, T L, const Tables &t, T *S, cudaStream_t s,
+                         int64_t first, int64_t count, __nv_bfloat16 *sp, const int64_t *rows, const HeavyLeaves &h) {
+  p2m_kernel<T, NN><<<grid_for(count, 4, 148 * 64), 128, 0, s>>>(pos4, leaf_start, maxlev, L, t, S, first, count, sp, rows,
+                                                              h.cap, nullptr, 0, nullptr);
+  if (h.nitems <= 0) return;
+  p2m_kernel<T, NN><<<grid_for(h.nitems, 4, 148 * 64), 128, 0, s>>>(pos4, leaf_start, maxlev, L, t, S, first, count, sp,
+                                                                 rows, h.cap, h.items, h.nitems, (T *)h.part);
+  p2m_join_kernel<T, NN><<<(h.nheavy + 3) / 4, 128, 0, s>>>(h.heavy, h.nheavy, (const T *)h.part, S, first, count, sp);
+}
+
 template <typename T>
 int launch_p2m(int n, const T *pos4, const int *leaf_start, int maxlev, T L, const Tables &t, T *S, cudaStream_t s,
-               int nsets, int64_t first, int64_t count, void *Ssplit, const int64_t *rows) {
+               int nsets, int64_t first, int64_t count, void *Ssplit, const int64_t *rows, const HeavyLeaves &h) {
   if (count < 0) count = nsets * pow8i(maxlev) - first;
   if (count <= 0) return BBFMM_OK;
-  const int grid = grid_for(count, 4, 148 * 64);
   __nv_bfloat16 *sp = (__nv_bfloat16 *)Ssplit;
-  if (n == 4) p2m_kernel<T, 4><<<grid, 128, 0, s>>>(pos4, leaf_start, maxlev, L, t, S, first, count, sp, rows);
-  else if (n == 8) p2m_kernel<T, 8><<<grid, 128, 0, s>>>(pos4, leaf_start, maxlev, L, t, S, first, count, sp, rows);
+  if (n == 4) p2m_launches<T, 4>(pos4, leaf_start, maxlev, L, t, S, s, first, count, sp, rows, h);
+  else if (n == 8) p2m_launches<T, 8>(pos4, leaf_start, maxlev, L, t, S, s, first, count, sp, rows, h);
   else return bbfmm_set_error(BBFMM_ERR_UNSUPPORTED, "order n must be 4 or 8");
   return bbfmm_set_cuda_error(cudaGetLastError(), "p2m", __FILE__, __LINE__);
 }
@@ -707,18 +833,25 @@ int launch_l2l(int n, const T *Fp, T *Fc, int level, const Tables &t, cudaStream
   return bbfmm_set_cuda_error(cudaGetLastError(), "l2l", __FILE__, __LINE__);
 }
 
+template <typename T, int NN>
+static void l2p_launches(const T *pos4, const int *leaf_start, int maxlev, T L, const Tables &t, const T *F, T *phi,
+                         cudaStream_t s, int64_t first, int64_t count, const int64_t *rows, const HeavyLeaves &h) {
+  constexpr int sm = l2p_smem_bytes<T, NN>();
+  const int most = resident_grid<l2p_kernel<T, NN>>(128, sm);
+  l2p_kernel<T, NN><<<grid_for(count, 4, most), 128, sm, s>>>(pos4, leaf_start, maxlev, L, t, F, phi, first, count, rows,
+                                                           h.cap, nullptr, 0);
+  if (h.nitems > 0)
+    l2p_kernel<T, NN><<<grid_for(h.nitems, 4, most), 128, sm, s>>>(pos4, leaf_start, maxlev, L, t, F, phi, first, count,
+                                                                rows, h.cap, h.items, h.nitems);
+}
+
 template <typename T>
 int launch_l2p(int n, const T *pos4, const int *leaf_start, int maxlev, T L, const Tables &t, const T *F, T *phi,
-               cudaStream_t s, int nsets, int64_t first, int64_t count, const int64_t *rows) {
+               cudaStream_t s, int nsets, int64_t first, int64_t count, const int64_t *rows, const HeavyLeaves &h) {
   if (count < 0) count = nsets * pow8i(maxlev) - first;
   if (count <= 0) return BBFMM_OK;
-  constexpr int sm4 = l2p_smem_bytes<T, 4>(), sm8 = l2p_smem_bytes<T, 8>();
-  if (n == 4)
-    l2p_kernel<T, 4><<<grid_for(count, 4, resident_grid<l2p_kernel<T, 4>>(128, sm4)), 128, sm4, s>>>(
-        pos4, leaf_start, maxlev, L, t, F, phi, first, count, rows);
-  else if (n == 8)
-    l2p_kernel<T, 8><<<grid_for(count, 4, resident_grid<l2p_kernel<T, 8>>(128, sm8)), 128, sm8, s>>>(
-        pos4, leaf_start, maxlev, L, t, F, phi, first, count, rows);
+  if (n == 4) l2p_launches<T, 4>(pos4, leaf_start, maxlev, L, t, F, phi, s, first, count, rows, h);
+  else if (n == 8) l2p_launches<T, 8>(pos4, leaf_start, maxlev, L, t, F, phi, s, first, count, rows, h);
   else return bbfmm_set_error(BBFMM_ERR_UNSUPPORTED, "order n must be 4 or 8");
   return bbfmm_set_cuda_error(cudaGetLastError(), "l2p", __FILE__, __LINE__);
 }
@@ -763,11 +896,11 @@ int launch_morton_cpg(int level, int r, const T *src, T *dst, int inverse, cudaS
 
 #define INST(T)                                                                                           \
   template int launch_p2m<T>(int, const T *, const int *, int, T, const Tables &, T *, cudaStream_t, int,   \
-                             int64_t, int64_t, void *, const int64_t *);                                   \
+                             int64_t, int64_t, void *, const int64_t *, const HeavyLeaves &);               \
   template int launch_m2m<T>(int, const T *, T *, int, const Tables &, cudaStream_t, int, int64_t, int64_t); \
   template int launch_l2l<T>(int, const T *, T *, int, const Tables &, cudaStream_t, int, int64_t, int64_t); \
   template int launch_l2p<T>(int, const T *, const int *, int, T, const Tables &, const T *, T *,          \
-                             cudaStream_t, int, int64_t, int64_t, const int64_t *);                        \
+                             cudaStream_t, int, int64_t, int64_t, const int64_t *, const HeavyLeaves &);    \
   template int launch_proj<T>(int64_t, int, int, const T *, const float *, const T *, const T *, T, T *,   \
                               int, int, cudaStream_t, int64_t, int, int, const int64_t *);                 \
   template int launch_morton_cpg<T>(int, int, const T *, T *, int, cudaStream_t);
@@ -843,7 +976,8 @@ template <typename T, int NN>
 __global__ void __launch_bounds__(128, 4) l2p_field_kernel(const T *__restrict__ pos4, const int *__restrict__ leaf_start,
                                                         int maxlev, T L, Tables tabs, const T *__restrict__ F,
                                                         T *__restrict__ pot, T *__restrict__ fld, int64_t m0,
-                                                        int64_t count, const int64_t *__restrict__ rows) {
+                                                        int64_t count, const int64_t *__restrict__ rows, int cap,
+                                                        const int4 *__restrict__ items, int nitems) {
   __shared__ T s_tkzT[NN * NN];  // transposed: s_tkzT[j n + m] = T_j(x_m)
   const T *tkz = tab_tkz<T>(tabs);
   for (int i = threadIdx.x; i < NN * NN; i += blockDim.x) s_tkzT[(i % NN) * NN + i / NN] = tkz[i];
@@ -862,8 +996,8 @@ __global__ void __launch_bounds__(128, 4) l2p_field_kernel(const T *__restrict__
   __shared__ T s_S[L2P_WARPS][2][3 * NN], s_D[L2P_WARPS][2][3 * NN];
   const int h = lane >> 4, s = lane & 15;
   T *sS = s_S[threadIdx.x >> 5][h], *sD = s_D[threadIdx.x >> 5][h];
-  l2p_pipeline<T, NN>(leaf_start, F, pos4, maxlev, L, m0, count, rows, reinterpret_cast<T *>(l2p_ring), l2p_bars,
-                      l2p_offs, [&](int p0, int p1, const T *slot, T cx, T cy, T cz) {
+  l2p_pipeline<T, NN>(leaf_start, F, pos4, maxlev, L, m0, count, rows, cap, items, nitems,
+                      reinterpret_cast<T *>(l2p_ring), l2p_bars, l2p_offs, [&](int p0, int p1, const T *slot, T cx, T cy, T cz) {
     const T *spos = slot + NN * NN * NN;
     const T *sF = slot + s;  // this lane's values s + 16 k are sF[16 k]
     for (int pb = p0; pb < p1; pb += 2) {
@@ -943,18 +1077,27 @@ __global__ void scatter_field_kernel(int N, const int *__restrict__ perm, const 
   }
 }
 
+template <typename T, int NN>
+static void l2p_field_launches(const T *pos4, const int *leaf_start, int maxlev, T L, const Tables &t, const T *F, T *pot,
+                               T *fld, cudaStream_t s, int64_t first, int64_t count, const int64_t *rows,
+                               const HeavyLeaves &h) {
+  constexpr int sm = l2p_smem_bytes<T, NN>();
+  const int most = resident_grid<l2p_field_kernel<T, NN>>(128, sm);
+  l2p_field_kernel<T, NN><<<grid_for(count, 4, most), 128, sm, s>>>(pos4, leaf_start, maxlev, L, t, F, pot, fld, first,
+                                                                 count, rows, h.cap, nullptr, 0);
+  if (h.nitems > 0)
+    l2p_field_kernel<T, NN><<<grid_for(h.nitems, 4, most), 128, sm, s>>>(pos4, leaf_start, maxlev, L, t, F, pot, fld, first,
+                                                                      count, rows, h.cap, h.items, h.nitems);
+}
+
 template <typename T>
 int launch_l2p_field(int n, const T *pos4, const int *leaf_start, int maxlev, T L, const Tables &t, const T *F,
-                     T *pot, T *fld, cudaStream_t s, int nsets, int64_t first, int64_t count, const int64_t *rows) {
+                     T *pot, T *fld, cudaStream_t s, int nsets, int64_t first, int64_t count, const int64_t *rows,
+                     const HeavyLeaves &h) {
   if (count < 0) count = nsets * pow8i(maxlev) - first;
   if (count <= 0) return BBFMM_OK;
-  constexpr int sm4 = l2p_smem_bytes<T, 4>(), sm8 = l2p_smem_bytes<T, 8>();
-  if (n == 4)
-    l2p_field_kernel<T, 4><<<grid_for(count, 4, resident_grid<l2p_field_kernel<T, 4>>(128, sm4)), 128, sm4, s>>>(
-        pos4, leaf_start, maxlev, L, t, F, pot, fld, first, count, rows);
-  else if (n == 8)
-    l2p_field_kernel<T, 8><<<grid_for(count, 4, resident_grid<l2p_field_kernel<T, 8>>(128, sm8)), 128, sm8, s>>>(
-        pos4, leaf_start, maxlev, L, t, F, pot, fld, first, count, rows);
+  if (n == 4) l2p_field_launches<T, 4>(pos4, leaf_start, maxlev, L, t, F, pot, fld, s, first, count, rows, h);
+  else if (n == 8) l2p_field_launches<T, 8>(pos4, leaf_start, maxlev, L, t, F, pot, fld, s, first, count, rows, h);
   else return bbfmm_set_error(BBFMM_ERR_UNSUPPORTED, "order n must be 4 or 8");
   return bbfmm_set_cuda_error(cudaGetLastError(), "l2p_field", __FILE__, __LINE__);
 }
@@ -968,9 +1111,11 @@ int launch_scatter_field(int N, const int *perm, const T *pot, const T *fld, TO 
 }
 
 template int launch_l2p_field<double>(int, const double *, const int *, int, double, const Tables &, const double *,
-                                      double *, double *, cudaStream_t, int, int64_t, int64_t, const int64_t *);
+                                      double *, double *, cudaStream_t, int, int64_t, int64_t, const int64_t *,
+                                      const HeavyLeaves &);
 template int launch_l2p_field<float>(int, const float *, const int *, int, float, const Tables &, const float *,
-                                     float *, float *, cudaStream_t, int, int64_t, int64_t, const int64_t *);
+                                     float *, float *, cudaStream_t, int, int64_t, int64_t, const int64_t *,
+                                     const HeavyLeaves &);
 template int launch_scatter_field<double, double>(int, const int *, const double *, const double *, double *,
                                                   double *, cudaStream_t);
 template int launch_scatter_field<float, float>(int, const int *, const float *, const float *, float *, float *,

@@ -308,6 +308,7 @@ int Solver<T>::set_particles_global(int nsets_, int N_, const int *perm_h, const
   if (N > 0) BBFMM_CUDA_OK(cudaMemcpy(perm, perm_h, sizeof(int) * N, cudaMemcpyHostToDevice));
   BBFMM_CUDA_OK(cudaMemcpy(leaf_start, leaf_start_h, sizeof(int) * (nl + 1), cudaMemcpyHostToDevice));
   BBFMM_CUDA_OK(cudaDeviceSynchronize());
+  TRY(build_heavy());
   TRY(build_near_work());
   if (N > 0) {
     T *xyz_d = nullptr;
@@ -367,6 +368,7 @@ int Solver<T>::set_particles_sets_device(int nsets_, const int *off_h, const int
   TRY(dalloc(&pos4, 4 * (size_t)(N > 0 ? N : 1)));
   TRY(dalloc(&phis, N > 0 ? N : 1));
   TRY(build_tree_device_sets<T>(nsets, off_h, count_h, xyz_d, (T)L, maxlev, perm, leaf_start, stream));
+  TRY(build_heavy());
   TRY(build_near_work());
   if (N > 0) TRY((launch_gather<T, T>(N, perm, xyz_d, nullptr, pos4, stream)));
   TRY(alloc_work());
@@ -415,8 +417,9 @@ int Solver<T>::upward(const void *q_dev, int q_is_double) {
     const int64_t c = nl - a < sl ? nl - a : sl;
     // mixed mode: P2M also writes the BF16 split of S that the tensor-core up projection reads
     void *sp = proj_tc() && c <= Ssplit_rows ? Ssplit : nullptr;
-    TRY(launch_p2m<T>(n, pos4, leaf_start, maxlev, (T)L, tb, Sl, stream, nsets, a, c, sp, lr ? lr + a : nullptr));
-    mark(ST_P2M);
+    TRY(launch_p2m<T>(n, pos4, leaf_start, maxlev, (T)L, tb, Sl, stream, nsets, a, c, sp, lr ? lr + a : nullptr,
+                      heavy_up));
+    mark(ST_P2M, heavy_up.nitems > 0 ? 3 : 1);
     TRY(proj_up(c, Sl, maxlev, a, sp != nullptr, lr ? lr + a : nullptr));
     mark(ST_PROJ_UP);
     if (maxlev - 1 >= lowest) {
@@ -522,9 +525,10 @@ int Solver<T>::leaf_down(bool field) {
       }
     }
     if (field)
-      TRY(launch_l2p_field<T>(n, pos4, leaf_start, maxlev, (T)L, tb, Fl, phis, flds, stream, nsets, a, c, rl));
-    else TRY(launch_l2p<T>(n, pos4, leaf_start, maxlev, (T)L, tb, Fl, phis, stream, nsets, a, c, rl));
-    mark(ST_L2P);
+      TRY(launch_l2p_field<T>(n, pos4, leaf_start, maxlev, (T)L, tb, Fl, phis, flds, stream, nsets, a, c, rl, heavy_down));
+    else
+      TRY(launch_l2p<T>(n, pos4, leaf_start, maxlev, (T)L, tb, Fl, phis, stream, nsets, a, c, rl, heavy_down));
+    mark(ST_L2P, heavy_down.nitems > 0 ? 2 : 1);
   }
   return BBFMM_OK;
 }
@@ -698,14 +702,17 @@ int Solver<T>::set_target_region(int level, const unsigned char *active_host) {
     TRY(build_region_tiles());
   }
   TRY(build_local());
-  return pos4 ? build_near_work() : BBFMM_OK;
+  if (!pos4) return BBFMM_OK;
+  TRY(build_heavy());
+  return build_near_work();
 }
 
 template <typename T>
 int Solver<T>::set_m2l_first(int level) {
   if (level < BBFMM_MINLEV || level > maxlev) return bbfmm_set_error(BBFMM_ERR_ARG, "first M2L level in [2, maxlev]");
   m2l_first = level;
-  return build_local();
+  TRY(build_local());
+  return pos4 ? build_heavy() : BBFMM_OK;
 }
 
 template <typename T>
@@ -716,6 +723,63 @@ void Solver<T>::free_local() {
     src_list[l] = tgt_list[l] = nullptr;
     n_src[l] = n_tgt[l] = 0;
   }
+}
+
+template <typename T>
+void Solver<T>::free_heavy() {
+  for (HeavyLeaves *h : {&heavy_up, &heavy_down}) {
+    if (h->part) cudaFree(h->part);
+    if (h == &heavy_up || h->items != heavy_up.items) {
+      if (h->items) cudaFree(h->items);
+      if (h->heavy) cudaFree(h->heavy);
+    }
+  }
+  heavy_up = heavy_down = HeavyLeaves();
+}
+
+// Lists of the leaves of more than `cap` particles among the rows of P2M and of L2P (the same rows
+// unless the solve is local). cap: 64 (measured: a warp takes about 10 us for that), more above a
+// million particles so that the partial sums stay below 16,384 + N / cap rows.
+template <typename T>
+int Solver<T>::build_heavy() {
+  free_heavy();
+  const int cap = 64 * (int)(((int64_t)N + (1 << 20) - 1) / (1 << 20) > 1 ? ((int64_t)N + (1 << 20) - 1) / (1 << 20) : 1);
+  int *counts = nullptr;
+  TRY(dalloc(&counts, 2));
+  auto list = [&](HeavyLeaves &h, const int64_t *rows, int64_t count, bool parts) -> int {
+    int c[2] = {0, 0};
+    BBFMM_CUDA_OK(cudaMemsetAsync(counts, 0, 8, stream));
+    TRY(launch_heavy(leaf_start, rows, count, cap, counts, nullptr, nullptr, stream));
+    BBFMM_CUDA_OK(cudaMemcpyAsync(c, counts, 8, cudaMemcpyDeviceToHost, stream));
+    BBFMM_CUDA_OK(cudaStreamSynchronize(stream));
+    h.cap = cap;
+    if (c[0] == 0) return BBFMM_OK;
+    TRY(dalloc(&h.items, c[0]));
+    TRY(dalloc(&h.heavy, c[1]));
+    if (parts) {
+      T *p = nullptr;
+      TRY(dalloc(&p, (size_t)c[0] * n3));
+      h.part = p;
+    }
+    BBFMM_CUDA_OK(cudaMemsetAsync(counts, 0, 8, stream));
+    TRY(launch_heavy(leaf_start, rows, count, cap, counts, h.items, h.heavy, stream));
+    h.nitems = c[0];
+    h.nheavy = c[1];
+    return BBFMM_OK;
+  };
+  int rc = local_solve ? list(heavy_up, src_list[maxlev], n_src[maxlev], true) : list(heavy_up, nullptr, cells(maxlev), true);
+  if (rc == BBFMM_OK) {
+    if (local_solve) {
+      rc = list(heavy_down, tgt_list[maxlev], n_tgt[maxlev], false);
+    } else {
+      heavy_down = heavy_up;
+      heavy_down.part = nullptr;
+    }
+  }
+  if (rc == BBFMM_OK) rc = bbfmm_set_cuda_error(cudaStreamSynchronize(stream), "heavy leaves", __FILE__, __LINE__);
+  cudaFree(counts);
+  if (rc != BBFMM_OK) free_heavy();
+  return rc;
 }
 
 // Runs of the region cells (tgt) and of those with their neighbours (src) at region_level,
@@ -1100,6 +1164,7 @@ void Solver<T>::release() {
     if (region_tcboxes[l]) cudaFree(region_tcboxes[l]);
   }
   free_local();
+  free_heavy();
   if (region_mask) cudaFree(region_mask);
   void *ptrs[] = {offs, perm, leaf_start, near_work, pos4, S[0], S[1], F[0], F[1], Mall, Lbuf, Lpart, Msplit,
                   phis, flds, Ssplit, Lsplit, io_q, io_phi, phis2, flds2, qs2, phisn, fldsn};

@@ -33,10 +33,11 @@ int build_tree_device(int N, const T *xyz, T L, int maxlev, int *perm, int *leaf
 template <typename T>
 int build_tree_device_sets(int nseg, const int *off, const int *count, const T *xyz, T L, int maxlev, int *perm,
                            int *leaf_start, cudaStream_t s);
-template <typename T> int launch_p2m(int n, const T *pos4, const int *leaf_start, int maxlev, T L, const Tables &t, T *S, cudaStream_t s, int nsets = 1, int64_t first = 0, int64_t count = -1, void *Ssplit = nullptr, const int64_t *rows = nullptr);
+template <typename T> int launch_p2m(int n, const T *pos4, const int *leaf_start, int maxlev, T L, const Tables &t, T *S, cudaStream_t s, int nsets = 1, int64_t first = 0, int64_t count = -1, void *Ssplit = nullptr, const int64_t *rows = nullptr, const HeavyLeaves &heavy = HeavyLeaves());
+int launch_heavy(const int *leaf_start, const int64_t *rows, int64_t count, int cap, int *counts, int4 *items, int4 *heavy, cudaStream_t s);
 template <typename T> int launch_m2m(int n, const T *Sc, T *Sp, int level, const Tables &t, cudaStream_t s, int nsets = 1, int64_t first = 0, int64_t count = -1);
 template <typename T> int launch_l2l(int n, const T *Fp, T *Fc, int level, const Tables &t, cudaStream_t s, int nsets = 1, int64_t first = 0, int64_t count = -1);
-template <typename T> int launch_l2p(int n, const T *pos4, const int *leaf_start, int maxlev, T L, const Tables &t, const T *F, T *phi, cudaStream_t s, int nsets = 1, int64_t first = 0, int64_t count = -1, const int64_t *rows = nullptr);
+template <typename T> int launch_l2p(int n, const T *pos4, const int *leaf_start, int maxlev, T L, const Tables &t, const T *F, T *phi, cudaStream_t s, int nsets = 1, int64_t first = 0, int64_t count = -1, const int64_t *rows = nullptr, const HeavyLeaves &heavy = HeavyLeaves());
 // rows are a slab of the level starting at cell row0 (the cpg side is indexed by level cell)
 template <typename T> int launch_proj(int64_t M, int K, int N, const T *A, const float *A2, const T *B, const T *cs, T scale, T *C, int level, int mapmode, cudaStream_t s, int64_t row0 = 0, int ldc = 0, int lda = 0, const int64_t *rows = nullptr);
 template <typename T, typename TI> int launch_gather(int N, const int *perm, const TI *xyz, const TI *q, T *pos4, cudaStream_t s);
@@ -63,7 +64,7 @@ int launch_near2(int mode, int N, const void *pos4, const int *leaf_start, int m
                  int nitems, int threads, const void *q2, void *pot, void *fld, void *pot2, void *fld2, cudaStream_t s,
                  const unsigned char *mask = nullptr, int mask_level = 0);
 int pass_status(int clear);  // the passes' bounded waits (L2P leaf copies)
-template <typename T> int launch_l2p_field(int n, const T *pos4, const int *leaf_start, int maxlev, T L, const Tables &t, const T *F, T *pot, T *fld, cudaStream_t s, int nsets = 1, int64_t first = 0, int64_t count = -1, const int64_t *rows = nullptr);
+template <typename T> int launch_l2p_field(int n, const T *pos4, const int *leaf_start, int maxlev, T L, const Tables &t, const T *F, T *pot, T *fld, cudaStream_t s, int nsets = 1, int64_t first = 0, int64_t count = -1, const int64_t *rows = nullptr, const HeavyLeaves &heavy = HeavyLeaves());
 template <typename T, typename TO> int launch_scatter_field(int N, const int *perm, const T *pot, const T *fld, TO *pot_out, TO *fld_out, cudaStream_t s);
 template <typename T> int launch_m2l_simt(int r, const T *M, const T *Ert, T *Lout, int level, int j0, int j1, const int4 *offs, int accumulate, cudaStream_t s, int nsets = 1, int ngroups = 1, T *part = nullptr, int64_t part_elems = 0, const int4 *boxes = nullptr, int nboxes = 0);
 void build_offset_table(int *out);
@@ -295,6 +296,9 @@ struct Solver {
   int build_near_work();                         // the work list for tune.p2p_threads
   int set_target_region(int level, const unsigned char *active_host);  // level < 0 clears
   int set_m2l_first(int level);                                        // m2l_first, then the runs
+  HeavyLeaves heavy_up, heavy_down;  // of the rows that P2M and L2P run over
+  int build_heavy();
+  void free_heavy();
   int build_local();                                                   // runs and row lists
   void free_local();
   bool chunked() const { return slabbed() || local_solve; }  // leaf passes run per leaf chunk
