@@ -1,4 +1,4 @@
-// M2L on CUDA cores over the dense class-major grid of one level.
+// M2L on CUDA cores over the dense class-major grid of one level (FP32 at r = 256).
 //
 //   L(F) = sum_{S in IL(F)} E_{k(F,S)} M(S)     (m2l_kern_basic.cu:82-130 semantics,
 //                                                k from m2l_aux.c:1135-1191)
@@ -11,8 +11,7 @@
 // CTA tile: a box of up to 4x4x4 targets of one class x all r outputs. The kernel loops
 // over the class's offsets and over chunks of 16 contraction indices j in [j0, j1),
 // staging the shifted source box and the operator chunk in shared memory, and keeps a
-// register-blocked accumulator. With [j0, j1) = [0, r) this is the plain FP64 (or FP32)
-// M2L; with [0, 16) it is the FP64 leading-component part of the mixed-precision M2L.
+// register-blocked accumulator.
 // With a box list (a target region) a tile is instead 8 listed 2 x 2 x 2 blocks of parent
 // cells of one class, each of its own set and origin (slots past the list's end are not
 // written).
@@ -29,11 +28,11 @@ struct OffsetTable {
 };
 
 // TM x TN outputs per thread; the CTA has (64 / TM) (R / TN) threads (256 at r = 256 with an
-// 8 x 8 tile, 128 at r = 32 with a 4 x 4 tile: 8 shared-memory loads per 16 FMAs).
+// 8 x 8 tile).
 template <typename T, int R, int TM, int TN>
 __global__ void __launch_bounds__((64 / TM) * (R / TN)) m2l_simt_kernel(const T *__restrict__ M, const T *__restrict__ Ert,
                                                        T *__restrict__ Lout, int level, int j0, int j1,
-                                                       const int4 *__restrict__ offs, int accumulate,
+                                                       const int4 *__restrict__ offs,
                                                        const int4 *__restrict__ boxes, int nboxes, int nsets) {
   constexpr int BK = 16;
   constexpr int NT = 64;  // targets per tile (4x4x4 box)
@@ -149,13 +148,12 @@ __global__ void __launch_bounds__((64 / TM) * (R / TN)) m2l_simt_kernel(const T 
 #pragma unroll
     for (int y = 0; y < TN; ++y) {
       const int i = og + (R / TN) * y;
-      if (accumulate) dst[i] += acc[x][y];
-      else dst[i] = acc[x][y];
+      dst[i] = acc[x][y];
     }
   }
 }
 
-int m2l_simt_tiles(int level) {
+static int m2l_simt_tiles(int level) {
   const int P = 1 << (level - 1);
   const int bw = P < 4 ? P : 4;
   const int nbox = P / bw;
@@ -174,13 +172,11 @@ __global__ void simt_sum_parts_kernel(int64_t count, int ng, const T *__restrict
 
 // ngroups > 1 splits the 189 offsets over that many CTAs per target tile; their partials go
 // to `part` (part_elems elements) and are summed in a fixed order (groups are reduced to
-// fit the scratch; accumulate then does not apply). With a list of nboxes 2 x 2 x 2 blocks of
-// parent cells (set, x0, y0, z0) only their targets are computed, in one group, and the rest
-// of Lout is left as it is.
-template <typename T>
-int launch_m2l_simt(int r, const T *M, const T *Ert, T *Lout, int level, int j0, int j1, const int4 *offs,
-                    int accumulate, cudaStream_t s, int nsets, int ngroups, T *part, int64_t part_elems,
-                    const int4 *boxes, int nboxes) {
+// fit the scratch). With a list of nboxes 2 x 2 x 2 blocks of parent cells (set, x0, y0, z0) only
+// their targets are computed, in one group, and the rest of Lout is left as it is.
+int launch_m2l_simt(int r, const float *M, const float *Ert, float *Lout, int level, int j0, int j1, const int4 *offs,
+                    cudaStream_t s, int nsets, int ngroups, float *part, int64_t part_elems, const int4 *boxes, int nboxes) {
+  if (r != 256) return bbfmm_set_error(BBFMM_ERR_UNSUPPORTED, "CUDA-core M2L is built for r = 256");
   const int64_t P = (int64_t)1 << (level - 1);
   if (boxes && (nboxes < 0 || nboxes > nsets * P * P * P / 8 || P < 2))
     return bbfmm_set_error(BBFMM_ERR_ARG, "box list longer than the level");
@@ -193,29 +189,15 @@ int launch_m2l_simt(int r, const T *M, const T *Ert, T *Lout, int level, int j0,
   if (!part || boxes) ng = 1;
   else if ((int64_t)ng * count > part_elems) ng = (int)(part_elems / count);
   if (ng < 1) ng = 1;
-  T *dst = ng > 1 ? part : Lout;
-  const dim3 grid(tiles, ng);
-  if (r == 256) {
-    m2l_simt_kernel<T, 256, 8, 8><<<grid, 256, 0, s>>>(M, Ert, dst, level, j0, j1, offs, ng > 1 ? 0 : accumulate,
-                                                       boxes, nboxes, nsets);
-  } else if (r == 32) {
-    m2l_simt_kernel<T, 32, 4, 4><<<grid, 128, 0, s>>>(M, Ert, dst, level, j0, j1, offs, ng > 1 ? 0 : accumulate,
-                                                     boxes, nboxes, nsets);
-  } else {
-    return bbfmm_set_error(BBFMM_ERR_UNSUPPORTED, "M2L rank must be 32 or 256 (n = 4 or 8)");
-  }
+  m2l_simt_kernel<float, 256, 8, 8><<<dim3(tiles, ng), 256, 0, s>>>(M, Ert, ng > 1 ? part : Lout, level, j0, j1, offs, boxes,
+                                                                   nboxes, nsets);
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess || ng == 1) return bbfmm_set_cuda_error(e, "m2l_simt", __FILE__, __LINE__);
   int sg = (int)((count + 255) / 256);
   if (sg > 148 * 32) sg = 148 * 32;
-  simt_sum_parts_kernel<T><<<sg, 256, 0, s>>>(count, ng, part, Lout);
+  simt_sum_parts_kernel<float><<<sg, 256, 0, s>>>(count, ng, part, Lout);
   return bbfmm_set_cuda_error(cudaGetLastError(), "m2l_simt parts", __FILE__, __LINE__);
 }
-
-template int launch_m2l_simt<double>(int, const double *, const double *, double *, int, int, int, const int4 *, int,
-                                     cudaStream_t, int, int, double *, int64_t, const int4 *, int);
-template int launch_m2l_simt<float>(int, const float *, const float *, float *, int, int, int, const int4 *, int,
-                                    cudaStream_t, int, int, float *, int64_t, const int4 *, int);
 
 // Host table of the 189 offsets of each sibling class, as (k, vx, vy, vz).
 void build_offset_table(int *out /* 8*189*4 */) {

@@ -136,6 +136,11 @@ int Solver<T>::set_operators(const T *U, const T *E) {
     BBFMM_CUDA_OK(cudaMemcpy(Bup, bup.data(), sizeof(T) * bup.size(), cudaMemcpyHostToDevice));
     BBFMM_CUDA_OK(cudaMemcpy(Bdn, bdn.data(), sizeof(T) * bdn.size(), cudaMemcpyHostToDevice));
     BBFMM_CUDA_OK(cudaDeviceSynchronize());
+    if (r == 32) {
+      if (!P32) TRY(dalloc(&P32, 2 * (size_t)n3 * r));
+      TRY(r32_pack_proj<T>(Bup, Bdn, P32, stream));
+      BBFMM_CUDA_OK(cudaStreamSynchronize(stream));
+    }
     if (mode == MODE_MIXED && r == 256 && sizeof(T) == 8) {
       std::vector<T> blead((size_t)n3 * PROJ_LEAD);
       for (int l = 0; l < n3; ++l)
@@ -161,6 +166,11 @@ int Solver<T>::set_operators(const T *U, const T *E) {
   BBFMM_CUDA_OK(cudaMemcpy(Ert, ert.data(), sizeof(T) * ert.size(), cudaMemcpyHostToDevice));
   BBFMM_CUDA_OK(cudaMemcpy(Ecol, E, sizeof(T) * ert.size(), cudaMemcpyHostToDevice));
   BBFMM_CUDA_OK(cudaDeviceSynchronize());
+  if (r == 32) {
+    if (!B32) TRY(dalloc(&B32, r32_pack_doubles()));
+    TRY(r32_pack<T>(Ecol, B32, stream));
+    BBFMM_CUDA_OK(cudaStreamSynchronize(stream));
+  }
   if (mode == MODE_MIXED && r == 256) {  // r = 32 (n = 4): the M2L stays in FP64 on CUDA cores
     if (!tc_supported()) return bbfmm_set_error(BBFMM_ERR_UNSUPPORTED, "mixed mode needs an sm_100 GPU");
     if (tcops) tc_free_operators(tcops);
@@ -177,7 +187,7 @@ int Solver<T>::share_operators(const Solver<T> &o) {
     return bbfmm_set_error(BBFMM_ERR_ARG, "operators can only be shared between solvers of the same n and mode");
   if (!o.Ert || !o.kw) return bbfmm_set_error(BBFMM_ERR_STATE, "the sharing solver has no operators");
   if (own_ops) {
-    void *mine[] = {tkz, cw, kw, Ert, Ecol, Bup, Bdn, kwcol, Bup_lead};
+    void *mine[] = {tkz, cw, kw, Ert, Ecol, Bup, Bdn, kwcol, Bup_lead, B32, P32};
     for (void *p : mine)
       if (p) cudaFree(p);
     if (tcops) tc_free_operators(tcops);
@@ -186,6 +196,8 @@ int Solver<T>::share_operators(const Solver<T> &o) {
   tkz = o.tkz; cw = o.cw; kw = o.kw; Ert = o.Ert; Ecol = o.Ecol; Bup = o.Bup; Bdn = o.Bdn; kwcol = o.kwcol;
   tcops = o.tcops;
   tcproj = o.tcproj;
+  B32 = o.B32;
+  P32 = o.P32;
   Bup_lead = o.Bup_lead;
   own_ops = false;
   return BBFMM_OK;
@@ -199,7 +211,7 @@ int Solver<T>::alloc_partials() {
     for (int l = BBFMM_MINLEV; l <= maxlev; ++l) {
       const bool tc = tc_m2l(l);
       if (tc) continue;
-      const int g = tune.m2l_groups[l] > 0 ? tune.m2l_groups[l] : dmma_default_groups(l, nsets);
+      const int g = m2l_groups(l);
       const int64_t e = dmma_part_elems(l, nsets, g, r);
       if (e > need) need = e;
     }
@@ -442,19 +454,24 @@ int Solver<T>::upward(const void *q_dev, int q_is_double) {
   return BBFMM_OK;
 }
 
-// FP64 with r = 256 runs on the FP64 tensor path (DMMA); FP32 and r = 32 on CUDA cores.
+// r = 32 runs on the FP64 tensor path in either precision, r = 256 there in FP64 and on CUDA cores
+// in FP32.
 template <typename T>
 int Solver<T>::m2l_fp(const T *Ml, int level, int j0, int j1, int ni, const int4 *boxes, int nboxes) {
+  if (r == 32)
+    return launch_m2l_r32<T>(B32, Ml, Lbuf, level, offs, Lpart, Lpart_elems, stream, nsets, m2l_groups(level), boxes,
+                             nboxes);
   if (sizeof(T) == 8 && r == 256)
     return launch_m2l_dmma(r, (const double *)Ml, (const double *)Ecol, (double *)Lbuf, level, j0, j1, ni, offs,
                            (double *)Lpart, Lpart_elems, stream, nsets, tune.m2l_groups[level], boxes, nboxes);
-  // the SIMT kernel writes all r outputs; in the rank mode (ni = rk()) the outputs i >= rank
+  // FP32 at r = 256 writes all r outputs; in the rank mode (ni = rk()) the outputs i >= rank
   // of the zero-padded operators come out as zeros, so only other partial ranges are refused
   if (ni != r && ni != rk())
     return bbfmm_set_error(BBFMM_ERR_UNSUPPORTED, "partial output range needs the FP64 r = 256 path");
-  const int g = tune.m2l_groups[level] > 0 ? tune.m2l_groups[level] : dmma_default_groups(level, nsets);
-  return launch_m2l_simt<T>(r, Ml, Ert, Lbuf, level, j0, j1, offs, 0, stream, nsets, g, Lpart, Lpart_elems, boxes,
-                            nboxes);
+  if constexpr (sizeof(T) == 4)
+    return launch_m2l_simt(r, Ml, Ert, Lbuf, level, j0, j1, offs, stream, nsets, m2l_groups(level), Lpart, Lpart_elems,
+                           boxes, nboxes);
+  return bbfmm_set_error(BBFMM_ERR_UNSUPPORTED, "M2L rank must be 32 or 256 (n = 4 or 8)");
 }
 
 template <typename T>
@@ -474,6 +491,7 @@ template <typename T>
 int Solver<T>::proj_up(int64_t rows, const T *S_rows, int level, int64_t row0, bool presplit,
                        const int64_t *rowlist) {
   T *Mdst = Mall + Moff[level];
+  if (r == 32) return launch_proj_r32<T>(true, rows, S_rows, P32, nullptr, (T)1, Mdst, level, row0, rowlist, stream);
   if (!proj_tc() || rows > Ssplit_rows)
     return proj(rows, n3, r, S_rows, Bup, nullptr, (T)1, Mdst, level, MAP_OUT_CPG, row0, 0, rowlist);
   // the tensor cores write all r columns (zero for j < PROJ_LEAD: those operator rows are
@@ -492,6 +510,7 @@ int Solver<T>::proj_down(int level, int64_t rows, int64_t row0, T *F_rows, bool 
   // (1/L_l)^homogen in T, as the reference's POW(iL, homogen) (anotherFMMInteraction.c:7545-7549)
   const T iL = (T)1 / cell_length<T>(level, (T)L);
   const T scale = homogen == 1 ? iL : (T)std::pow(iL, (T)homogen);
+  if (r == 32) return launch_proj_r32<T>(false, rows, Lbuf, P32, kw, scale, F_rows, level, row0, rowlist, stream);
   if (!proj_tc() || rows > Lsplit_rows)  // contraction over the effective rank (j < rk())
     return proj(rows, rk(), n3, Lbuf, Bdn, kw, scale, F_rows, level, MAP_IN_CPG, row0, r, rowlist);
   // components j < 16 in FP64 and the rest as split-BF16 tensor-core products, one pass
@@ -587,7 +606,7 @@ int Solver<T>::m2l_post(int l) {
       mark(ST_M2L, 1);
     } else {
       TRY(m2l_fp(Ml, l, 0, rk(), rk()));
-      int g = tune.m2l_groups[l] > 0 ? tune.m2l_groups[l] : dmma_default_groups(l, nsets);
+      int g = m2l_groups(l);
       if ((int64_t)g * cells(l) * r > Lpart_elems) g = 1;
       mark(ST_M2L, g > 1 ? 2 : 1);  // groups add the partial sum
     }
@@ -1171,7 +1190,7 @@ void Solver<T>::release() {
   for (void *p : ptrs)
     if (p) cudaFree(p);
   if (own_ops) {
-    void *ops[] = {tkz, cw, kw, Ert, Ecol, Bup, Bdn, kwcol, Bup_lead};
+    void *ops[] = {tkz, cw, kw, Ert, Ecol, Bup, Bdn, kwcol, Bup_lead, B32, P32};
     for (void *p : ops)
       if (p) cudaFree(p);
     if (tcops) tc_free_operators(tcops);

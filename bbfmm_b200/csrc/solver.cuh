@@ -66,7 +66,13 @@ int launch_near2(int mode, int N, const void *pos4, const int *leaf_start, int m
 int pass_status(int clear);  // the passes' bounded waits (L2P leaf copies)
 template <typename T> int launch_l2p_field(int n, const T *pos4, const int *leaf_start, int maxlev, T L, const Tables &t, const T *F, T *pot, T *fld, cudaStream_t s, int nsets = 1, int64_t first = 0, int64_t count = -1, const int64_t *rows = nullptr, const HeavyLeaves &heavy = HeavyLeaves());
 template <typename T, typename TO> int launch_scatter_field(int N, const int *perm, const T *pot, const T *fld, TO *pot_out, TO *fld_out, cudaStream_t s);
-template <typename T> int launch_m2l_simt(int r, const T *M, const T *Ert, T *Lout, int level, int j0, int j1, const int4 *offs, int accumulate, cudaStream_t s, int nsets = 1, int ngroups = 1, T *part = nullptr, int64_t part_elems = 0, const int4 *boxes = nullptr, int nboxes = 0);
+size_t r32_pack_doubles();
+template <typename T> int r32_pack(const T *Ecol, double *Bpack, cudaStream_t s);
+int r32_default_groups(int level, int nsets);
+template <typename T> int r32_pack_proj(const T *Bup, const T *Bdn, double *frag, cudaStream_t s);
+template <typename T> int launch_proj_r32(bool up, int64_t rows, const T *A, const double *frag, const T *cs, T scale, T *C, int level, int64_t row0, const int64_t *rowlist, cudaStream_t s);
+template <typename T> int launch_m2l_r32(const double *Bpack, const T *M, T *Lout, int level, const int4 *offs, T *part, int64_t part_elems, cudaStream_t s, int nsets = 1, int ngroups = 0, const int4 *boxes = nullptr, int nboxes = 0);
+int launch_m2l_simt(int r, const float *M, const float *Ert, float *Lout, int level, int j0, int j1, const int4 *offs, cudaStream_t s, int nsets = 1, int ngroups = 1, float *part = nullptr, int64_t part_elems = 0, const int4 *boxes = nullptr, int nboxes = 0);
 void build_offset_table(int *out);
 constexpr int DMMA_PARTS = 21;  // most offset groups of the FP64 M2L (189 = 9 x 21)
 int launch_m2l_dmma(int r, const double *M, const double *Ecol, double *Lout, int level, int j0, int j1, int ni,
@@ -203,6 +209,11 @@ struct Solver {
   T *Bup = nullptr;  // [n3][r]  Kweights[l] U(l, i)
   T *Bdn = nullptr;  // [r][n3]  U(l, j)
   T *kwcol = nullptr;
+  double *B32 = nullptr, *P32 = nullptr;  // r = 32: operators and projections in fragment order
+  int m2l_groups(int l) const {  // offset groups of the level's FP64 / FP32 M2L
+    if (tune.m2l_groups[l] > 0) return tune.m2l_groups[l];
+    return r == 32 ? r32_default_groups(l, nsets) : dmma_default_groups(l, nsets);
+  }
   int4 *offs = nullptr;
   void *tcops = nullptr;  // mixed mode: split operators for the tensor-core kernel
   // mixed mode, n = 8: projections with the leading PROJ_LEAD components in FP64 and the rest
