@@ -625,80 +625,6 @@ __global__ void __launch_bounds__(128, 4) l2p_kernel(const T *__restrict__ pos4,
   });
 }
 
-// --------------------------------------------------------------- projections (GEMM)
-// C[out_row(m)][0:N] = scale * cs[0:N] o sum_k A[in_row(m)][k] B[k][0:N] for m < M,
-// where rows are mapped between Morton and cpg order at the given level.
-// A may be the sum of two sources (T and float) for the split M2L output.
-// Register-blocked SIMT GEMM: CTA tile 128 x BN, K-chunks of 16, 256 threads.
-// Local row m of a slab starting at cell row0: its cpg index when `which` is the mapped
-// side, else m itself.
-__device__ __forceinline__ int64_t map_row(int64_t m, int64_t row0, const int64_t *rows, int level, int which,
-                                           int mode) {
-  return mode == which ? morton_to_cpg_row(pass_cell(rows, row0, m), level) : m;
-}
-
-template <typename T, int BN>
-__global__ void __launch_bounds__(256) proj_gemm_kernel(int64_t M, int K, int N, const T *__restrict__ A,
-                                                        const float *__restrict__ A2, const T *__restrict__ B,
-                                                        const T *__restrict__ cs, T scale, T *__restrict__ C,
-                                                        int level, int mapmode, int64_t row0, int ldc, int lda,
-                                                        const int64_t *__restrict__ rows) {
-  constexpr int BM = 128, BK = 16, TN = BN / 16;
-  __shared__ T sa[BK][BM + 1];
-  __shared__ T sb[BK][BN];
-  const int tx = threadIdx.x % 16, ty = threadIdx.x / 16;
-  const int64_t m0 = (int64_t)blockIdx.x * BM;
-  const int n0 = blockIdx.y * BN;
-  T acc[8][TN];
-#pragma unroll
-  for (int i = 0; i < 8; ++i)
-#pragma unroll
-    for (int j = 0; j < TN; ++j) acc[i][j] = 0;
-  // each thread loads 8 A elements (rows) per chunk
-  for (int k0 = 0; k0 < K; k0 += BK) {
-    for (int e = threadIdx.x; e < BM * BK; e += 256) {
-      const int r = e / BK, c = e % BK;
-      const int64_t m = m0 + r;
-      T v = 0;
-      if (m < M && k0 + c < K) {
-        const int64_t ar = map_row(m, row0, rows, level, MAP_IN_CPG, mapmode);
-        v = A[ar * lda + k0 + c];
-        if (A2) v += (T)A2[ar * lda + k0 + c];
-      }
-      sa[c][r] = v;
-    }
-    for (int e = threadIdx.x; e < BK * BN; e += 256) {
-      const int r = e / BN, c = e % BN;
-      sb[r][c] = (k0 + r < K && n0 + c < N) ? B[(int64_t)(k0 + r) * N + n0 + c] : (T)0;
-    }
-    __syncthreads();
-#pragma unroll
-    for (int k = 0; k < BK; ++k) {
-      T a[8], b[TN];
-#pragma unroll
-      for (int i = 0; i < 8; ++i) a[i] = sa[k][ty * 8 + i];
-#pragma unroll
-      for (int j = 0; j < TN; ++j) b[j] = sb[k][tx + 16 * j];
-#pragma unroll
-      for (int i = 0; i < 8; ++i)
-#pragma unroll
-        for (int j = 0; j < TN; ++j) acc[i][j] += a[i] * b[j];
-    }
-    __syncthreads();
-  }
-#pragma unroll
-  for (int i = 0; i < 8; ++i) {
-    const int64_t m = m0 + ty * 8 + i;
-    if (m >= M) continue;
-    const int64_t cr = map_row(m, row0, rows, level, MAP_OUT_CPG, mapmode);
-#pragma unroll
-    for (int j = 0; j < TN; ++j) {
-      const int n = n0 + tx + 16 * j;
-      if (n < N) C[cr * ldc + n] = scale * (cs ? cs[n] : (T)1) * acc[i][j];
-    }
-  }
-}
-
 // ----------------------------------------------------------------- permutations
 template <typename T, typename TI>
 __global__ void gather_pos4_kernel(int N, const int *__restrict__ perm, const TI *__restrict__ xyz,
@@ -856,24 +782,6 @@ int launch_l2p(int n, const T *pos4, const int *leaf_start, int maxlev, T L, con
   return bbfmm_set_cuda_error(cudaGetLastError(), "l2p", __FILE__, __LINE__);
 }
 
-template <typename T>
-int launch_proj(int64_t M, int K, int N, const T *A, const float *A2, const T *B, const T *cs, T scale, T *C,
-                int level, int mapmode, cudaStream_t s, int64_t row0, int ldc, int lda, const int64_t *rows) {
-  if (M <= 0) return BBFMM_OK;
-  if (ldc <= 0) ldc = N;
-  if (lda <= 0) lda = K;
-  if (N >= 64) {
-    dim3 grid((unsigned)((M + 127) / 128), (unsigned)((N + 63) / 64));
-    proj_gemm_kernel<T, 64><<<grid, 256, 0, s>>>(M, K, N, A, A2, B, cs, scale, C, level, mapmode, row0, ldc, lda,
-                                                 rows);
-  } else {
-    dim3 grid((unsigned)((M + 127) / 128), (unsigned)((N + 31) / 32));
-    proj_gemm_kernel<T, 32><<<grid, 256, 0, s>>>(M, K, N, A, A2, B, cs, scale, C, level, mapmode, row0, ldc, lda,
-                                                 rows);
-  }
-  return bbfmm_set_cuda_error(cudaGetLastError(), "proj", __FILE__, __LINE__);
-}
-
 template <typename T, typename TI>
 int launch_gather(int N, const int *perm, const TI *xyz, const TI *q, T *pos4, cudaStream_t s) {
   if (N <= 0) return BBFMM_OK;
@@ -901,8 +809,6 @@ int launch_morton_cpg(int level, int r, const T *src, T *dst, int inverse, cudaS
   template int launch_l2l<T>(int, const T *, T *, int, const Tables &, cudaStream_t, int, int64_t, int64_t); \
   template int launch_l2p<T>(int, const T *, const int *, int, T, const Tables &, const T *, T *,          \
                              cudaStream_t, int, int64_t, int64_t, const int64_t *, const HeavyLeaves &);    \
-  template int launch_proj<T>(int64_t, int, int, const T *, const float *, const T *, const T *, T, T *,   \
-                              int, int, cudaStream_t, int64_t, int, int, const int64_t *);                 \
   template int launch_morton_cpg<T>(int, int, const T *, T *, int, cudaStream_t);
 INST(float)
 INST(double)

@@ -1,21 +1,27 @@
-// FP64 U-projections around M2L on the FP64 tensor path (mma.sync m8n8k4 f64):
+// U-projections around M2L at r = 256 on the FP64 tensor path (FP32 operands are widened as they
+// leave shared memory) (mma.sync m8n8k4 f64):
 //   up   : M[cpg(m)][i] = sum_l S[m][l] (Kweights[l] U(l, i))           (P2M/M2M -> M2L)
 //   down : F[m][l] = (1/L_l) Kweights[l] sum_j U(l, j) L[cpg(m)][j]      (M2L -> L2L/L2P)
 // (anotherUpwardPass.c:311-324 with atransx.c:48-86; auxAnotherFMMInteraction.c:398-416).
 // C[out(m)][n] = scale * cs[n] * sum_k A[in(m)][k] B[k][n] with rows remapped between
-// Morton and cpg order. CTA tile 64 rows x 256 columns, K-chunks of 16 double-buffered
-// with cp.async, 8 warps in a 2 x 4 grid of 32 x 64 warp tiles.
+// Morton and cpg order. CTA tile 64 rows x BN columns (256 or 64), K-chunks of 16 in a
+// four-stage cp.async ring, 8 warps in a 2 x 4 grid of 32 x BN / 4 warp tiles.
 #include "common.cuh"
 
 namespace bbfmm {
 
 namespace pj {
 
-constexpr int BM = 64, BN = 256, BK = 16;
+constexpr int BM = 64, BK = 16;
 constexpr int AST = BK + 4;   // A stored [row][k]: fragment reads hit distinct banks
-constexpr int BST = BN + 4;   // B stored [k][n]
-constexpr int STAGE_DOUBLES = BM * AST + BK * BST;
-constexpr int SMEM_BYTES = 2 * STAGE_DOUBLES * 8;
+// B stored [k][n], rows BN + 4 doubles or BN + 8 floats apart
+template <typename T>
+constexpr int bst(int BN) { return BN + (sizeof(T) == 8 ? 4 : 8); }
+template <typename T>
+constexpr int stage_elems(int BN) { return BM * AST + BK * bst<T>(BN); }
+constexpr int STAGES = 4;     // three K-chunks in flight while one is contracted, one barrier a chunk
+template <typename T>
+constexpr int smem_bytes(int BN) { return STAGES * stage_elems<T>(BN) * (int)sizeof(T); }
 
 __device__ __forceinline__ void cp_async16(uint32_t dst, const void *src, bool valid) {
   const int n = valid ? 16 : 0;
@@ -36,12 +42,17 @@ __device__ __forceinline__ int64_t remap(int64_t m, int64_t row0, const int64_t 
   return to_cpg ? morton_to_cpg_row(pass_cell(rows, row0, m), level) : m;
 }
 
-__global__ void __launch_bounds__(256, 1) proj_dmma_kernel(int64_t M, int K, int N, const double *__restrict__ A,
-                                                           const double *__restrict__ B,
-                                                           const double *__restrict__ cs, double scale,
-                                                           double *__restrict__ C, int level, int mapmode,
+// BN columns a CTA: 256 where the row tiles alone fill the SMs, 64 for the few rows of the upper
+// levels (four times the CTAs, each with a quarter of the work between its barriers).
+template <typename T, int BN>
+__global__ void __launch_bounds__(256, 1) proj_dmma_kernel(int64_t M, int K, int N, const T *__restrict__ A,
+                                                           const T *__restrict__ B,
+                                                           const T *__restrict__ cs, T scale,
+                                                           T *__restrict__ C, int level, int mapmode,
                                                            int64_t row0, int lda, const int64_t *__restrict__ rows) {
-  extern __shared__ __align__(16) double smem[];
+  constexpr int BST = bst<T>(BN), STAGE = stage_elems<T>(BN), V = 16 / (int)sizeof(T), WN = BN / 4, NF = WN / 8;  // columns, fragments a warp
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  T *smem = reinterpret_cast<T *>(smem_raw);
   __shared__ int64_t arow[BM];
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int wm = warp & 1, wn = warp >> 1;
@@ -55,65 +66,67 @@ __global__ void __launch_bounds__(256, 1) proj_dmma_kernel(int64_t M, int K, int
   }
   __syncthreads();
 
-  auto issue = [&](int kc, int buf) {
-    const uint32_t sa = sbase + (uint32_t)(buf * STAGE_DOUBLES) * 8u;
-    const uint32_t sb = sa + (uint32_t)(BM * AST) * 8u;
-    const int k0 = kc * BK;
-    for (int e = tid; e < BM * (BK / 2); e += 256) {  // 64 rows x 8 pairs
-      const int row = e / (BK / 2), k2 = (e % (BK / 2)) * 2;
-      const int64_t ar = arow[row];
-      const double *src = ar >= 0 ? A + ar * lda + k0 + k2 : A;
-      cp_async16(sa + (uint32_t)(row * AST + k2) * 8u, src, ar >= 0);
+  auto issue = [&](int kc) {
+    if (kc >= nk) {  // an empty group keeps the wait counts uniform
+      cp_commit();
+      return;
     }
-    for (int e = tid; e < BK * (BN / 2); e += 256) {  // 16 rows x 128 pairs
-      const int k = e / (BN / 2), n2 = (e % (BN / 2)) * 2;
-      cp_async16(sb + (uint32_t)(k * BST + n2) * 8u, B + (int64_t)(k0 + k) * N + n0 + n2, true);
+    const uint32_t sa = sbase + (uint32_t)((kc % STAGES) * STAGE * sizeof(T));
+    const uint32_t sb = sa + (uint32_t)(BM * AST * sizeof(T));
+    const int k0 = kc * BK;
+    for (int e = tid; e < BM * (BK / V); e += 256) {  // V values a copy
+      const int row = e / (BK / V), kv = (e % (BK / V)) * V;
+      const int64_t ar = arow[row];
+      const T *src = ar >= 0 ? A + ar * lda + k0 + kv : A;
+      cp_async16(sa + (uint32_t)((row * AST + kv) * sizeof(T)), src, ar >= 0);
+    }
+    for (int e = tid; e < BK * (BN / V); e += 256) {
+      const int k = e / (BN / V), nv = (e % (BN / V)) * V;
+      cp_async16(sb + (uint32_t)((k * BST + nv) * sizeof(T)), B + (int64_t)(k0 + k) * N + n0 + nv, true);
     }
     cp_commit();
   };
 
-  double acc[4][8][2];
+  double acc[4][NF][2];
 #pragma unroll
   for (int a = 0; a < 4; ++a)
 #pragma unroll
-    for (int b = 0; b < 8; ++b) acc[a][b][0] = acc[a][b][1] = 0.0;
-  issue(0, 0);
+    for (int b = 0; b < NF; ++b) acc[a][b][0] = acc[a][b][1] = 0.0;
+#pragma unroll
+  for (int kc = 0; kc < STAGES - 1; ++kc) issue(kc);
   for (int kc = 0; kc < nk; ++kc) {
-    const int buf = kc & 1;
-    if (kc + 1 < nk) {
-      issue(kc + 1, buf ^ 1);
-      cp_wait_one();
-    } else {
-      cp_wait_all();
-    }
-    __syncthreads();
-    const double *As = smem + buf * STAGE_DOUBLES;
-    const double *Bs = As + BM * AST;
+    asm volatile("cp.async.wait_group %0;" ::"n"(STAGES - 2) : "memory");
+    __syncthreads();  // chunk kc has landed, and every warp is done with chunk kc - 1
+    issue(kc + STAGES - 1);
+    const int buf = kc % STAGES;
+    const T *As = smem + buf * STAGE;
+    const T *Bs = As + BM * AST;
 #pragma unroll
     for (int ks = 0; ks < BK / 4; ++ks) {
       const int k = ks * 4 + (lane & 3);
-      double af[4], bf[8];
+      double af[4], bf[NF];
 #pragma unroll
-      for (int mf = 0; mf < 4; ++mf) af[mf] = As[(wm * 32 + mf * 8 + (lane >> 2)) * AST + k];
+      for (int mf = 0; mf < 4; ++mf) af[mf] = (double)As[(wm * 32 + mf * 8 + (lane >> 2)) * AST + k];
 #pragma unroll
-      for (int nf = 0; nf < 8; ++nf) bf[nf] = Bs[k * BST + wn * 64 + nf * 8 + (lane >> 2)];
+      for (int nf = 0; nf < NF; ++nf) bf[nf] = (double)Bs[k * BST + wn * WN + nf * 8 + (lane >> 2)];
 #pragma unroll
       for (int mf = 0; mf < 4; ++mf)
 #pragma unroll
-        for (int nf = 0; nf < 8; ++nf) dmma(acc[mf][nf][0], acc[mf][nf][1], af[mf], bf[nf]);
+        for (int nf = 0; nf < NF; ++nf) dmma(acc[mf][nf][0], acc[mf][nf][1], af[mf], bf[nf]);
     }
-    __syncthreads();
   }
+  cp_wait_all();
 #pragma unroll
   for (int mf = 0; mf < 4; ++mf) {
     const int64_t m = m0 + wm * 32 + mf * 8 + (lane >> 2);
     if (m >= M) continue;
-    double *dst = C + remap(m, row0, rows, level, mapmode == MAP_OUT_CPG) * N;
+    T *dst = C + remap(m, row0, rows, level, mapmode == MAP_OUT_CPG) * N;
 #pragma unroll
-    for (int nf = 0; nf < 8; ++nf) {
-      const int n = n0 + wn * 64 + nf * 8 + 2 * (lane & 3);
-      const double c0 = cs ? scale * cs[n] : scale, c1 = cs ? scale * cs[n + 1] : scale;
-      *reinterpret_cast<double2 *>(dst + n) = make_double2(c0 * acc[mf][nf][0], c1 * acc[mf][nf][1]);
+    for (int nf = 0; nf < NF; ++nf) {
+      const int n = n0 + wn * WN + nf * 8 + 2 * (lane & 3);
+      const T c0 = cs ? scale * cs[n] : scale, c1 = cs ? scale * cs[n + 1] : scale;
+      dst[n] = (T)(c0 * acc[mf][nf][0]);
+      dst[n + 1] = (T)(c1 * acc[mf][nf][1]);
     }
   }
 }
@@ -214,24 +227,32 @@ int launch_proj_narrow(int64_t M, int K, const double *A, const double *B, doubl
   return bbfmm_set_cuda_error(cudaGetLastError(), "proj_narrow", __FILE__, __LINE__);
 }
 
-// Returns BBFMM_ERR_UNSUPPORTED (without recording an error) when the shape does not fit
-// the tile (K % 16, N % 256); the caller then uses the CUDA-core GEMM.
-int launch_proj_dmma(int64_t M, int K, int N, const double *A, const double *B, const double *cs, double scale,
-                     double *C, int level, int mapmode, cudaStream_t s, int64_t row0, int lda,
-                     const int64_t *rows) {
-  if (K % pj::BK || N % pj::BN) return BBFMM_ERR_UNSUPPORTED;
+template <typename T, int BN>
+static int proj_dmma_attr() {  // dynamic shared memory above 48 KB needs the opt-in
+  return bbfmm_set_cuda_error(cudaFuncSetAttribute(pj::proj_dmma_kernel<T, BN>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                                   pj::smem_bytes<T>(BN)),
+                              "proj_dmma smem attribute", __FILE__, __LINE__);
+}
+
+template <typename T>
+int launch_proj_dmma(int64_t M, int K, int N, const T *A, const T *B, const T *cs, T scale, T *C, int level, int mapmode,
+                     cudaStream_t s, int64_t row0, int lda, const int64_t *rows) {
+  if (K % pj::BK || N % 256) return bbfmm_set_error(BBFMM_ERR_UNSUPPORTED, "projection: K % 16 and N % 256 must be 0");
   if (M <= 0) return BBFMM_OK;
-  static bool attr = false;
-  if (!attr) {
-    cudaError_t e =
-        cudaFuncSetAttribute(pj::proj_dmma_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, pj::SMEM_BYTES);
-    if (e != cudaSuccess) return bbfmm_set_cuda_error(e, "proj_dmma smem attribute", __FILE__, __LINE__);
-    attr = true;
-  }
-  dim3 grid((unsigned)((M + pj::BM - 1) / pj::BM), (unsigned)(N / pj::BN));
-  pj::proj_dmma_kernel<<<grid, 256, pj::SMEM_BYTES, s>>>(M, K, N, A, B, cs, scale, C, level, mapmode, row0,
-                                                          lda > 0 ? lda : K, rows);
+  static const int attr = proj_dmma_attr<T, 256>() | proj_dmma_attr<T, 64>();
+  if (attr) return BBFMM_ERR_CUDA;
+  const unsigned mt = (unsigned)((M + pj::BM - 1) / pj::BM);
+  if ((int64_t)mt * (N / 256) < 148)
+    pj::proj_dmma_kernel<T, 64><<<dim3(mt, (unsigned)(N / 64)), 256, pj::smem_bytes<T>(64), s>>>(
+        M, K, N, A, B, cs, scale, C, level, mapmode, row0, lda > 0 ? lda : K, rows);
+  else
+    pj::proj_dmma_kernel<T, 256><<<dim3(mt, (unsigned)(N / 256)), 256, pj::smem_bytes<T>(256), s>>>(
+        M, K, N, A, B, cs, scale, C, level, mapmode, row0, lda > 0 ? lda : K, rows);
   return bbfmm_set_cuda_error(cudaGetLastError(), "proj_dmma", __FILE__, __LINE__);
 }
+template int launch_proj_dmma<double>(int64_t, int, int, const double *, const double *, const double *, double, double *,
+                                      int, int, cudaStream_t, int64_t, int, const int64_t *);
+template int launch_proj_dmma<float>(int64_t, int, int, const float *, const float *, const float *, float, float *, int,
+                                     int, cudaStream_t, int64_t, int, const int64_t *);
 
 }  // namespace bbfmm

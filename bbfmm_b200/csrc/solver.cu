@@ -474,17 +474,6 @@ int Solver<T>::m2l_fp(const T *Ml, int level, int j0, int j1, int ni, const int4
   return bbfmm_set_error(BBFMM_ERR_UNSUPPORTED, "M2L rank must be 32 or 256 (n = 4 or 8)");
 }
 
-template <typename T>
-int Solver<T>::proj(int64_t Mrows, int K, int Ncols, const T *A, const T *B, const T *cs, T scale, T *C, int level,
-                    int mapmode, int64_t row0, int lda, const int64_t *rowlist) {
-  if (sizeof(T) == 8) {
-    int rc = launch_proj_dmma(Mrows, K, Ncols, (const double *)A, (const double *)B, (const double *)cs,
-                              (double)scale, (double *)C, level, mapmode, stream, row0, lda, rowlist);
-    if (rc != BBFMM_ERR_UNSUPPORTED) return rc;
-  }
-  return launch_proj<T>(Mrows, K, Ncols, A, nullptr, B, cs, scale, C, level, mapmode, stream, row0, 0, lda, rowlist);
-}
-
 // Up projection of `rows` S rows (Morton cells row0 .. of `level`) into the level's M (cpg).
 // Mixed mode: components j < PROJ_LEAD in FP64, the rest as split-BF16 tensor-core products.
 template <typename T>
@@ -493,7 +482,8 @@ int Solver<T>::proj_up(int64_t rows, const T *S_rows, int level, int64_t row0, b
   T *Mdst = Mall + Moff[level];
   if (r == 32) return launch_proj_r32<T>(true, rows, S_rows, P32, nullptr, (T)1, Mdst, level, row0, rowlist, stream);
   if (!proj_tc() || rows > Ssplit_rows)
-    return proj(rows, n3, r, S_rows, Bup, nullptr, (T)1, Mdst, level, MAP_OUT_CPG, row0, 0, rowlist);
+    return launch_proj_dmma<T>(rows, n3, r, S_rows, Bup, nullptr, (T)1, Mdst, level, MAP_OUT_CPG, stream, row0, 0,
+                               rowlist);
   // the tensor cores write all r columns (zero for j < PROJ_LEAD: those operator rows are
   // zero in the split copy), then the FP64 pass overwrites the leading columns
   if (!presplit) TRY(tc_split_rows(rows, n3, (const double *)S_rows, 0, level, row0, Ssplit, stream));
@@ -512,7 +502,8 @@ int Solver<T>::proj_down(int level, int64_t rows, int64_t row0, T *F_rows, bool 
   const T scale = homogen == 1 ? iL : (T)std::pow(iL, (T)homogen);
   if (r == 32) return launch_proj_r32<T>(false, rows, Lbuf, P32, kw, scale, F_rows, level, row0, rowlist, stream);
   if (!proj_tc() || rows > Lsplit_rows)  // contraction over the effective rank (j < rk())
-    return proj(rows, rk(), n3, Lbuf, Bdn, kw, scale, F_rows, level, MAP_IN_CPG, row0, r, rowlist);
+    return launch_proj_dmma<T>(rows, rk(), n3, Lbuf, Bdn, kw, scale, F_rows, level, MAP_IN_CPG, stream, row0, r,
+                               rowlist);
   // components j < 16 in FP64 and the rest as split-BF16 tensor-core products, one pass
   if (!presplit) TRY(tc_split_rows(rows, r, (const double *)Lbuf, 1, level, row0, Lsplit, stream, 16, rowlist));
   return launch_proj_down(tcproj, Lsplit, (const double *)Lbuf, rows, (double *)F_rows, level, row0,

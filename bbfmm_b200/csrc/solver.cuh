@@ -39,7 +39,6 @@ template <typename T> int launch_m2m(int n, const T *Sc, T *Sp, int level, const
 template <typename T> int launch_l2l(int n, const T *Fp, T *Fc, int level, const Tables &t, cudaStream_t s, int nsets = 1, int64_t first = 0, int64_t count = -1);
 template <typename T> int launch_l2p(int n, const T *pos4, const int *leaf_start, int maxlev, T L, const Tables &t, const T *F, T *phi, cudaStream_t s, int nsets = 1, int64_t first = 0, int64_t count = -1, const int64_t *rows = nullptr, const HeavyLeaves &heavy = HeavyLeaves());
 // rows are a slab of the level starting at cell row0 (the cpg side is indexed by level cell)
-template <typename T> int launch_proj(int64_t M, int K, int N, const T *A, const float *A2, const T *B, const T *cs, T scale, T *C, int level, int mapmode, cudaStream_t s, int64_t row0 = 0, int ldc = 0, int lda = 0, const int64_t *rows = nullptr);
 template <typename T, typename TI> int launch_gather(int N, const int *perm, const TI *xyz, const TI *q, T *pos4, cudaStream_t s);
 template <typename T> int launch_charges_of(int N, const T *pos4, T *q, cudaStream_t s);  // sorted charges
 template <typename T> int launch_add(int64_t n, const T *x, T *y, cudaStream_t s);        // y += x
@@ -80,9 +79,9 @@ int launch_m2l_dmma(int r, const double *M, const double *Ecol, double *Lout, in
                     int ngroups = 0, const int4 *boxes = nullptr, int nboxes = 0);
 int dmma_default_groups(int level, int nsets);
 int64_t dmma_part_elems(int level, int nsets, int groups, int r);
-int launch_proj_dmma(int64_t M, int K, int N, const double *A, const double *B, const double *cs, double scale,
-                     double *C, int level, int mapmode, cudaStream_t s, int64_t row0 = 0, int lda = 0,
-                     const int64_t *rows = nullptr);
+template <typename T>
+int launch_proj_dmma(int64_t M, int K, int N, const T *A, const T *B, const T *cs, T scale, T *C, int level, int mapmode,
+                     cudaStream_t s, int64_t row0 = 0, int lda = 0, const int64_t *rows = nullptr);
 // C[out(m)][0:32] = sum_k A[m][k] B[k][0:32] on the FP64 tensor path (B: K x 32 contiguous).
 int launch_proj_narrow(int64_t M, int K, const double *A, const double *B, double *C, int ldc, int level,
                        int mapmode, cudaStream_t s, int64_t row0, const int64_t *rows = nullptr);
@@ -356,8 +355,6 @@ struct Solver {
   int time_m2l(int level, int reps, float *ms);
   int m2l_fp(const T *Ml, int level, int j0, int j1, int ni,  // FP64 (DMMA) / FP32 (SIMT) M2L part
              const int4 *boxes = nullptr, int nboxes = 0);
-  int proj(int64_t M, int K, int N, const T *A, const T *B, const T *cs, T scale, T *C, int level, int mapmode,
-           int64_t row0 = 0, int lda = 0, const int64_t *rowlist = nullptr);
   void release();
 };
 
