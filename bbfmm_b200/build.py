@@ -32,6 +32,7 @@ UNITS = [
     ("m2l_r32.cu", [], "m2l_r32"),
     ("m2l_tc.cu", [], "m2l_tc"),
     ("m2l_dmma.cu", [], "m2l_dmma"),
+    ("m2l_sym.cu", [], "m2l_sym"),
     ("proj_dmma.cu", [], "proj_dmma"),
     ("direct.cu", [], "direct"),
     ("solver.cu", [], "solver"),

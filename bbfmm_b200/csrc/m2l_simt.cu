@@ -1,4 +1,5 @@
-// M2L on CUDA cores over the dense class-major grid of one level (FP32 at r = 256).
+// M2L on CUDA cores over the dense class-major grid of one level: FP32 at r = 256 for operators
+// without the mirror symmetry of m2l_sym.cu.
 //
 //   L(F) = sum_{S in IL(F)} E_{k(F,S)} M(S)     (m2l_kern_basic.cu:82-130 semantics,
 //                                                k from m2l_aux.c:1135-1191)

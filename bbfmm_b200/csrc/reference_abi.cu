@@ -71,6 +71,7 @@ static int order_of_rank(int r) { return r == 32 ? 4 : (r == 256 ? 8 : 0); }
 // Solver with the caller's (or our own) Chebyshev tables.
 template <typename T>
 int make_solver(Solver<T> &s, int n, int maxlev, double L0, const T *Tkz, const T *Cw, const T *Kw) {
+  s.fold = false;  // multipoles cross these entry points in the basis of the reference's operators
   int dev = 0;
   if (cudaGetDevice(&dev) != cudaSuccess) dev = 0;
   TRY(s.init(n, maxlev, L0, mode_of<T>(), 0, 0, dev, nullptr));

@@ -55,6 +55,17 @@ static int dalloc(T **p, size_t count) {
   return BBFMM_OK;
 }
 
+// dst[k][i][j] = src[k][j][i] for r x r blocks, 32 x 32 tiles through shared memory.
+template <typename T>
+__global__ void transpose_blocks_kernel(int r, const T *__restrict__ src, T *__restrict__ dst) {
+  __shared__ T t[32][33];
+  const int64_t b = (int64_t)blockIdx.z * r * r;
+  const int i0 = blockIdx.x * 32, j0 = blockIdx.y * 32;
+  for (int y = threadIdx.y; y < 32; y += 8) t[y][threadIdx.x] = src[b + (int64_t)(j0 + y) * r + i0 + threadIdx.x];
+  __syncthreads();
+  for (int y = threadIdx.y; y < 32; y += 8) dst[b + (int64_t)(i0 + y) * r + j0 + threadIdx.x] = t[threadIdx.x][y];
+}
+
 #define TRY(x)                       \
   do {                               \
     int rc__ = (x);                  \
@@ -154,22 +165,30 @@ int Solver<T>::set_operators(const T *U, const T *E) {
     }
   }
   if (!E) return BBFMM_OK;
-  std::vector<T> ert((size_t)BBFMM_NUM_OFFSETS * r * r);
-  for (int k = 0; k < BBFMM_NUM_OFFSETS; ++k)
-    for (int i = 0; i < r; ++i)
-      for (int j = 0; j < r; ++j)
-        ert[((size_t)k * r + i) * r + j] = E[((size_t)k * r + j) * r + i];
+  const size_t ne = (size_t)BBFMM_NUM_OFFSETS * r * r;
   if (!Ert) {
-    TRY(dalloc(&Ert, ert.size()));
-    TRY(dalloc(&Ecol, ert.size()));
+    TRY(dalloc(&Ert, ne));
+    TRY(dalloc(&Ecol, ne));
   }
-  BBFMM_CUDA_OK(cudaMemcpy(Ert, ert.data(), sizeof(T) * ert.size(), cudaMemcpyHostToDevice));
-  BBFMM_CUDA_OK(cudaMemcpy(Ecol, E, sizeof(T) * ert.size(), cudaMemcpyHostToDevice));
+  BBFMM_CUDA_OK(cudaMemcpy(Ecol, E, sizeof(T) * ne, cudaMemcpyHostToDevice));
   BBFMM_CUDA_OK(cudaDeviceSynchronize());
+  transpose_blocks_kernel<T><<<dim3(r / 32, r / 32, BBFMM_NUM_OFFSETS), dim3(32, 8), 0, stream>>>(r, Ecol, Ert);
+  BBFMM_CUDA_OK(cudaGetLastError());
+  BBFMM_CUDA_OK(cudaStreamSynchronize(stream));
   if (r == 32) {
     if (!B32) TRY(dalloc(&B32, r32_pack_doubles()));
     TRY(r32_pack<T>(Ecol, B32, stream));
     BBFMM_CUDA_OK(cudaStreamSynchronize(stream));
+  }
+  if (symops) sym_free(symops);
+  symops = nullptr;
+  if (fold && U && r == 256) {
+    if (!Bup_sym) {
+      TRY(dalloc(&Bup_sym, (size_t)n3 * r));
+      TRY(dalloc(&Bdn_sym, (size_t)r * n3));
+    }
+    // images of an operator agree to the rounding of its entries
+    TRY(sym_prepare<T>(n, r, U, Ecol, sizeof(T) == 8 ? 1e-13 : 4e-6, Bup, Bdn, Bup_sym, Bdn_sym, &symops, stream));
   }
   if (mode == MODE_MIXED && r == 256) {  // r = 32 (n = 4): the M2L stays in FP64 on CUDA cores
     if (!tc_supported()) return bbfmm_set_error(BBFMM_ERR_UNSUPPORTED, "mixed mode needs an sm_100 GPU");
@@ -187,17 +206,21 @@ int Solver<T>::share_operators(const Solver<T> &o) {
     return bbfmm_set_error(BBFMM_ERR_ARG, "operators can only be shared between solvers of the same n and mode");
   if (!o.Ert || !o.kw) return bbfmm_set_error(BBFMM_ERR_STATE, "the sharing solver has no operators");
   if (own_ops) {
-    void *mine[] = {tkz, cw, kw, Ert, Ecol, Bup, Bdn, kwcol, Bup_lead, B32, P32};
+    void *mine[] = {tkz, cw, kw, Ert, Ecol, Bup, Bdn, kwcol, Bup_lead, Bup_sym, Bdn_sym, B32, P32};
     for (void *p : mine)
       if (p) cudaFree(p);
     if (tcops) tc_free_operators(tcops);
     if (tcproj) tc_free_projections(tcproj);
+    if (symops) sym_free(symops);
   }
   tkz = o.tkz; cw = o.cw; kw = o.kw; Ert = o.Ert; Ecol = o.Ecol; Bup = o.Bup; Bdn = o.Bdn; kwcol = o.kwcol;
   tcops = o.tcops;
   tcproj = o.tcproj;
+  symops = o.symops;
   B32 = o.B32;
   P32 = o.P32;
+  Bup_sym = o.Bup_sym;
+  Bdn_sym = o.Bdn_sym;
   Bup_lead = o.Bup_lead;
   own_ops = false;
   return BBFMM_OK;
@@ -428,7 +451,7 @@ int Solver<T>::upward(const void *q_dev, int q_is_double) {
   for (int64_t a = 0; a < nl; a += sl) {
     const int64_t c = nl - a < sl ? nl - a : sl;
     // mixed mode: P2M also writes the BF16 split of S that the tensor-core up projection reads
-    void *sp = proj_tc() && c <= Ssplit_rows ? Ssplit : nullptr;
+    void *sp = proj_tc() && c <= Ssplit_rows && !sym_level(maxlev) ? Ssplit : nullptr;
     TRY(launch_p2m<T>(n, pos4, leaf_start, maxlev, (T)L, tb, Sl, stream, nsets, a, c, sp, lr ? lr + a : nullptr,
                       heavy_up));
     mark(ST_P2M, heavy_up.nitems > 0 ? 3 : 1);
@@ -454,13 +477,15 @@ int Solver<T>::upward(const void *q_dev, int q_is_double) {
   return BBFMM_OK;
 }
 
-// r = 32 runs on the FP64 tensor path in either precision, r = 256 there in FP64 and on CUDA cores
-// in FP32.
+// r = 32 and mirror-symmetric operators run on the FP64 tensor path in either precision, other
+// r = 256 operators there in FP64 and on CUDA cores in FP32.
 template <typename T>
 int Solver<T>::m2l_fp(const T *Ml, int level, int j0, int j1, int ni, const int4 *boxes, int nboxes) {
   if (r == 32)
     return launch_m2l_r32<T>(B32, Ml, Lbuf, level, offs, Lpart, Lpart_elems, stream, nsets, m2l_groups(level), boxes,
                              nboxes);
+  if (msym[level])
+    return launch_m2l_sym<T>(symops, Ml, Lbuf, level, Lpart, Lpart_elems, stream, nsets, m2l_groups(level), boxes, nboxes);
   if (sizeof(T) == 8 && r == 256)
     return launch_m2l_dmma(r, (const double *)Ml, (const double *)Ecol, (double *)Lbuf, level, j0, j1, ni, offs,
                            (double *)Lpart, Lpart_elems, stream, nsets, tune.m2l_groups[level], boxes, nboxes);
@@ -481,9 +506,10 @@ int Solver<T>::proj_up(int64_t rows, const T *S_rows, int level, int64_t row0, b
                        const int64_t *rowlist) {
   T *Mdst = Mall + Moff[level];
   if (r == 32) return launch_proj_r32<T>(true, rows, S_rows, P32, nullptr, (T)1, Mdst, level, row0, rowlist, stream);
-  if (!proj_tc() || rows > Ssplit_rows)
-    return launch_proj_dmma<T>(rows, n3, r, S_rows, Bup, nullptr, (T)1, Mdst, level, MAP_OUT_CPG, stream, row0, 0,
-                               rowlist);
+  msym[level] = sym_level(level);
+  if (!proj_tc() || rows > Ssplit_rows || msym[level])
+    return launch_proj_dmma<T>(rows, n3, r, S_rows, msym[level] ? Bup_sym : Bup, nullptr, (T)1, Mdst, level, MAP_OUT_CPG,
+                               stream, row0, 0, rowlist);
   // the tensor cores write all r columns (zero for j < PROJ_LEAD: those operator rows are
   // zero in the split copy), then the FP64 pass overwrites the leading columns
   if (!presplit) TRY(tc_split_rows(rows, n3, (const double *)S_rows, 0, level, row0, Ssplit, stream));
@@ -501,9 +527,9 @@ int Solver<T>::proj_down(int level, int64_t rows, int64_t row0, T *F_rows, bool 
   const T iL = (T)1 / cell_length<T>(level, (T)L);
   const T scale = homogen == 1 ? iL : (T)std::pow(iL, (T)homogen);
   if (r == 32) return launch_proj_r32<T>(false, rows, Lbuf, P32, kw, scale, F_rows, level, row0, rowlist, stream);
-  if (!proj_tc() || rows > Lsplit_rows)  // contraction over the effective rank (j < rk())
-    return launch_proj_dmma<T>(rows, rk(), n3, Lbuf, Bdn, kw, scale, F_rows, level, MAP_IN_CPG, stream, row0, r,
-                               rowlist);
+  if (!proj_tc() || rows > Lsplit_rows || msym[level])  // contraction over the effective rank (j < rk())
+    return launch_proj_dmma<T>(rows, rk(), n3, Lbuf, msym[level] ? Bdn_sym : Bdn, kw, scale, F_rows, level, MAP_IN_CPG,
+                               stream, row0, r, rowlist);
   // components j < 16 in FP64 and the rest as split-BF16 tensor-core products, one pass
   if (!presplit) TRY(tc_split_rows(rows, r, (const double *)Lbuf, 1, level, row0, Lsplit, stream, 16, rowlist));
   return launch_proj_down(tcproj, Lsplit, (const double *)Lbuf, rows, (double *)F_rows, level, row0,
@@ -563,7 +589,7 @@ int Solver<T>::m2l_post(int l) {
   {
     const T *Ml = Mall + Moff[l];
     bool presplit = false;  // the M2L kernel wrote the split rows of the down projection
-    const bool split = tc_m2l(l);
+    const bool split = tc_m2l(l) && !msym[l];
     if (split) {
       // FP64 leading block (i < lead_rows, j < lead) on the FP64 tensor path, then the
       // split-bf16 tensor-core kernel adds everything else into the same FP64 output; the
@@ -648,6 +674,7 @@ int Solver<T>::time_m2l(int level, int reps, float *ms) {
   BBFMM_CUDA_OK(cudaEventCreate(&b));
   const T *Ml = Mall + Moff[level];
   const bool split = tc_m2l(level);
+  msym[level] = sym_level(level);  // the launch that the current tuning makes
   const bool fused = split && lead > 0 && tc_fuses_lead(tcops, tc_products, rk());
   // the launch as the solve makes it: a whole level with the mixed projections also writes
   // the split rows of the down projection (m2l_post)
@@ -711,6 +738,7 @@ int Solver<T>::set_target_region(int level, const unsigned char *active_host) {
     region_level = level;
     TRY(build_region_tiles());
   }
+  if (pos4) TRY(alloc_partials());
   TRY(build_local());
   if (!pos4) return BBFMM_OK;
   TRY(build_heavy());
@@ -1035,7 +1063,7 @@ int Solver<T>::autotune(const void *q_dev, int io_double) {
   BBFMM_CUDA_OK(cudaStreamSynchronize(stream));
   for (int l = BBFMM_MINLEV; l <= maxlev; ++l) {
     char key[96];
-    snprintf(key, sizeof(key), "m2l/%d/%d/%d/%d", mode, n, l, bucket(cells(l)));
+    snprintf(key, sizeof(key), "m2l/%d/%d/%d/%d/%d", mode, n, l, bucket(cells(l)), sym_on() ? 1 : 0);
     {
       std::lock_guard<std::mutex> g(g_tune_mutex);
       auto it = g_tune_cache.find(key);
@@ -1048,6 +1076,7 @@ int Solver<T>::autotune(const void *q_dev, int io_double) {
     // candidates: (kind, offset groups); only the mixed mode has the tensor-core kind
     std::vector<std::pair<int, int>> cand;
     if (tc_default(l)) cand.push_back({0, 0});
+    if (sym_on()) cand.push_back({1, 0});
     // the DMMA and the SIMT M2L both split their offsets over groups
     for (int g : {1, 3, 7, 21})
       if (dmma_part_elems(l, nsets, g, r) * (int64_t)sizeof(T) <= ((int64_t)1 << 30)) cand.push_back({1, g});
@@ -1073,6 +1102,7 @@ int Solver<T>::autotune(const void *q_dev, int io_double) {
     g_tune_cache[key] = pick;
   }
   TRY(alloc_partials());
+  TRY(upward(q_dev, io_double));  // multipoles in the bases that the choices take
   // near field: threads per block
   char key[96];
   snprintf(key, sizeof(key), "p2p/%d/%d/%d", mode, bucket(N), bucket(cells(maxlev)));
@@ -1120,20 +1150,33 @@ int Solver<T>::autotune(const void *q_dev, int io_double) {
   return BBFMM_OK;
 }
 
+// r values per cell of one level (class-major rows on the device) to the host in the reference's
+// Morton order, in the basis of the operators as given.
+template <typename T>
+int Solver<T>::copy_rows_morton(const T *rows, int level, T *host_out) {
+  T *tmp = nullptr, *given = nullptr;
+  TRY(dalloc(&tmp, (size_t)pow8i(level) * r));
+  int rc = launch_morton_cpg<T>(level, r, rows, tmp, 1, stream);
+  if (rc == BBFMM_OK && msym[level]) {
+    rc = dalloc(&given, (size_t)pow8i(level) * r);
+    if (rc == BBFMM_OK) rc = sym_to_given<T>(symops, pow8i(level), tmp, given, stream);
+  }
+  if (rc == BBFMM_OK) {
+    cudaError_t e = cudaMemcpyAsync(host_out, given ? given : tmp, sizeof(T) * pow8i(level) * r, cudaMemcpyDeviceToHost,
+                                    stream);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(stream);
+    rc = bbfmm_set_cuda_error(e, "copy expansions", __FILE__, __LINE__);
+  }
+  cudaFree(tmp);
+  if (given) cudaFree(given);
+  return rc;
+}
+
 template <typename T>
 int Solver<T>::copy_multipoles_morton(int level, T *host_out) {
   if (level < BBFMM_MINLEV || level > maxlev) return bbfmm_set_error(BBFMM_ERR_ARG, "level out of range");
   if (nsets != 1) return bbfmm_set_error(BBFMM_ERR_UNSUPPORTED, "multipole copies are per single-set solver");
-  T *tmp = nullptr;
-  TRY(dalloc(&tmp, (size_t)pow8i(level) * r));
-  int rc = launch_morton_cpg<T>(level, r, Mall + Moff[level], tmp, 1, stream);
-  if (rc == BBFMM_OK) {
-    cudaError_t e = cudaMemcpyAsync(host_out, tmp, sizeof(T) * pow8i(level) * r, cudaMemcpyDeviceToHost, stream);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(stream);
-    rc = bbfmm_set_cuda_error(e, "copy multipoles", __FILE__, __LINE__);
-  }
-  cudaFree(tmp);
-  return rc;
+  return copy_rows_morton(Mall + Moff[level], level, host_out);
 }
 
 // The M2L output of one level (L = sum E_k M over the interaction lists, before the post-M2L
@@ -1146,7 +1189,7 @@ int Solver<T>::copy_m2l_morton(int level, T *host_out) {
   if (nsets != 1) return bbfmm_set_error(BBFMM_ERR_UNSUPPORTED, "M2L copies are per single-set solver");
   if (!pos4 || !Lbuf) return bbfmm_set_error(BBFMM_ERR_STATE, "particles not set");
   const T *Ml = Mall + Moff[level];
-  const bool split = tc_m2l(level);
+  const bool split = tc_m2l(level) && !msym[level];
   if (split) {
     const bool fused = lead > 0 && tc_fuses_lead(tcops, tc_products, rk());
     if (lead > 0 && !fused) TRY(m2l_fp(Ml, level, 0, lead, lead_rows));
@@ -1155,16 +1198,7 @@ int Solver<T>::copy_m2l_morton(int level, T *host_out) {
   } else {
     TRY(m2l_fp(Ml, level, 0, rk(), rk()));
   }
-  T *tmp = nullptr;
-  TRY(dalloc(&tmp, (size_t)pow8i(level) * r));
-  int rc = launch_morton_cpg<T>(level, r, Lbuf, tmp, 1, stream);
-  if (rc == BBFMM_OK) {
-    cudaError_t e = cudaMemcpyAsync(host_out, tmp, sizeof(T) * pow8i(level) * r, cudaMemcpyDeviceToHost, stream);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(stream);
-    rc = bbfmm_set_cuda_error(e, "copy M2L output", __FILE__, __LINE__);
-  }
-  cudaFree(tmp);
-  return rc;
+  return copy_rows_morton(Lbuf, level, host_out);
 }
 
 template <typename T>
@@ -1181,11 +1215,12 @@ void Solver<T>::release() {
   for (void *p : ptrs)
     if (p) cudaFree(p);
   if (own_ops) {
-    void *ops[] = {tkz, cw, kw, Ert, Ecol, Bup, Bdn, kwcol, Bup_lead, B32, P32};
+    void *ops[] = {tkz, cw, kw, Ert, Ecol, Bup, Bdn, kwcol, Bup_lead, Bup_sym, Bdn_sym, B32, P32};
     for (void *p : ops)
       if (p) cudaFree(p);
     if (tcops) tc_free_operators(tcops);
     if (tcproj) tc_free_projections(tcproj);
+    if (symops) sym_free(symops);
   }
   if (ev[ST_COUNT]) cudaEventDestroy(ev[ST_COUNT]);
   for (cudaEvent_t e : side_ev)
@@ -1231,10 +1266,13 @@ int bbfmm_b200_create(const bbfmm_b200_config *cfg, const void *U, const void *E
       std::vector<int> kt(343);
       rc = bbfmm_weights<float>(n, tkz.data(), kt.data(), kw.data(), cw.data());
       if (rc == BBFMM_OK) rc = h->f->set_tables(tkz.data(), cw.data(), kw.data());
-      std::vector<float> Uf((size_t)n3 * r), Ef((size_t)316 * r * r);
-      for (size_t i = 0; i < Uf.size(); ++i) Uf[i] = operators_fp32 ? ((const float *)U)[i] : (float)((const double *)U)[i];
-      for (size_t i = 0; i < Ef.size(); ++i) Ef[i] = operators_fp32 ? ((const float *)E)[i] : (float)((const double *)E)[i];
-      if (rc == BBFMM_OK) rc = h->f->set_operators(Uf.data(), Ef.data());
+      std::vector<float> Uf, Ef;
+      if (!operators_fp32) {
+        Uf.assign((const double *)U, (const double *)U + (size_t)n3 * r);
+        Ef.assign((const double *)E, (const double *)E + (size_t)316 * r * r);
+      }
+      if (rc == BBFMM_OK)
+        rc = h->f->set_operators(operators_fp32 ? (const float *)U : Uf.data(), operators_fp32 ? (const float *)E : Ef.data());
     }
   } else {
     h->d = new Solver<double>();
@@ -1244,10 +1282,13 @@ int bbfmm_b200_create(const bbfmm_b200_config *cfg, const void *U, const void *E
       std::vector<int> kt(343);
       rc = bbfmm_weights<double>(n, tkz.data(), kt.data(), kw.data(), cw.data());
       if (rc == BBFMM_OK) rc = h->d->set_tables(tkz.data(), cw.data(), kw.data());
-      std::vector<double> Ud((size_t)n3 * r), Ed((size_t)316 * r * r);
-      for (size_t i = 0; i < Ud.size(); ++i) Ud[i] = operators_fp32 ? ((const float *)U)[i] : ((const double *)U)[i];
-      for (size_t i = 0; i < Ed.size(); ++i) Ed[i] = operators_fp32 ? ((const float *)E)[i] : ((const double *)E)[i];
-      if (rc == BBFMM_OK) rc = h->d->set_operators(Ud.data(), Ed.data());
+      std::vector<double> Ud, Ed;
+      if (operators_fp32) {
+        Ud.assign((const float *)U, (const float *)U + (size_t)n3 * r);
+        Ed.assign((const float *)E, (const float *)E + (size_t)316 * r * r);
+      }
+      if (rc == BBFMM_OK)
+        rc = h->d->set_operators(operators_fp32 ? Ud.data() : (const double *)U, operators_fp32 ? Ed.data() : (const double *)E);
     }
   }
   if (rc != BBFMM_OK) {

@@ -78,6 +78,18 @@ int launch_m2l_dmma(int r, const double *M, const double *Ecol, double *Lout, in
                     const int4 *offs, double *part, int64_t part_elems, cudaStream_t s, int nsets = 1,
                     int ngroups = 0, const int4 *boxes = nullptr, int nboxes = 0);
 int dmma_default_groups(int level, int nsets);
+// M2L folded over mirrored offsets (m2l_sym.cu): n = 8 operators whose basis splits into parity
+// classes. U is on the host, the rest on the device; *out stays null without the symmetry.
+template <typename T>
+int sym_prepare(int n, int r, const T *U, const T *Ecol, double tol, const T *Bup, const T *Bdn, T *Bup_sym, T *Bdn_sym,
+                void **out, cudaStream_t s);
+void sym_free(void *ops);
+template <typename T>
+int sym_to_given(const void *ops, int64_t cells, const T *src, T *dst, cudaStream_t s);
+int sym_default_groups(int level, int nsets);
+template <typename T>
+int launch_m2l_sym(const void *ops, const T *M, T *Lout, int level, T *part, int64_t part_elems, cudaStream_t s,
+                   int nsets = 1, int ngroups = 0, const int4 *boxes = nullptr, int nboxes = 0);
 int64_t dmma_part_elems(int level, int nsets, int groups, int r);
 template <typename T>
 int launch_proj_dmma(int64_t M, int K, int N, const T *A, const T *B, const T *cs, T scale, T *C, int level, int mapmode,
@@ -208,10 +220,23 @@ struct Solver {
   T *Bup = nullptr;  // [n3][r]  Kweights[l] U(l, i)
   T *Bdn = nullptr;  // [r][n3]  U(l, j)
   T *kwcol = nullptr;
+  // mirror-symmetric operators: the rotated basis, its operators in step order and its projections;
+  // the multipoles and the M2L outputs of a solve are then in that basis
+  bool fold = true;  // cleared where multipoles in the given basis come from outside
+  void *symops = nullptr;
+  T *Bup_sym = nullptr, *Bdn_sym = nullptr;
   double *B32 = nullptr, *P32 = nullptr;  // r = 32: operators and projections in fragment order
-  int m2l_groups(int l) const {  // offset groups of the level's FP64 / FP32 M2L
+  bool sym_on() const { return symops && rank_eff == 0; }
+  // whether the level's solve runs the folded M2L, and whether its multipoles of the last upward
+  // pass are in the rotated basis
+  bool sym_level(int l) const { return sym_on() && !tc_m2l(l); }
+  bool msym[11] = {};
+  int m2l_groups(int l) const {  // offset (or step) groups of the level's FP64 / FP32 M2L
+    // (of a target region's short block lists: up to 8, the scratch of small levels only)
+    if (region_boxes[l] && sym_on() && cells(l) <= 4096) return 8;
     if (tune.m2l_groups[l] > 0) return tune.m2l_groups[l];
-    return r == 32 ? r32_default_groups(l, nsets) : dmma_default_groups(l, nsets);
+    return r == 32 ? r32_default_groups(l, nsets)
+                   : (sym_on() ? sym_default_groups(l, nsets) : dmma_default_groups(l, nsets));
   }
   int4 *offs = nullptr;
   void *tcops = nullptr;  // mixed mode: split operators for the tensor-core kernel
@@ -349,6 +374,7 @@ struct Solver {
   // solve_fields for two charge vectors, the near-field pairs evaluated once for both
   int solve_fields2(const void *q1_dev, const void *q2_dev, void *pot1_dev, void *fld1_dev, void *pot2_dev,
                     void *fld2_dev);
+  int copy_rows_morton(const T *rows, int level, T *host_out);
   int copy_multipoles_morton(int level, T *host_out);  // level's M in reference (Morton) order
   int copy_m2l_morton(int level, T *host_out);         // level's M2L output, recomputed, Morton order
   void mark(int stage, int launches = 1);

@@ -1,0 +1,123 @@
+"""M2L folded over mirrored offsets (m2l_sym.cu), the r = 32 kernels (m2l_r32.cu) and the heavy
+leaves of P2M / L2P, against the oracle (-m gpu).
+
+Tolerances: FP64 1e-12 (order of the sums; measured 1e-15 class), FP32 2e-5 (as the parity tests of
+the FP32 solve), mixed 3e-7 against FP64 (the split products' rounding, measured 4e-8)."""
+import numpy as np
+import pytest
+
+from conftest import uniform_inputs
+from oracle.oracle import Oracle, rel_l2
+
+pytestmark = pytest.mark.gpu
+
+
+def _ops(n, single=False, kernel="laplacian"):
+    from bbfmm_b200 import operators as ops
+    _, U, E = ops.load_operators(n, single=single, kernel=kernel)
+    return np.asarray(U), np.asarray(E)
+
+
+def _solve(x, q, n, lev, mode, U, E, **kw):
+    import torch
+    from bbfmm_b200 import Solver
+    s = Solver(n, lev, 1.0, mode=mode, operators=(U, E), **kw)
+    s.set_particles(x)
+    out = s.solve(torch.as_tensor(q, dtype=s.dtype, device="cuda")).double().cpu().numpy()
+    return s, out
+
+
+@pytest.mark.parametrize("n", [4, 8])
+@pytest.mark.parametrize("lev", [2, 3, 4])
+def test_levels_match_the_oracle(n, lev):
+    """Every level's tile form (stacked 2 x 2 x 2 grids, one box, many boxes), FP64 and FP32."""
+    x, q = uniform_inputs(3001, seed=10 * n + lev)
+    U, E = _ops(n)
+    ref = Oracle("d").fmm(x, q, n, lev, U, E)
+    s, got = _solve(x, q, n, lev, "d", U, E)
+    assert rel_l2(got, ref) < 1e-12
+    tree = Oracle("d").build_tree(x, lev)
+    _, P = Oracle("d").upward(tree, x, q, n, U)
+    r = n ** 3 // 2
+    for l in range(2, lev + 1):  # in the basis of the operators as given
+        lo = (8 ** l - 1) // 7
+        assert rel_l2(s.multipoles(l), P[lo * r:(lo + 8 ** l) * r]) < 1e-13
+    s.close()
+    Us, Es = _ops(n, single=True)
+    s, got = _solve(x, q, n, lev, "s", Us, Es)
+    assert rel_l2(got, ref) < 2e-5
+    s.close()
+
+
+@pytest.mark.parametrize("mode", ["d", "s", "mixed"])
+@pytest.mark.parametrize("sets", [1, 7, 8, 9, 17])
+def test_stacked_sets(mode, sets):
+    """Sets stacked at levels 2 and 3: counts around the eight sets of a level-2 tile."""
+    import torch
+    from bbfmm_b200 import Batch, Solver
+    rng = np.random.default_rng(sets)
+    xs = [rng.random((50 + 13 * k, 3)) - 0.5 for k in range(sets)]
+    b = Batch([(x, n, 3) for x in xs for n in (4, 8)], mode=mode)
+    q = rng.uniform(-1, 1, b.N)
+    got = b.solve(torch.as_tensor(q, dtype=b.dtype, device="cuda")).double().cpu().numpy()
+    b.close()
+    for n in (4, 8):
+        s = Solver(n, 3, 1.0, mode="d")
+        for k, x in enumerate(xs):
+            i = 2 * k + (n == 8)
+            a, e = int(b.offsets[i]), int(b.offsets[i + 1])
+            s.set_particles(x)
+            want = s.solve(torch.as_tensor(q[a:e], device="cuda")).cpu().numpy()
+            assert rel_l2(got[a:e], want) < {"d": 1e-12, "s": 2e-5, "mixed": 3e-7}[mode]
+        s.close()
+
+
+def test_any_basis_of_the_same_span():
+    """U Q and Q^T E Q for a random orthogonal Q: the same potentials (the rotation that sorts the
+    components by parity starts from whatever basis is given)."""
+    n, lev, r, n3 = 8, 3, 256, 512
+    U, E = _ops(n)
+    Q, _ = np.linalg.qr(np.random.default_rng(1).standard_normal((r, r)))
+    U2 = (U.reshape(r, n3).T @ Q).T.reshape(-1)
+    Ek = E.reshape(316, r, r).transpose(0, 2, 1)
+    E2 = (Q.T @ Ek @ Q).transpose(0, 2, 1).reshape(-1)
+    x, q = uniform_inputs(4000, seed=3)
+    s, a = _solve(x, q, n, lev, "d", U, E)
+    s.close()
+    s, b = _solve(x, q, n, lev, "d", np.ascontiguousarray(U2), np.ascontiguousarray(E2))
+    s.close()
+    # the products that make U2 and E2 round at 1e-15 of their largest entries
+    assert rel_l2(b, a) < 1e-11
+
+
+def test_operators_without_the_symmetry_take_the_general_path():
+    """One offset's operator changed: the images no longer agree, and the solve follows the given
+    operators all the same."""
+    n, lev, r = 8, 3, 256
+    U, E = _ops(n)
+    E = E.copy()
+    E[5 * r * r:6 * r * r] *= 1.5
+    x, q = uniform_inputs(3000, seed=4)
+    ref = Oracle("d").fmm(x, q, n, lev, U, E)
+    s, got = _solve(x, q, n, lev, "d", U, E)
+    assert rel_l2(got, ref) < 1e-12
+    s.close()
+
+
+@pytest.mark.parametrize("count", [63, 64, 65, 128, 129, 1000])
+@pytest.mark.parametrize("n,mode", [(4, "d"), (8, "d"), (4, "s"), (8, "mixed")])
+def test_heavy_leaves(count, n, mode):
+    """Leaves around the cap of 64 particles a warp takes: P2M chunks, their join, L2P chunks."""
+    import torch
+    rng = np.random.default_rng(count)
+    x = np.concatenate([rng.random((count, 3)) * 0.12 - 0.5, rng.random((count // 2, 3)) * 0.12 + 0.26,
+                        rng.random((200, 3)) - 0.5])
+    q = rng.uniform(-1, 1, len(x))
+    U, E = _ops(n)
+    ref = Oracle("d").fmm(x, q, n, 3, U, E)
+    Um, Em = _ops(n, single=mode == "s")
+    s, got = _solve(x, q, n, 3, mode, Um, Em)
+    assert rel_l2(got, ref) < {"d": 1e-12, "s": 2e-5, "mixed": 3e-7}[mode]
+    pot, fld = s.solve_fields(torch.as_tensor(q, dtype=s.dtype, device="cuda"))
+    assert rel_l2(pot.double().cpu().numpy() * q, ref) < {"d": 1e-12, "s": 2e-5, "mixed": 3e-7}[mode]
+    s.close()
