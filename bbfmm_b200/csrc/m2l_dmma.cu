@@ -8,7 +8,7 @@
 // The A tile (sources x 16 j) is gathered from the cpg multipole grid and the B tile
 // (16 j x 256 i) is read from the operators in the reference's own column-major layout
 // E[k][j][i] (K file, bbfmm.c:1384-1405), so both global reads are contiguous. Tiles are
-// double-buffered with cp.async; 8 warps in a 2 x 4 grid each own a 32-target x 64-output
+// held in a four-stage cp.async ring; 8 warps in a 2 x 4 grid each own a 32-target x 64-output
 // accumulator (4 x 8 fragments of 8x8); warps whose outputs lie beyond ni skip the math.
 #include "solver.cuh"
 
@@ -17,14 +17,15 @@ namespace bbfmm {
 namespace dm {
 
 constexpr int NT = 64, R = 256, BK = 16;
-constexpr int AST = NT + 4;   // padded row strides (doubles): conflict-free fragment reads
+constexpr int AST = BK + 4;   // A [target][j], B [j][i]: padded row strides, conflict-free fragment reads
 constexpr int BST = R + 4;
-constexpr int STAGE_DOUBLES = BK * AST + BK * BST;
-constexpr int SMEM_BYTES = 2 * STAGE_DOUBLES * 8;
+constexpr int STAGE_DOUBLES = NT * AST + BK * BST;
+constexpr int STAGES = 4;     // three chunks in flight while one is contracted, one barrier a chunk
+constexpr int SMEM_BYTES = STAGES * STAGE_DOUBLES * 8;
 
-__device__ __forceinline__ void cp_async8(uint32_t dst, const void *src, bool valid) {
-  const int n = valid ? 8 : 0;  // zero-fill when the source lies outside the grid
-  asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;" ::"r"(dst), "l"(src), "r"(n) : "memory");
+__device__ __forceinline__ void cp_async16z(uint32_t dst, const void *src, bool valid) {
+  const int n = valid ? 16 : 0;  // zero-fill when the source lies outside the grid
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(n) : "memory");
 }
 __device__ __forceinline__ void cp_async16(uint32_t dst, const void *src) {
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");
@@ -99,7 +100,26 @@ __global__ void __launch_bounds__(256, 1) m2l_dmma_kernel(const double *__restri
   Lout += (int64_t)og * 8 * nsets * P3 * R;  // all classes of all sets
   const uint32_t sbase = (uint32_t)__cvta_generic_to_shared(smem);
 
-  auto issue = [&](int it, int buf) {
+  // this thread copies the component pair 2 (tid & 7) of targets tid / 8 and 32 + tid / 8 every
+  // chunk: their cells are found once (targets outside the tile fall outside every grid)
+  int tx[2], ty[2], tz[2];
+  int64_t tbase[2];
+#pragma unroll
+  for (int e = 0; e < 2; ++e) {
+    const int t = 32 * e + (tid >> 3);
+    int sb;
+    bool wr;
+    cell(t, sb, tx[e], ty[e], tz[e], wr);
+    if (t >= nt) tx[e] = -(1 << 20);
+    tbase[e] = (int64_t)sb * P3;
+  }
+  const int j2 = 2 * (tid & 7);
+  auto issue = [&](int it) {
+    if (it >= niter) {  // an empty group keeps the wait counts uniform
+      cp_commit();
+      return;
+    }
+    const int buf = it % STAGES;
     const int o = o0 + it / nchunk, jc = j0 + (it % nchunk) * BK;
     const int4 ov = offs[(c & 7) * 189 + o];
     const int gx = cbx + ov.y, gy = cby + ov.z, gz = cbz + ov.w;
@@ -107,26 +127,24 @@ __global__ void __launch_bounds__(256, 1) m2l_dmma_kernel(const double *__restri
     const int shx = (gx - scx) / 2, shy = (gy - scy) / 2, shz = (gz - scz) / 2;
     const int sc = (scx << 2) | (scy << 1) | scz;
     const uint32_t sa = sbase + (uint32_t)(buf * STAGE_DOUBLES) * 8u;
-    const uint32_t sb = sa + (uint32_t)(BK * AST) * 8u;
-    // A: 64 targets x 16 j, 8-byte copies, zero outside the grid / j range
-    for (int e = tid; e < NT * BK; e += 256) {
-      const int t = e / BK, jj = e % BK;
-      int sb, px, py, pz;
-      bool wr;
-      cell(t, sb, px, py, pz, wr);
-      px += shx;
-      py += shy;
-      pz += shz;
-      const bool ok = t < nt && jc + jj < j1 && px >= 0 && px < P && py >= 0 && py < P && pz >= 0 && pz < P;
-      const double *src = ok ? M + ((int64_t)(sb + sc) * P3 + ((int64_t)pz * P + py) * P + px) * R + jc + jj : M;
-      cp_async8(sa + (uint32_t)(jj * AST + t) * 8u, src, ok);
+    const uint32_t sb = sa + (uint32_t)(NT * AST) * 8u;
+    // A: 64 targets x 16 j, zero outside the grid / j range (an even count of components)
+#pragma unroll
+    for (int e = 0; e < 2; ++e) {
+      const int px = tx[e] + shx, py = ty[e] + shy, pz = tz[e] + shz;
+      const bool ok = jc + j2 < j1 && (unsigned)px < (unsigned)P && (unsigned)py < (unsigned)P && (unsigned)pz < (unsigned)P;
+      const double *src = ok ? M + (tbase[e] + sc * P3 + ((int64_t)pz * P + py) * P + px) * R + jc + j2 : M;
+      cp_async16z(sa + (uint32_t)((32 * e + (tid >> 3)) * AST + j2) * 8u, src, ok);
     }
-    // B: 16 rows j of E_k (the first nb outputs i), 16-byte copies
+    // B: 16 rows j of E_k (the first nb outputs i), two rows a warp
     const double *Ek = Ecol + (int64_t)ov.x * R * R;
-    for (int e = tid; e < BK * (nb / 2); e += 256) {
-      const int jj = e / (nb / 2), i2 = (e % (nb / 2)) * 2;
+#pragma unroll
+    for (int w = 0; w < 2; ++w) {
+      const int jj = warp + 8 * w;
       const int j = jc + jj < j1 ? jc + jj : j1 - 1;  // rows past j1 meet zero A columns
-      cp_async16(sb + (uint32_t)(jj * BST + i2) * 8u, Ek + (int64_t)j * R + i2);
+#pragma unroll
+      for (int i2 = 2 * lane; i2 < R; i2 += 64)
+        if (i2 < nb) cp_async16(sb + (uint32_t)(jj * BST + i2) * 8u, Ek + (int64_t)j * R + i2);
     }
     cp_commit();
   };
@@ -137,25 +155,22 @@ __global__ void __launch_bounds__(256, 1) m2l_dmma_kernel(const double *__restri
 #pragma unroll
     for (int b = 0; b < 8; ++b) acc[a][b][0] = acc[a][b][1] = 0.0;
 
-  issue(0, 0);
+#pragma unroll
+  for (int it = 0; it < STAGES - 1; ++it) issue(it);
   for (int it = 0; it < niter; ++it) {
-    const int buf = it & 1;
-    if (it + 1 < niter) {
-      issue(it + 1, buf ^ 1);
-      cp_wait_one();
-    } else {
-      cp_wait_all();
-    }
-    __syncthreads();
+    asm volatile("cp.async.wait_group %0;" ::"n"(STAGES - 2) : "memory");
+    __syncthreads();  // chunk it has landed, and every warp is done with chunk it - 1
+    issue(it + STAGES - 1);
+    const int buf = it % STAGES;
     if (active) {
       const double *A = smem + buf * STAGE_DOUBLES;
-      const double *B = A + BK * AST;
+      const double *B = A + NT * AST;
 #pragma unroll
       for (int ks = 0; ks < BK / 4; ++ks) {
         const int k = ks * 4 + (lane & 3);
         double af[4], bf[8];
 #pragma unroll
-        for (int mf = 0; mf < 4; ++mf) af[mf] = A[k * AST + wm * 32 + mf * 8 + (lane >> 2)];
+        for (int mf = 0; mf < 4; ++mf) af[mf] = A[(wm * 32 + mf * 8 + (lane >> 2)) * AST + k];
 #pragma unroll
         for (int nf = 0; nf < 8; ++nf) bf[nf] = B[k * BST + wn * 64 + nf * 8 + (lane >> 2)];
 #pragma unroll
@@ -164,8 +179,8 @@ __global__ void __launch_bounds__(256, 1) m2l_dmma_kernel(const double *__restri
           for (int nf = 0; nf < 8; ++nf) dmma(acc[mf][nf][0], acc[mf][nf][1], af[mf], bf[nf]);
       }
     }
-    __syncthreads();
   }
+  cp_wait_all();
   if (!active) return;
   // D fragment: row = lane >> 2, columns 2 (lane & 3) + {0, 1}
 #pragma unroll
@@ -352,7 +367,7 @@ int launch_m2l_dmma(int r, const double *M, const double *Ecol, double *Lout, in
                     const int4 *offs, double *part, int64_t part_elems, cudaStream_t s, int nsets, int ngroups,
                     const int4 *boxes, int nboxes) {
   if (r != dm::R) return bbfmm_set_error(BBFMM_ERR_UNSUPPORTED, "FP64 tensor M2L is built for r = 256");
-  if (j0 < 0 || j1 > r || j0 >= j1 || ni < 2 || ni > r || ni % 2)
+  if (j0 < 0 || j1 > r || j0 >= j1 || (j0 | j1) % 2 || ni < 2 || ni > r || ni % 2)
     return bbfmm_set_error(BBFMM_ERR_ARG, "bad contraction / output range");
   const int P = 1 << (level - 1);
   const int bw = P < 4 ? P : 4;
