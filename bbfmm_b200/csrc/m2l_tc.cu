@@ -127,6 +127,17 @@ __device__ __forceinline__ uint64_t sw64_desc(uint32_t saddr) {
   return d;
 }
 
+// The same with rows of 128 B (64 bf16) in the 128-byte swizzle, 8-row groups 1,024 B apart.
+__device__ __forceinline__ uint64_t sw128_desc(uint32_t saddr) {
+  uint64_t d = 0;
+  d |= (uint64_t)((saddr >> 4) & 0x3FFF);
+  d |= (uint64_t)1 << 16;
+  d |= (uint64_t)(1024 >> 4) << 32;
+  d |= (uint64_t)1 << 46;
+  d |= (uint64_t)2 << 61;  // 128-byte swizzle
+  return d;
+}
+
 // kind::f16 instruction descriptor: BF16 x BF16 -> FP32, both K-major, M = 128, N columns
 // (a multiple of 16 up to 256; the accumulator columns [0, N) of the tile are updated).
 __host__ __device__ constexpr uint32_t idesc(int N) {
@@ -165,6 +176,48 @@ __device__ __forceinline__ void tmem_ld32(uint32_t taddr, float *v) {
   asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 #pragma unroll
   for (int i = 0; i < 32; ++i) v[i] = __uint_as_float(r[i]);
+}
+
+// The cta_group::2 forms: a load that may signal the other CTA's barrier (its address by
+// even_cta), products over both CTAs' operands, commits to both CTAs' barriers.
+__device__ __forceinline__ uint32_t even_cta(uint32_t addr) {  // the even CTA's copy of a shared address
+  uint32_t r;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, 0;" : "=r"(r) : "r"(addr));
+  return r;
+}
+__device__ __forceinline__ void tma_pair_5d(uint32_t dst, const CUtensorMap *map, uint32_t bar, int c0, int c1, int c2,
+                                            int c3, int c4) {
+  asm volatile(
+      "cp.async.bulk.tensor.5d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes"
+      " [%0], [%1, {%3, %4, %5, %6, %7}], [%2];" ::"r"(dst),
+      "l"((uint64_t)map), "r"(bar), "r"(c0), "r"(c1), "r"(c2), "r"(c3), "r"(c4)
+      : "memory");
+}
+__device__ __forceinline__ void tma_pair_3d(uint32_t dst, const CUtensorMap *map, uint32_t bar, int c0, int c1, int c2) {
+  asm volatile(
+      "cp.async.bulk.tensor.3d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes"
+      " [%0], [%1, {%3, %4, %5}], [%2];" ::"r"(dst),
+      "l"((uint64_t)map), "r"(bar), "r"(c0), "r"(c1), "r"(c2)
+      : "memory");
+}
+__host__ __device__ constexpr uint32_t idesc_pair(int N) { return (idesc(N) & 0xFFFFFFu) | ((uint32_t)(2 * BM >> 4) << 24); }
+__device__ __forceinline__ void mma_pair(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc, uint32_t acc, uint32_t id) {
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "setp.ne.b32 p, %4, 0;\n\t"
+      "tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n\t}" ::"r"(tmem_d),
+      "l"(adesc), "l"(bdesc), "r"(id), "r"(acc)
+      : "memory");
+}
+__device__ __forceinline__ void commit_pair(uint32_t bar) {
+  asm volatile(
+      "tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;" ::"r"(bar),
+      "h"((uint16_t)3)
+      : "memory");
+}
+__device__ __forceinline__ void cluster_barrier() {
+  asm volatile("barrier.cluster.arrive.aligned;" ::: "memory");
+  asm volatile("barrier.cluster.wait.aligned;" ::: "memory");
 }
 
 // Grid: one CTA per tile (class c, 8x4x4 box). Lacc: the level's FP64 output, cpg layout
@@ -321,10 +374,17 @@ __global__ void __launch_bounds__(192, 1)
 // origin (one box load per block and operand half; slots past the list's end load its last
 // block and write nothing), so the tiles follow the region. The box of slot k is loaded by
 // lane k of the producer warp, so the small boxes of a stage go out together.
-// Stage: A_hi 16 KB | A_lo 16 KB | B_hi 16 KB | B_lo TC_SPLIT_ROWS x 32 BF16 (4 KB).
-// With Mlead and Erow given (leading block i < 32, j < 16), the four epilogue warps, idle
-// while the tensor cores run the ~1 ms mainloop of a CTA, compute that block in FP64 for the
-// rows they later read from tensor memory: DMMA m8n8k4 with fragments loaded straight from
+// Two CTAs of a cluster, on two SMs, take two boxes of the same class and run their products as
+// one (cta_group::2, M = 256): each loads its own targets and half of the operator rows, which the
+// tensor cores of both read, so the operator crosses from L2 once for 512 targets. The even CTA
+// issues the products; its full barriers count the bytes of both CTAs, its commits free the stages
+// of both. Stages of 48 KB, rows of 64 bf16 (128 bytes, 128-byte swizzle): A_hi (256 targets) and
+// the CTA's half of B_hi for each chunk of 64 components, and after the first chunk's a stage with
+// A_lo and the halves of B_hi and B_lo for the TC_SPLIT_ROWS three-product outputs.
+// With Mlead and Erow given (leading block i < 32, j < 16), the eight epilogue warps, idle
+// while the tensor cores run the mainloop of a CTA, compute that block in FP64 for the
+// 32 rows each later reads from tensor memory (with four warps of 64 rows, one half after the
+// other, these chains of loads and DMMAs took longer than the mainloop): DMMA m8n8k4 with fragments loaded straight from
 // global memory (shared memory is taken by the stages), k-slot u of step ks standing for
 // component 4u + ks so that each fragment load is one contiguous 32-byte run of M or of
 // Erow[k][i][j] = E_k(i, j). The block is written to Lacc (assign) before the accumulator
@@ -333,27 +393,32 @@ __global__ void __launch_bounds__(192, 1)
 // for i < 32 and, for every i < ncols, its [hi | lo] BF16 split into the Morton row of the
 // cell (planes of `nrows` rows of 256), components i < DNZ zero: the input of the fused down
 // projection, which otherwise gathers and splits the rows in a separate pass.
-constexpr int A2_BYTES = 2 * A_BYTES, BLO2_BYTES = TC_SPLIT_ROWS * BK * 2;
-constexpr int STAGE2_BYTES = 2 * A2_BYTES + B_BYTES + BLO2_BYTES;
+constexpr int TC2_THREADS = 32 * (2 + 8);  // producer, MMA issuer, eight leading-block / epilogue warps
+constexpr int BK2 = 64, KS2 = BK2 / 16;        // bf16 per K-chunk: 128-byte rows
+constexpr int A2_BYTES = 2 * BM * BK2 * 2;     // a CTA's 256 targets
+constexpr int B2_BYTES = BN / 2 * BK2 * 2;     // its half of the operator rows
+constexpr int BC_BYTES = TC_SPLIT_ROWS / 2 * BK2 * 2;  // its half of the three-product rows
+constexpr int STAGE2_BYTES = A2_BYTES + B2_BYTES;
 constexpr int SMEM2_BYTES = STAGES * STAGE2_BYTES + 1024 /*align*/ + 256 /*barriers*/;
-static_assert(SMEM2_BYTES <= 232448, "two-box stages exceed the shared memory of a CTA");
+static_assert(SMEM2_BYTES + 1024 <= 232448, "two-box stages exceed the shared memory of a CTA");
+static_assert(TC_SPLIT_CHUNKS * BK <= BK2, "the three-product components are within the first chunk");
 
-__global__ void __launch_bounds__(192, 1)
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(TC2_THREADS, 1)
     m2l_tc2_kernel(const __grid_constant__ CUtensorMap mapAhi, const __grid_constant__ CUtensorMap mapAlo,
-                   const __grid_constant__ CUtensorMap mapBhi, const __grid_constant__ CUtensorMap mapBlo,
+                   const __grid_constant__ CUtensorMap mapBhi, const __grid_constant__ CUtensorMap mapBhiC,
+                   const __grid_constant__ CUtensorMap mapBloC,
                    double *__restrict__ Lacc, int level, const int4 *__restrict__ offs, int kfirst, int ilead,
                    int split_chunks, int ncols, const double *__restrict__ Mlead, const double *__restrict__ Erow,
                    __nv_bfloat16 *__restrict__ Lsplit, int64_t nrows, const int4 *__restrict__ boxes,
                    int nboxes, int lgeom, int nsets) {
-  constexpr int STAGE_BYTES = STAGE2_BYTES;
   constexpr int DNZ = 16;  // components the fused down projection takes in FP64
   constexpr int split_rows = TC_SPLIT_ROWS;
   extern __shared__ uint8_t smem_raw[];
   const uint32_t raw = smem_u32(smem_raw);
   const uint32_t base = (raw + 1023u) & ~1023u;
   uint8_t *gbase = smem_raw + (base - raw);
-  const uint32_t bar_base = base + STAGES * STAGE_BYTES;
-  uint64_t *bars = reinterpret_cast<uint64_t *>(gbase + STAGES * STAGE_BYTES);
+  const uint32_t bar_base = base + STAGES * STAGE2_BYTES;
+  uint64_t *bars = reinterpret_cast<uint64_t *>(gbase + STAGES * STAGE2_BYTES);
   // bars[0..S-1] = full, bars[S..2S-1] = empty, bars[2S] = accumulator ready; tmem slot after
   uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(bars + 2 * STAGES + 1);
   auto full_bar = [&](int s) { return bar_base + 8u * s; };
@@ -368,9 +433,10 @@ __global__ void __launch_bounds__(192, 1)
   const int tiles_per_class = listed ? 1 : nbx * nby * nbz;
   // sibling class fastest (the set group or list group above it): the CTAs resident at one
   // time are the 8 classes of neighbouring boxes, which read one source region that stays in L2
-  const int bid_ = (int)blockIdx.x;
-  const int sg_ = bid_ / (8 * tiles_per_class), loc_ = bid_ % (8 * tiles_per_class);
-  const int cls = loc_ % 8, tb = loc_ / 8;
+  // (a pair past an odd count of tiles has a second tile whose slots are all past the end)
+  const int odd = (int)blockIdx.x & 1, pair_ = (int)blockIdx.x >> 1;
+  const int cls = pair_ % 8, tile_ = 2 * (pair_ / 8) + odd;
+  const int sg_ = tile_ / tiles_per_class, tb = tile_ % tiles_per_class;
   const int set0 = sg_ << (8 - g.lb());  // first set (or list entry) of the tile
   const int bx0 = (tb % nbx) << g.lx, by0 = ((tb / nbx) % nby) << g.ly, bz0 = (tb / (nbx * nby)) << g.lz;
   const int cbx = (cls >> 2) & 1, cby = (cls >> 1) & 1, cbz = cls & 1;
@@ -409,11 +475,9 @@ __global__ void __launch_bounds__(192, 1)
     y += y0;
     z += z0;
   };
-  const int nchunk = ncols / BK;  // K-chunks per offset: the effective rank / 32 (8 for r = 256)
-  const int chunk0 = kfirst / KS;  // whole chunks skipped
-  const int kstep0 = kfirst % KS;  // K-steps skipped in the first used chunk
-  const int used_chunks = nchunk - chunk0;
-  const int niter = 189 * used_chunks;
+  const int nchunk = (ncols + BK2 - 1) / BK2;  // K-chunks per offset: the effective rank / 64, the last
+                                               // perhaps half used (its other operator columns are zero)
+  const bool three = split_chunks > 0;         // the first chunk takes three products
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < STAGES; ++s) {
@@ -425,13 +489,14 @@ __global__ void __launch_bounds__(192, 1)
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
   }
   if (warp == 0) {
-    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)),
+    asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)),
                  "r"(512)
                  : "memory");
-    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
   }
   tc_fence_before();
   __syncthreads();
+  cluster_barrier();  // both CTAs' barriers and tensor memory are set up
   tc_fence_after();
   const uint32_t tmem = *tmem_slot;
 
@@ -444,78 +509,106 @@ __global__ void __launch_bounds__(192, 1)
       bool ok;
       slot(lane, set_k, x0_k, y0_k, z0_k, ok);
     }
-    const uint32_t box_bytes = (uint32_t)BK * 2u << g.lb();
-    for (int it = 0; it < niter; ++it) {
-      const int s = it % STAGES;
-      const uint32_t ph = (uint32_t)(it / STAGES) & 1u;
-      const bool got = lane == 0 ? mbar_wait(empty_bar(s), ph ^ 1u, 1) : true;
-      if (!__shfl_sync(0xffffffffu, got ? 1 : 0, 0)) break;
-      const int o = it / used_chunks, kc = chunk0 + it % used_chunks;
+    const uint32_t box_bytes = (uint32_t)BK2 * 2u << g.lb();
+    int s = 0;
+    uint32_t ph = 1u;  // parity of the stage's empty barrier (the first round passes)
+    const uint32_t even_full = even_cta(full_bar(0));
+    const uint32_t main_bytes = 2u * A2_BYTES + (uint32_t)ncols * BK2 * 2;  // of both CTAs
+    constexpr uint32_t corr_bytes = 2u * (A2_BYTES + 2 * BC_BYTES);
+    bool alive = true;
+    for (int o = 0; o < 189 && alive; ++o) {
       const int4 ov = offs[cls * 189 + o];
       const int gx = cbx + ov.y, gy = cby + ov.z, gz = cbz + ov.w;
       const int scx = gx & 1, scy = gy & 1, scz = gz & 1;
       const int sc = (scx << 2) | (scy << 1) | scz;
       const int shx = (gx - scx) / 2, shy = (gy - scy) / 2, shz = (gz - scz) / 2;  // parent-grid step
-      const uint32_t st = base + s * STAGE_BYTES;
-      // chunks kc < split_chunks take three products and need the lo halves (of B only its
-      // first split_rows rows, the box of mapBlo); the others take hi x hi alone
-      const bool three = kc < split_chunks;
-      const uint32_t bhi_bytes = (uint32_t)ncols * BK * 2;  // the B box holds the first ncols rows i
-      if (lane == 0) {
-        mbar_expect_tx(full_bar(s), three ? 2 * A2_BYTES + bhi_bytes + BLO2_BYTES : A2_BYTES + bhi_bytes);
-        tma_load_3d(st + 2 * A2_BYTES, &mapBhi, full_bar(s), kc * BK, 0, ov.x);
-        if (three) tma_load_3d(st + 2 * A2_BYTES + B_BYTES, &mapBlo, full_bar(s), kc * BK, 0, ov.x);
-      }
-      __syncwarp();
-      // a slot past the last set or list entry loads a valid box: the same bytes
-      if (lane < nslot) {
-        const int sidx = set_k * 8 + sc;
-        tma_load_5d(st + lane * box_bytes, &mapAhi, full_bar(s), kc * BK, x0_k + shx, y0_k + shy, z0_k + shz, sidx);
-        if (three)
-          tma_load_5d(st + A2_BYTES + lane * box_bytes, &mapAlo, full_bar(s), kc * BK, x0_k + shx, y0_k + shy,
-                      z0_k + shz, sidx);
-      }
-    }
-  } else if (warp == 1 && lane == 0) {
-    // ---------------- MMA issuer
-    uint32_t acc = 0;
-    for (int it = 0; it < niter; ++it) {
-      const int s = it % STAGES;
-      const uint32_t ph = (uint32_t)(it / STAGES) & 1u;
-      if (!mbar_wait(full_bar(s), ph, 2)) break;
-      tc_fence_after();
-      const uint32_t st = base + s * STAGE_BYTES;
-      const int k0 = (it % used_chunks == 0) ? kstep0 : 0;
-      const bool three = chunk0 + it % used_chunks < split_chunks;
-      const uint32_t id_part = idesc(split_rows), id_all = idesc(ncols);
-      for (int ks = k0; ks < KS; ++ks) {
-        const uint64_t bhi = sw64_desc(st + 2 * A2_BYTES + ks * 32);
-        const uint64_t blo = sw64_desc(st + 2 * A2_BYTES + B_BYTES + ks * 32);
-#pragma unroll
-        for (int h = 0; h < 2; ++h) {  // the two 128-target halves of the box, accumulators h * 256
-          const uint64_t ahi = sw64_desc(st + h * A_BYTES + ks * 32);
-          const uint64_t alo = sw64_desc(st + A2_BYTES + h * A_BYTES + ks * 32);
-          mma_bf16(tmem + h * 256, ahi, bhi, acc, id_all);  // all ncols outputs (the first initialises)
-          if (three) {                              // corrections for the outputs i < split_rows
-            mma_bf16(tmem + h * 256, ahi, blo, 1u, id_part);
-            mma_bf16(tmem + h * 256, alo, bhi, 1u, id_part);
+      for (int c = 0; c < nchunk + (three ? 1 : 0); ++c) {
+        const bool corr = three && c == 1;  // stages: chunk 0, its corrections, chunks 1 ..
+        const int kc = three && c > 0 ? c - 1 : c;
+        const bool got = lane == 0 ? mbar_wait(empty_bar(s), ph, 1) : true;
+        if (!__shfl_sync(0xffffffffu, got ? 1 : 0, 0)) {
+          alive = false;
+          break;
+        }
+        const uint32_t st = base + s * STAGE2_BYTES;
+        if (lane == 0) {
+          if (!odd) mbar_expect_tx(full_bar(s), corr ? corr_bytes : main_bytes);
+          if (corr) {
+            tma_pair_3d(st + A2_BYTES, &mapBhiC, even_full + 8u * s, kc * BK2, odd * (TC_SPLIT_ROWS / 2), ov.x);
+            tma_pair_3d(st + A2_BYTES + BC_BYTES, &mapBloC, even_full + 8u * s, kc * BK2, odd * (TC_SPLIT_ROWS / 2), ov.x);
+          } else {
+            tma_pair_3d(st + A2_BYTES, &mapBhi, even_full + 8u * s, kc * BK2, odd * (ncols / 2), ov.x);
           }
         }
-        acc = 1u;
+        __syncwarp();
+        if (lane < nslot)  // a slot past the last set or list entry loads a valid box: the same bytes
+          tma_pair_5d(st + lane * box_bytes, corr ? &mapAlo : &mapAhi, even_full + 8u * s, kc * BK2, x0_k + shx, y0_k + shy,
+                      z0_k + shz, set_k * 8 + sc);
+        if (++s == STAGES) {
+          s = 0;
+          ph ^= 1u;
+        }
       }
-      mma_commit(empty_bar(s));
     }
-    mma_commit(acc_bar);  // also after an early exit: the epilogue must not wait forever
+  } else if (warp == 1 && lane == 0 && !odd) {
+    // ---------------- MMA issuer (the even CTA, for both)
+    const uint32_t id_part = idesc_pair(split_rows), id_all = idesc_pair(ncols);
+    uint32_t acc = 0, ph = 0;
+    int s = 0;
+    auto take = [&](uint32_t &addr, uint32_t &bar) -> bool {  // the next stage, once it has landed
+      if (!mbar_wait(full_bar(s), ph, 2)) return false;
+      addr = base + s * STAGE2_BYTES;
+      bar = empty_bar(s);
+      if (++s == STAGES) {
+        s = 0;
+        ph ^= 1u;
+      }
+      return true;
+    };
+    bool alive = true;
+    for (int o = 0; o < 189 && alive; ++o)
+      for (int kc = 0; kc < nchunk && alive; ++kc) {
+        uint32_t ahi, alo, ea, ec;
+        alive = take(ahi, ea);
+        if (!alive) break;
+        tc_fence_after();
+        const uint32_t bhi = ahi + A2_BYTES;
+        const int nks = ncols - kc * BK2 < BK2 ? (ncols - kc * BK2) / 16 : KS2;
+        const int k0 = kc == 0 ? kfirst : 0;  // K-steps of a full-width leading strip are skipped
+        for (int ks = k0; ks < nks; ++ks) {
+#pragma unroll
+          for (int h = 0; h < 2; ++h)  // the two 128-target halves of each box, accumulators h * 256
+            mma_pair(tmem + h * 256, sw128_desc(ahi + h * (A2_BYTES / 2) + ks * 32), sw128_desc(bhi + ks * 32), acc, id_all);
+          acc = 1u;  // all ncols outputs (the first of each half initialises them)
+        }
+        if (three && kc == 0) {  // corrections for the outputs i < split_rows
+          alive = take(alo, ec);
+          if (alive) {
+            tc_fence_after();
+            const uint32_t bhc = alo + A2_BYTES, blc = bhc + BC_BYTES;
+            for (int ks = k0; ks < nks; ++ks)
+#pragma unroll
+              for (int h = 0; h < 2; ++h) {
+                mma_pair(tmem + h * 256, sw128_desc(ahi + h * (A2_BYTES / 2) + ks * 32), sw128_desc(blc + ks * 32), 1u, id_part);
+                mma_pair(tmem + h * 256, sw128_desc(alo + h * (A2_BYTES / 2) + ks * 32), sw128_desc(bhc + ks * 32), 1u, id_part);
+              }
+            commit_pair(ec);
+          }
+        }
+        commit_pair(ea);
+      }
+    commit_pair(acc_bar);  // also after an early exit: the epilogues must not wait forever
   } else if (warp >= 2) {
     // ---------------- epilogue: TMEM -> registers -> Lacc
-    const int q = warp & 3;  // TMEM lane quarter this warp may access
+    const int q = warp & 3;         // TMEM lane quarter this warp may access
+    const int h = (warp - 2) >> 2;  // its half of the box
     const int row = q * 32 + lane;
     const int64_t P3 = (int64_t)P * P * P;
     if (Mlead) {
       // FP64 leading block of rows h * 128 + q * 32 + [0, 32): fragment m holds the 8 rows
       // 8m .. 8m + 7 of that range, this lane's A row being 8m + (lane >> 2)
       const int u = lane & 3, tr = lane >> 2;
-      for (int h = 0; h < 2; ++h) {
+      {
         double acc[4][4][2];
         int ax[4], ay[4], az[4], aset[4];  // grid position and set of this lane's A rows
         bool aok[4];                       // whether those rows are written
@@ -578,9 +671,9 @@ __global__ void __launch_bounds__(192, 1)
       __threadfence_block();
       __syncwarp();  // the rows written here are read back below by other lanes of this warp
     }
-    const bool ok = mbar_wait(acc_bar, 0, 3);
+    const bool ok = __all_sync(0xffffffffu, mbar_wait(acc_bar, 0, 3));
     tc_fence_after();
-    for (int h = 0; h < 2 && ok; ++h) {
+    if (ok) {
       int tx, ty, tz, set;
       bool valid;  // rows of slots past the last set or list entry: read from TMEM, not written
       row_cell(h * 128 + row, set, tx, ty, tz, valid);
@@ -622,9 +715,10 @@ __global__ void __launch_bounds__(192, 1)
   }
   tc_fence_before();
   __syncthreads();
+  cluster_barrier();  // the other CTA's products, commits and reads are over
   tc_fence_after();
   if (warp == 0) {
-    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(512) : "memory");
+    asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(512) : "memory");
   }
 }
 
@@ -986,7 +1080,9 @@ struct TcOps {
   int r = 0, lead = 0, lead_rows = 0;
   __nv_bfloat16 *Ehi = nullptr, *Elo = nullptr;
   CUtensorMap mapBhi, mapBlo;
-  CUtensorMap mapBlo_part;  // the first TC_SPLIT_ROWS rows i of the lo operator chunk
+  // the two-box kernel's chunks of 64 components, each CTA's half of the rows i: all of hi, and the
+  // TC_SPLIT_ROWS three-product ones of hi and lo
+  CUtensorMap mapBhi_two, mapBhi_c, mapBlo_c;
 };
 
 int tc_supported() {
@@ -997,10 +1093,10 @@ int tc_supported() {
 }
 
 static int make_map(CUtensorMap *m, void *ptr, int rank, const cuuint64_t *dims, const cuuint64_t *strides_bytes,
-                    const cuuint32_t *box) {
+                    const cuuint32_t *box, CUtensorMapSwizzle swizzle = CU_TENSOR_MAP_SWIZZLE_64B) {
   cuuint32_t es[5] = {1, 1, 1, 1, 1};
   CUresult rc = encode_fn()(m, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, (cuuint32_t)rank, ptr, dims, strides_bytes, box, es,
-                            CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_64B,
+                            CU_TENSOR_MAP_INTERLEAVE_NONE, swizzle,
                             CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   if (rc != CUDA_SUCCESS) {
     char buf[96];
@@ -1038,8 +1134,10 @@ int tc_prepare_operators(int r, const double *Ert, int lead, int lead_rows, void
   const cuuint32_t box[3] = {tc::BK, (cuuint32_t)tc::BN, 1};
   int rc = make_map(&ops->mapBhi, ops->Ehi, 3, dims, strides, box);
   if (rc == BBFMM_OK) rc = make_map(&ops->mapBlo, ops->Elo, 3, dims, strides, box);
-  const cuuint32_t box_part[3] = {tc::BK, (cuuint32_t)TC_SPLIT_ROWS, 1};
-  if (rc == BBFMM_OK) rc = make_map(&ops->mapBlo_part, ops->Elo, 3, dims, strides, box_part);
+  const cuuint32_t box2[3] = {tc::BK2, (cuuint32_t)tc::BN / 2, 1}, boxc[3] = {tc::BK2, (cuuint32_t)TC_SPLIT_ROWS / 2, 1};
+  if (rc == BBFMM_OK) rc = make_map(&ops->mapBhi_two, ops->Ehi, 3, dims, strides, box2, CU_TENSOR_MAP_SWIZZLE_128B);
+  if (rc == BBFMM_OK) rc = make_map(&ops->mapBhi_c, ops->Ehi, 3, dims, strides, boxc, CU_TENSOR_MAP_SWIZZLE_128B);
+  if (rc == BBFMM_OK) rc = make_map(&ops->mapBlo_c, ops->Elo, 3, dims, strides, boxc, CU_TENSOR_MAP_SWIZZLE_128B);
   if (rc != BBFMM_OK) {
     tc_free_operators(ops);
     return rc;
@@ -1236,27 +1334,26 @@ int launch_m2l_tc(int r, const void *Msplit, int64_t ncell_total, int64_t cell_o
   const cuuint64_t dims[5] = {(cuuint64_t)r, (cuuint64_t)P, (cuuint64_t)P, (cuuint64_t)P, (cuuint64_t)8 * nsets};
   const cuuint64_t strides[4] = {(cuuint64_t)r * 2, (cuuint64_t)r * 2 * P, (cuuint64_t)r * 2 * P * P,
                                  (cuuint64_t)r * 2 * P * P * P};
-  const cuuint32_t box[5] = {tc::BK, two ? 1u << g2.lx : (cuuint32_t)tc::BOX_X,
+  const CUtensorMapSwizzle sw = two ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_64B;
+  const cuuint32_t kbox = two ? tc::BK2 : tc::BK;
+  const cuuint32_t box[5] = {kbox, two ? 1u << g2.lx : (cuuint32_t)tc::BOX_X,
                              two ? 1u << g2.ly : (cuuint32_t)tc::BOX_Y, two ? 1u << g2.lz : (cuuint32_t)tc::BOX_Z, 1};
-  int rc = make_map(&mapAhi, (void *)hi, 5, dims, strides, box);
-  if (rc == BBFMM_OK) rc = make_map(&mapAlo, (void *)lo, 5, dims, strides, box);
+  int rc = make_map(&mapAhi, (void *)hi, 5, dims, strides, box, sw);
+  if (rc == BBFMM_OK) rc = make_map(&mapAlo, (void *)lo, 5, dims, strides, box, sw);
   if (rc != BBFMM_OK) return rc;
   // with a full-width leading strip its K-steps are skipped; otherwise every K-step runs
   const int kfirst = ops->lead_rows >= r ? ops->lead / 16 : 0;
   const int ilead = ops->lead > 0 ? ops->lead_rows : 0;
   // B boxes of the first `rank` operator rows (the effective rank); the lo box keeps its
   // split_rows rows (box maps built here when they differ from the prepared ones)
-  CUtensorMap mapBhi = ops->mapBhi, mapBlo = split_rows < tc::BN ? ops->mapBlo_part : ops->mapBlo;
+  CUtensorMap mapBhi = two ? ops->mapBhi_two : ops->mapBhi, mapBlo = ops->mapBlo;
   {
     const cuuint64_t bd[3] = {(cuuint64_t)r, (cuuint64_t)r, (cuuint64_t)BBFMM_NUM_OFFSETS};
     const cuuint64_t bs[2] = {(cuuint64_t)r * 2, (cuuint64_t)r * r * 2};
     if (rank != tc::BN) {
-      const cuuint32_t bb[3] = {tc::BK, (cuuint32_t)rank, 1};
-      rc = make_map(&mapBhi, ops->Ehi, 3, bd, bs, bb);
-    }
-    if (rc == BBFMM_OK && split_rows != tc::BN && split_rows != TC_SPLIT_ROWS) {
-      const cuuint32_t bl[3] = {tc::BK, (cuuint32_t)split_rows, 1};
-      rc = make_map(&mapBlo, ops->Elo, 3, bd, bs, bl);
+      const cuuint32_t bb[3] = {kbox, (cuuint32_t)(two ? rank / 2 : rank), 1};
+      rc = make_map(&mapBhi, ops->Ehi, 3, bd, bs, bb, sw);
+      if (rc == BBFMM_OK && !two) rc = make_map(&mapBlo, ops->Elo, 3, bd, bs, bb, sw);  // split_rows = rank
     }
     if (rc != BBFMM_OK) return rc;
   }
@@ -1274,9 +1371,10 @@ int launch_m2l_tc(int r, const void *Msplit, int64_t ncell_total, int64_t cell_o
     if (boxes && (nboxes < 0 || nboxes > (int64_t)nsets * (P >> g2.lx) * (P >> g2.ly) * (P >> g2.lz)))
       return bbfmm_set_error(BBFMM_ERR_ARG, "box list longer than the level");
     if (boxes && nboxes == 0) return BBFMM_OK;
-    const int64_t tiles2 = boxes ? 8 * (int64_t)((nboxes + spl - 1) / spl) : tc2_tiles(level, nsets);
-    tc::m2l_tc2_kernel<<<(unsigned)tiles2, 192, tc::SMEM2_BYTES, s>>>(
-        mapAhi, mapAlo, mapBhi, mapBlo, Lacc, level, offs, kfirst, ilead, split_chunks, rank, fuse ? Mlead : nullptr,
+    const int64_t per_class = boxes ? (int64_t)((nboxes + spl - 1) / spl) : tc2_tiles(level, nsets) / 8;
+    const int64_t tiles2 = 16 * ((per_class + 1) / 2);  // pairs of a class's tiles
+    tc::m2l_tc2_kernel<<<(unsigned)tiles2, tc::TC2_THREADS, tc::SMEM2_BYTES, s>>>(
+        mapAhi, mapAlo, mapBhi, ops->mapBhi_c, ops->mapBlo_c, Lacc, level, offs, kfirst, ilead, split_chunks, rank, fuse ? Mlead : nullptr,
         fuse ? Erow : nullptr, (__nv_bfloat16 *)Lsplit, 8 * (int64_t)nsets * P * P * P, boxes, nboxes, lgeom, nsets);
     return bbfmm_set_cuda_error(cudaGetLastError(), "m2l_tc2", __FILE__, __LINE__);
   }
