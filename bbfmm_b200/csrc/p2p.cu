@@ -19,8 +19,8 @@
 // Regions larger than one tile (dense neighbours) stream in tiles in both kinds.
 //
 // Arithmetic (MODE):
-//  * FP64 / FP32: positions and arithmetic in the working precision, 1/sqrt as the reference
-//    (the d and s builds).
+//  * FP64 / FP32: positions and arithmetic in the working precision (the reference's d and s
+//    builds).
 //  * mixed: the pair's separation and its square in FP64 (FP32 coordinates would cost up to
 //    2^-24 h / r_ij of relative error on close pairs, h the leaf length), then 1/r in FP32
 //    (rsqrtf and one Newton step) and the pair value times the FP32 charge; per-target
@@ -55,6 +55,39 @@ __device__ __forceinline__ void flag_leaf_range(int *flag) {
 __device__ __forceinline__ float rsqrt_nr(float rr) {
   const float y = rsqrtf(rr);
   return y * fmaf(-0.5f * rr * y, y, 1.5f);
+}
+
+// The reciprocal distance of a pair from rr = r^2. For normal numbers the flushing form of the FP32
+// estimate gives the same bits as rsqrtf without the scaling that covers subnormal inputs; the rest
+// (0 for coincident points and at infinity, subnormal, NaN) takes the branch.
+__device__ __forceinline__ bool rsqrt_normal(float rr) { return rr >= 1.17549435e-38f && rr <= 3.40282347e38f; }
+__device__ __forceinline__ float rsqrt_ftz(float rr) {
+  float y;
+  asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(rr));
+  return y;
+}
+__device__ __forceinline__ float rsqrt_rest(float rr) {
+  return rr > 0.f ? (rr <= 3.40282347e38f ? rsqrt_nr(rr) : 0.f) : (rr == 0.f ? 0.f : rr);
+}
+// Mixed mode: one Newton step, as rsqrt_nr.
+__device__ __forceinline__ float recip_mixed(float rr) {
+  const float y = rsqrt_ftz(rr);
+  float r = y * fmaf(-0.5f * rr * y, y, 1.5f);
+  if (!rsqrt_normal(rr)) r = rsqrt_rest(rr);
+  return r;
+}
+// FP64: CUDA's reciprocal square root (within 1 ulp). FP32: the estimate y corrected by its residual
+// 1 - rr y^2, formed with the rounding error of rr y, so that one rounding is left (a rounded square
+// root and a rounded division have two, and took most of the instructions of a pair: near field of
+// 100,003 clustered particles 1.99 -> 1.3 ms).
+__device__ __forceinline__ double recip_dist(double rr) { return rsqrt(rr); }
+__device__ __forceinline__ float recip_dist(float rr) {
+  const float y = rsqrt_ftz(rr);
+  const float h = rr * y, l = fmaf(rr, y, -h);
+  const float e = fmaf(-l, y, fmaf(-h, y, 1.f));
+  float r = fmaf(0.5f * y, e, y);
+  if (!rsqrt_normal(rr)) r = rsqrt_rest(rr);
+  return r;
 }
 
 // Source particles as staged in shared memory: FP64 / FP32 (x, y, z, q); mixed: FP64
@@ -99,7 +132,7 @@ struct NearAcc {
       const double rr = fma(ex, ex, fma(ey, ey, ez * ez));
       const float rrf = (float)rr;
       // rrf = 0 only for coincident points (positions in the unit-scale root cell)
-      const float rinv = rrf > 0.f ? rsqrt_nr(rrf) : 0.f;
+      const float rinv = recip_mixed(rrf);
       // the term enters the sum rounded (an explicit __fmul_rn is never contracted into an
       // addition), so the compensation below sees the exact rounding error of each addition
       float t;
@@ -116,7 +149,7 @@ struct NearAcc {
     } else {
       const C rr = ex * ex + ey * ey + ez * ez;
       if (rr == (C)0) return (C)0;
-      const C rinv = (C)1 / sqrt(rr);
+      const C rinv = recip_dist(rr);
       if constexpr (FIELD) {
         const C qr = g.w * rinv, qr3 = qr * rinv * rinv;
         gx += qr3 * ex;
@@ -162,7 +195,7 @@ struct NearAcc {
     if constexpr (MODE == MODE_MIXED) {
       const double rr = fma(ex, ex, fma(ey, ey, ez * ez));
       const float rrf = (float)rr;
-      const float rinv = rrf > 0.f ? rsqrt_nr(rrf) : 0.f;
+      const float rinv = recip_mixed(rrf);
       const float t = __fmul_rn(g.q, rinv), u = __fmul_rn(q2, rinv);
       const float t3 = t * rinv * rinv, u3 = u * rinv * rinv;
       gx += t3 * (float)ex;
@@ -176,7 +209,7 @@ struct NearAcc {
     } else {
       const C rr = ex * ex + ey * ey + ez * ez;
       if (rr == (C)0) return;  // both terms 0, as add adds
-      const C rinv = (C)1 / sqrt(rr);
+      const C rinv = recip_dist(rr);
       const C qr = g.w * rinv, qr3 = qr * rinv * rinv;
       const C ur = q2 * rinv, ur3 = ur * rinv * rinv;
       gx += qr3 * ex;
@@ -199,7 +232,7 @@ struct NearAcc {
         const C ex = g[k].x - fx, ey = g[k].y - fy, ez = g[k].z - fz;
         const double rr = fma(ex, ex, fma(ey, ey, ez * ez));
         const float rrf = (float)rr;
-        const float rinv = rrf > 0.f ? rsqrt_nr(rrf) : 0.f;
+        const float rinv = recip_mixed(rrf);
         t[k] = __fmul_rn(g[k].q, rinv);
         u[k] = __fmul_rn(q2[k], rinv);
         const float t3 = t[k] * rinv * rinv, u3 = u[k] * rinv * rinv;
