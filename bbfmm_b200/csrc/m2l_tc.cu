@@ -410,7 +410,11 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(TC2_THREADS, 1)
                    double *__restrict__ Lacc, int level, const int4 *__restrict__ offs, int kfirst, int ilead,
                    int split_chunks, int ncols, const double *__restrict__ Mlead, const double *__restrict__ Erow,
                    __nv_bfloat16 *__restrict__ Lsplit, int64_t nrows, const int4 *__restrict__ boxes,
-                   int nboxes, int lgeom, int nsets) {
+                   int nboxes, int lgeom, int nsets, int64_t part_stride) {
+  // blockIdx.y selects one of gridDim.y groups of the 189 offsets; with several, each writes its sums
+  // to its own slice of Lacc (part_stride doubles apart)
+  const int o_begin = 189 * (int)blockIdx.y / (int)gridDim.y, o_end = 189 * ((int)blockIdx.y + 1) / (int)gridDim.y;
+  Lacc += (int64_t)blockIdx.y * part_stride;
   constexpr int DNZ = 16;  // components the fused down projection takes in FP64
   constexpr int split_rows = TC_SPLIT_ROWS;
   extern __shared__ uint8_t smem_raw[];
@@ -516,7 +520,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(TC2_THREADS, 1)
     const uint32_t main_bytes = 2u * A2_BYTES + (uint32_t)ncols * BK2 * 2;  // of both CTAs
     constexpr uint32_t corr_bytes = 2u * (A2_BYTES + 2 * BC_BYTES);
     bool alive = true;
-    for (int o = 0; o < 189 && alive; ++o) {
+    for (int o = o_begin; o < o_end && alive; ++o) {
       const int4 ov = offs[cls * 189 + o];
       const int gx = cbx + ov.y, gy = cby + ov.z, gz = cbz + ov.w;
       const int scx = gx & 1, scy = gy & 1, scz = gz & 1;
@@ -566,7 +570,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(TC2_THREADS, 1)
       return true;
     };
     bool alive = true;
-    for (int o = 0; o < 189 && alive; ++o)
+    for (int o = o_begin; o < o_end && alive; ++o)
       for (int kc = 0; kc < nchunk && alive; ++kc) {
         uint32_t ahi, alo, ea, ec;
         alive = take(ahi, ea);
@@ -619,7 +623,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(TC2_THREADS, 1)
           row_cell(h * 128 + q * 32 + 8 * m + tr, aset[m], ax[m], ay[m], az[m], aok[m]);
         }
         __syncwarp();
-        for (int o = 0; o < 189; ++o) {
+        for (int o = o_begin; o < o_end; ++o) {
           const int4 ov = offs[cls * 189 + o];
           const int gx = cbx + ov.y, gy = cby + ov.z, gz = cbz + ov.w;
           const int scx = gx & 1, scy = gy & 1, scz = gz & 1;
@@ -719,6 +723,61 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(TC2_THREADS, 1)
   tc_fence_after();
   if (warp == 0) {
     asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(512) : "memory");
+  }
+}
+
+// Sums the ng slices of the two-box kernel's offset groups in a fixed order and writes what its
+// epilogue writes: FP64 outputs (with Lsplit only i < 32), and with Lsplit the split Morton rows. One
+// warp per cell, eight outputs a lane; with a box list (geometry lgeom) only the listed blocks' cells.
+__global__ void __launch_bounds__(256) tc2_sum_parts_kernel(int64_t cells, int ng, const double *__restrict__ part,
+                                                            int64_t stride, double *__restrict__ Lacc, int level, int ncols,
+                                                            __nv_bfloat16 *__restrict__ Lsplit, int64_t nrows,
+                                                            const int4 *__restrict__ boxes, int lgeom) {
+  constexpr int DNZ = 16;
+  const int lane = threadIdx.x & 31;
+  const int P = 1 << (level - 1);
+  const int64_t P3 = (int64_t)P * P * P;
+  if (8 * lane >= ncols) return;
+  for (int64_t w = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5; w < cells;
+       w += ((int64_t)gridDim.x * blockDim.x) >> 5) {
+    int64_t cell = w;
+    if (boxes) {  // w = (block, class, cell of the block)
+      const Tc2Box g{lgeom & 15, (lgeom >> 4) & 15, (lgeom >> 8) & 15};
+      const int4 b = boxes[w >> (g.lb() + 3)];
+      int x, y, z, none;
+      g.pos((int)(w & ((1 << g.lb()) - 1)), x, y, z, none);
+      cell = (int64_t)(b.x * 8 + ((w >> g.lb()) & 7)) * P3 + ((int64_t)(b.w + z) * P + b.z + y) * P + b.y + x;
+    }
+    double v[8] = {};
+    for (int gidx = 0; gidx < ng; ++gidx) {
+      const double2 *src = reinterpret_cast<const double2 *>(part + gidx * stride + cell * BN + 8 * lane);
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const double2 t = src[i];
+        v[2 * i] += t.x;
+        v[2 * i + 1] += t.y;
+      }
+    }
+    if (!Lsplit || lane < 4) {
+      double2 *dst = reinterpret_cast<double2 *>(Lacc + cell * BN + 8 * lane);
+#pragma unroll
+      for (int i = 0; i < 4; ++i) dst[i] = make_double2(v[2 * i], v[2 * i + 1]);
+    }
+    if (Lsplit) {
+      const int64_t in = cell % P3, sc = cell / P3;
+      const int x = (int)(in % P), y = (int)((in / P) % P), z = (int)(in / ((int64_t)P * P)), c = (int)(sc & 7);
+      const int64_t mrow =
+          (sc >> 3) * 8 * P3 + grid_to_morton(2 * x + ((c >> 2) & 1), 2 * y + ((c >> 1) & 1), 2 * z + (c & 1), level);
+      __align__(16) __nv_bfloat16 h[8], l[8];
+#pragma unroll
+      for (int i = 0; i < 8; ++i) {
+        const double t = 8 * lane + i < DNZ ? 0.0 : v[i];
+        h[i] = __double2bfloat16(t);
+        l[i] = __double2bfloat16(t - (double)__bfloat162float(h[i]));
+      }
+      *reinterpret_cast<uint4 *>(Lsplit + mrow * BN + 8 * lane) = *reinterpret_cast<const uint4 *>(h);
+      *reinterpret_cast<uint4 *>(Lsplit + (nrows + mrow) * BN + 8 * lane) = *reinterpret_cast<const uint4 *>(l);
+    }
   }
 }
 
@@ -1305,7 +1364,8 @@ bool tc_fuses_lead(const void *opsv, int nprod, int rank) {
 
 int launch_m2l_tc(int r, const void *Msplit, int64_t ncell_total, int64_t cell_offset, const void *opsv, double *Lacc,
                   int level, const int4 *offs, cudaStream_t s, int nsets, int nprod, int rank, const double *Mlead,
-                  const double *Erow, void *Lsplit, const int4 *boxes, int nboxes, int lgeom) {
+                  const double *Erow, void *Lsplit, const int4 *boxes, int nboxes, int lgeom, double *part, int64_t part_elems,
+                  int ngroups) {
   const TcOps *ops = (const TcOps *)opsv;
   if (nprod != 0 && nprod != 1 && nprod != 3)
     return bbfmm_set_error(BBFMM_ERR_ARG, "tensor-core products must be 0 (adaptive), 1 or 3");
@@ -1373,10 +1433,20 @@ int launch_m2l_tc(int r, const void *Msplit, int64_t ncell_total, int64_t cell_o
     if (boxes && nboxes == 0) return BBFMM_OK;
     const int64_t per_class = boxes ? (int64_t)((nboxes + spl - 1) / spl) : tc2_tiles(level, nsets) / 8;
     const int64_t tiles2 = 16 * ((per_class + 1) / 2);  // pairs of a class's tiles
-    tc::m2l_tc2_kernel<<<(unsigned)tiles2, tc::TC2_THREADS, tc::SMEM2_BYTES, s>>>(
-        mapAhi, mapAlo, mapBhi, ops->mapBhi_c, ops->mapBlo_c, Lacc, level, offs, kfirst, ilead, split_chunks, rank, fuse ? Mlead : nullptr,
-        fuse ? Erow : nullptr, (__nv_bfloat16 *)Lsplit, 8 * (int64_t)nsets * P * P * P, boxes, nboxes, lgeom, nsets);
-    return bbfmm_set_cuda_error(cudaGetLastError(), "m2l_tc2", __FILE__, __LINE__);
+    // offset groups need the leading block inside the kernel (or none), so that every slice is a sum
+    const int64_t ncell = 8 * (int64_t)nsets * P * P * P, count = ncell * r;
+    const int ng = part && ngroups > 1 && (fuse || ilead == 0) && ngroups * count <= part_elems ? ngroups : 1;
+    tc::m2l_tc2_kernel<<<dim3((unsigned)tiles2, ng), tc::TC2_THREADS, tc::SMEM2_BYTES, s>>>(
+        mapAhi, mapAlo, mapBhi, ops->mapBhi_c, ops->mapBlo_c, ng > 1 ? part : Lacc, level, offs, kfirst, ilead, split_chunks,
+        rank, fuse ? Mlead : nullptr, fuse ? Erow : nullptr, ng > 1 ? nullptr : (__nv_bfloat16 *)Lsplit, ncell, boxes, nboxes,
+        lgeom, nsets, ng > 1 ? count : 0);
+    cudaError_t e2 = cudaGetLastError();
+    if (e2 != cudaSuccess || ng == 1) return bbfmm_set_cuda_error(e2, "m2l_tc2", __FILE__, __LINE__);
+    const int64_t todo = boxes ? (int64_t)nboxes << (g2.lb() + 3) : ncell;
+    const int64_t sg = (todo + 7) / 8;
+    tc::tc2_sum_parts_kernel<<<(unsigned)(sg < 148 * 16 ? sg : 148 * 16), 256, 0, s>>>(
+        todo, ng, part, count, Lacc, level, rank, (__nv_bfloat16 *)Lsplit, ncell, boxes, lgeom);
+    return bbfmm_set_cuda_error(cudaGetLastError(), "m2l_tc2 parts", __FILE__, __LINE__);
   }
   static bool attr = false;
   if (!attr) {

@@ -232,9 +232,7 @@ int Solver<T>::alloc_partials() {
   int64_t need = 0;
   {  // every full M2L (FP64 DMMA or SIMT) may split its offsets
     for (int l = BBFMM_MINLEV; l <= maxlev; ++l) {
-      const bool tc = tc_m2l(l);
-      if (tc) continue;
-      const int g = m2l_groups(l);
+      const int g = tc_m2l(l) ? tc_groups(l) : m2l_groups(l);
       const int64_t e = dmma_part_elems(l, nsets, g, r);
       if (e > need) need = e;
     }
@@ -603,8 +601,9 @@ int Solver<T>::m2l_post(int l) {
         if (masked) BBFMM_CUDA_OK(cudaMemsetAsync(Lbuf, 0, sizeof(T) * (size_t)cells(l) * r, stream));
         TRY(launch_m2l_tc(r, Msplit, Mcells(), Moff[l] / r, tcops, (double *)Lbuf, l, offs, stream, nsets,
                           tc_products, rk(), (const double *)Ml, (const double *)Ert, presplit ? Lsplit : nullptr,
-                          region_tcboxes[l], region_ntcboxes[l], region_tcgeom[l]));
-        mark(ST_M2L, 1);
+                          region_tcboxes[l], region_ntcboxes[l], region_tcgeom[l], (double *)Lpart, Lpart_elems,
+                          tc_groups(l)));
+        mark(ST_M2L, tc_groups(l) > 1 ? 2 : 1);
       } else if (lead > 0) {
         TRY(m2l_fp(Ml, l, 0, lead, lead_rows));
         TRY(launch_m2l_tc(r, Msplit, Mcells(), Moff[l] / r, tcops, (double *)Lbuf, l, offs, stream, nsets,
@@ -612,8 +611,9 @@ int Solver<T>::m2l_post(int l) {
         mark(ST_M2L, 2);
       } else {
         TRY(launch_m2l_tc(r, Msplit, Mcells(), Moff[l] / r, tcops, (double *)Lbuf, l, offs, stream, nsets,
-                          tc_products, rk()));
-        mark(ST_M2L, 1);
+                          tc_products, rk(), nullptr, nullptr, nullptr, nullptr, 0, 0x111, (double *)Lpart, Lpart_elems,
+                          tc_groups(l)));
+        mark(ST_M2L, tc_groups(l) > 1 ? 2 : 1);
       }
     } else if (region_boxes[l]) {
       // a target region: only the blocks above active cells run (one offset group), the rest
@@ -688,7 +688,8 @@ int Solver<T>::time_m2l(int level, int reps, float *ms) {
       if (!split) rc = m2l_fp(Ml, level, 0, rk(), rk());
       else if (part == 0) rc = launch_m2l_tc(r, Msplit, Mcells(), Moff[level] / r, tcops, (double *)Lbuf, level, offs,
                                              stream, nsets, tc_products, rk(), fused ? (const double *)Ml : nullptr,
-                                             fused ? (const double *)Ert : nullptr, presplit ? Lsplit : nullptr);
+                                             fused ? (const double *)Ert : nullptr, presplit ? Lsplit : nullptr, nullptr,
+                                             0, 0x111, (double *)Lpart, Lpart_elems, tc_groups(level));
       else rc = lead > 0 && !fused ? m2l_fp(Ml, level, 0, lead, lead_rows) : BBFMM_OK;
     }
     cudaEventRecord(b, stream);
@@ -1194,7 +1195,8 @@ int Solver<T>::copy_m2l_morton(int level, T *host_out) {
     const bool fused = lead > 0 && tc_fuses_lead(tcops, tc_products, rk());
     if (lead > 0 && !fused) TRY(m2l_fp(Ml, level, 0, lead, lead_rows));
     TRY(launch_m2l_tc(r, Msplit, Mcells(), Moff[level] / r, tcops, (double *)Lbuf, level, offs, stream, nsets,
-                      tc_products, rk(), fused ? (const double *)Ml : nullptr, fused ? (const double *)Ert : nullptr));
+                      tc_products, rk(), fused ? (const double *)Ml : nullptr, fused ? (const double *)Ert : nullptr, nullptr,
+                      nullptr, 0, 0x111, (double *)Lpart, Lpart_elems, tc_groups(level)));
   } else {
     TRY(m2l_fp(Ml, level, 0, rk(), rk()));
   }

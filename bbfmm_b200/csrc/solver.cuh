@@ -126,7 +126,8 @@ constexpr int TC_SPLIT_CHUNKS = 2, TC_SPLIT_ROWS = 64;
 int launch_m2l_tc(int r, const void *Msplit, int64_t ncell_total, int64_t cell_offset, const void *ops, double *Lacc,
                   int level, const int4 *offs, cudaStream_t s, int nsets = 1, int nprod = 3, int rank = 0,
                   const double *Mlead = nullptr, const double *Erow = nullptr, void *Lsplit = nullptr,
-                  const int4 *boxes = nullptr, int nboxes = 0, int lgeom = 0x111);
+                  const int4 *boxes = nullptr, int nboxes = 0, int lgeom = 0x111, double *part = nullptr,
+                  int64_t part_elems = 0, int ngroups = 1);
 bool tc_fuses_lead(const void *ops, int nprod, int rank);
 // Whether launch_m2l_tc runs the two-box kernel (the adaptive product map at full split rows).
 inline bool tc_two_box(int nprod, int rank) { return nprod == 0 && (rank <= 0 || rank >= TC_SPLIT_ROWS); }
@@ -353,6 +354,16 @@ struct Solver {
   bool tc_m2l(int l) const {
     const int k = tune.m2l_kind[l];
     return k == 2 ? tc_level(l) : (k == 0 && tc_default(l));
+  }
+  // Offset groups of a level's two-box tensor-core M2L: a small level is a few tiles of 256 targets,
+  // each about 0.9 ms of 189 offsets one after the other, so up to nine CTAs share a tile's offsets
+  // where they find free SMs (level 4 of one set: 16 tiles on 144 SMs). By the whole level's tiles,
+  // so that a target region's cells get the sums of the unrestricted solve; one group where the
+  // leading block is another kernel's.
+  int tc_groups(int l) const {
+    if (!tc_two_box(tc_products, rk()) || (lead > 0 && !tc_fuses_lead(tcops, tc_products, rk()))) return 1;
+    const int64_t g = 148 / tc2_tiles(l, nsets);
+    return g < 1 ? 1 : (g > 9 ? 9 : (int)g);
   }
   // S rows -> Mall (cpg); F rows <- Lbuf (Morton, assign). Row t is cell row0 + t, or
   // rowlist[t] when a row list is given.

@@ -121,3 +121,23 @@ def test_heavy_leaves(count, n, mode):
     pot, fld = s.solve_fields(torch.as_tensor(q, dtype=s.dtype, device="cuda"))
     assert rel_l2(pot.double().cpu().numpy() * q, ref) < {"d": 1e-12, "s": 2e-5, "mixed": 3e-7}[mode]
     s.close()
+
+
+@pytest.mark.parametrize("lev,sets", [(2, 33), (3, 5), (3, 9), (4, 1), (4, 3)])
+def test_offset_groups_of_small_tensor_core_levels(lev, sets):
+    """Levels of a few tensor-core tiles split their offsets over CTAs: nine groups, fewer where
+    stacked sets fill more tiles (a partial last tile, an odd count of tiles per class)."""
+    import torch
+    from bbfmm_b200 import Batch
+    rng = np.random.default_rng(100 * lev + sets)
+    xs = [rng.random((300 * 2 ** (lev - 2) + 7 * k, 3)) - 0.5 for k in range(sets)]
+    out = {}
+    for mode in ("mixed", "d"):
+        b = Batch([(x, 8, lev) for x in xs], mode=mode)
+        q = np.random.default_rng(5).uniform(-1, 1, b.N)
+        out[mode] = b.solve(torch.as_tensor(q, device="cuda")).cpu().numpy()
+        off = b.offsets
+        b.close()
+    for k in range(sets):
+        a, e = int(off[k]), int(off[k + 1])
+        assert rel_l2(out["mixed"][a:e], out["d"][a:e]) < 3e-7
