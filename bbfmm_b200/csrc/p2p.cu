@@ -434,6 +434,75 @@ int near_work_build(int N, const int *leaf_start, int maxlev, int nsets, int thr
   return BBFMM_OK;
 }
 
+// Longest items first: a CTA takes one item, and the last CTAs of a clustered set's list, each walking
+// thousands of sources, would otherwise run alone (about 15% of the near field of 400,000 clustered
+// particles at depth 5). Items are dropped into buckets of about 19% of their cost, the sources a
+// thread walks; their results do not depend on the order.
+constexpr int NEAR_BUCKETS = 128;
+
+__device__ int near_bucket(const int *__restrict__ ls, int2 item, int N, int maxlev, int threads) {
+  float cost;
+  if (item.x < 0) {
+    const int64_t m = -(int64_t)item.x - 1, per = pow8i(maxlev), base = m - (m & (per - 1));
+    int ix, iy, iz, src = 0;
+    morton_to_grid(m & (per - 1), maxlev, ix, iy, iz);
+    const int n1 = 1 << maxlev;
+    for (int k = 0; k < 27; ++k) {
+      const int gx = ix + k / 9 - 1, gy = iy + (k / 3) % 3 - 1, gz = iz + k % 3 - 1;
+      if (gx < 0 || gx >= n1 || gy < 0 || gy >= n1 || gz < 0 || gz >= n1) continue;
+      const int64_t B = base + grid_to_morton(gx, gy, gz, maxlev);
+      src += max(0, clamp_n(ls[B + 1], N) - clamp_n(ls[B], N));
+    }
+    const int left = max(1, clamp_n(ls[m + 1], N) - clamp_n(ls[m], N) - item.y * threads);
+    cost = (float)src / (float)max(1, threads / min(left, threads));
+  } else {
+    const int n = max(0, clamp_n(ls[(int64_t)item.x * 64 + 64], N) - clamp_n(ls[(int64_t)item.x * 64], N));
+    cost = (float)((n + threads - 1) / threads) * 27.f * (float)n / 64.f;
+  }
+  const int b = (int)(4.f * log2f(cost + 1.f));
+  return NEAR_BUCKETS - 1 - min(b, NEAR_BUCKETS - 1);
+}
+
+__global__ void near_histogram_kernel(const int *__restrict__ ls, const int2 *__restrict__ items, int nitems, int N, int maxlev,
+                                      int threads, int *count) {
+  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < nitems; i += gridDim.x * blockDim.x)
+    atomicAdd(&count[near_bucket(ls, items[i], N, maxlev, threads)], 1);
+}
+
+__global__ void near_place_kernel(const int *__restrict__ ls, const int2 *__restrict__ items, int nitems, int N, int maxlev,
+                                  int threads, const int *count, int *used, int2 *__restrict__ out) {
+  __shared__ int start[NEAR_BUCKETS];
+  if (threadIdx.x == 0) {
+    int run = 0;
+    for (int b = 0; b < NEAR_BUCKETS; ++b) {
+      start[b] = run;
+      run += count[b];
+    }
+  }
+  __syncthreads();
+  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < nitems; i += gridDim.x * blockDim.x) {
+    const int b = near_bucket(ls, items[i], N, maxlev, threads);
+    out[start[b] + atomicAdd(&used[b], 1)] = items[i];
+  }
+}
+
+size_t near_order_bytes(int nitems) { return 2 * NEAR_BUCKETS * sizeof(int) + sizeof(int2) * (size_t)nitems; }
+
+// Puts the list that near_work_build left in `work` into that order (scratch: near_order_bytes).
+int near_order(int N, const int *leaf_start, int maxlev, int nsets, int threads, void *work, int nitems, void *scratch,
+               cudaStream_t s) {
+  if (nitems < 2) return BBFMM_OK;
+  int2 *items = const_cast<int2 *>(near_work_items(work, maxlev, nsets));
+  int *count = (int *)scratch, *used = count + NEAR_BUCKETS;
+  int2 *out = (int2 *)(used + NEAR_BUCKETS);
+  const int grid = nitems < 148 * 8 * 256 ? (nitems + 255) / 256 : 148 * 8;
+  BBFMM_CUDA_OK(cudaMemsetAsync(scratch, 0, 2 * NEAR_BUCKETS * sizeof(int), s));
+  near_histogram_kernel<<<grid, 256, 0, s>>>(leaf_start, items, nitems, N, maxlev, threads, count);
+  near_place_kernel<<<grid, 256, 0, s>>>(leaf_start, items, nitems, N, maxlev, threads, count, used, out);
+  BBFMM_CUDA_OK(cudaMemcpyAsync(items, out, sizeof(int2) * (size_t)nitems, cudaMemcpyDeviceToDevice, s));
+  return bbfmm_set_cuda_error(cudaGetLastError(), "near order", __FILE__, __LINE__);
+}
+
 // ------------------------------------------------------------------ the near-field kernel
 // RHS2: a second charge vector q2 (sorted order) whose potentials and fields go to pot2 and
 // fld2, from the same pair evaluations.

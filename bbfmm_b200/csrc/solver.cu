@@ -943,7 +943,13 @@ int Solver<T>::build_near_work() {
                       region_mask, region_level));
   if (flag) return bbfmm_set_error(BBFMM_ERR_ARG, "leaf offsets must rise from 0 to N without decreasing");
   near_threads = tune.p2p_threads;
-  return BBFMM_OK;
+  if (near_items < 2) return BBFMM_OK;
+  unsigned char *tmp = nullptr;  // longest items first
+  TRY(dalloc(&tmp, near_order_bytes(near_items)));
+  int rc = near_order(N, leaf_start, maxlev, nsets, near_threads, near_work, near_items, tmp, stream);
+  if (rc == BBFMM_OK) rc = bbfmm_set_cuda_error(cudaStreamSynchronize(stream), "near order", __FILE__, __LINE__);
+  cudaFree(tmp);
+  return rc;
 }
 
 // pot[i] = sum_j q_j / r_ij and fld[i] = grad pot at x_i (FMM), caller's order, no target

@@ -58,6 +58,9 @@ int near_work_build(int N, const int *leaf_start, int maxlev, int nsets, int thr
 int launch_near(int mode, int homogen, int N, const void *pos4, const int *leaf_start, int maxlev, const void *work,
                 int nsets, int nitems, int threads, void *pot, void *fld, cudaStream_t s,
                 const unsigned char *mask = nullptr, int mask_level = 0);
+size_t near_order_bytes(int nitems);
+int near_order(int N, const int *leaf_start, int maxlev, int nsets, int threads, void *work, int nitems, void *scratch,
+               cudaStream_t s);
 int near_status(int clear);
 int launch_near2(int mode, int N, const void *pos4, const int *leaf_start, int maxlev, const void *work, int nsets,
                  int nitems, int threads, const void *q2, void *pot, void *fld, void *pot2, void *fld2, cudaStream_t s,
