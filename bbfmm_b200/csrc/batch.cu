@@ -123,6 +123,11 @@ struct Batch {
       g.solver.reset(new Solver<T>());
       Solver<T> &sv = *g.solver;
       TRY_(sv.init(g.n, g.maxlev, L, mode, lead, lead_rows, device, nullptr));
+      // the mixed mode's stacked levels run on the tensor cores: folded operators are prepared only
+      // when a set of n = 8 is alone in its group (its levels 2-3 run as in a solver of its own)
+      bool alone = false;
+      for (const auto &o : by) alone = alone || (o.first.first == 8 && o.second.size() == 1);
+      sv.fold = mode != MODE_MIXED || alone;
       auto it = owner.find(g.n);
       if (it == owner.end()) {
         const int nn = g.n, n3 = nn * nn * nn, r = n3 / 2;

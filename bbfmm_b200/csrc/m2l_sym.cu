@@ -441,7 +441,7 @@ template <typename T>
 static bool sym_basis(int n, int r, const T *U, std::vector<double> &Q, int *cstart) {
   const int n3 = n * n * n, h = n / 2, hh = h * h * h;
   std::vector<std::vector<double>> cols;
-  std::vector<double> V((size_t)hh * r), G((size_t)r * r), d(r), q(r);
+  std::vector<double> V((size_t)hh * r), d(r), q(r);
   for (int p = 0; p < 8; ++p) {
     cstart[p] = (int)cols.size();
     for (int k = 0; k < r; ++k)
@@ -456,13 +456,10 @@ static bool sym_basis(int n, int r, const T *U, std::vector<double> &Q, int *cst
             }
             V[(size_t)((x * h + y) * h + z) * r + k] = v * 0.35355339059327376220;  // 1 / sqrt(8)
           }
-    std::fill(G.begin(), G.end(), 0.0);
-    for (int a = 0; a < hh; ++a) {
-      const double *v = V.data() + (size_t)a * r;
-      for (int i = 0; i < r; ++i)
-        for (int j = 0; j < r; ++j) G[(size_t)i * r + j] += v[i] * v[j];
+    for (int k = 0; k < r; ++k) {  // the diagonal of the Gram matrix; its columns are formed as they are taken
+      d[k] = 0.0;
+      for (int a = 0; a < hh; ++a) d[k] += V[(size_t)a * r + k] * V[(size_t)a * r + k];
     }
-    for (int k = 0; k < r; ++k) d[k] = G[(size_t)k * r + k];
     for (;;) {
       double m = 0.0;
       for (int k = 0; k < r; ++k) {
@@ -473,11 +470,17 @@ static bool sym_basis(int n, int r, const T *U, std::vector<double> &Q, int *cst
       if (cols.size() == (size_t)r) return false;
       int k = 0;
       while (d[k] < 0.5 * m) ++k;
-      std::copy(G.begin() + (size_t)k * r, G.begin() + (size_t)(k + 1) * r, q.begin());
+      std::fill(q.begin(), q.end(), 0.0);
+      for (int a = 0; a < hh; ++a) {
+        const double *v = V.data() + (size_t)a * r;
+        for (int i = 0; i < r; ++i) q[i] += v[k] * v[i];
+      }
       for (int pass = 0; pass < 2; ++pass)  // against every earlier column: Q is orthogonal to rounding
         for (const auto &c : cols) {
-          double t = 0.0;
-          for (int i = 0; i < r; ++i) t += c[i] * q[i];
+          double t4[4] = {};
+          for (int i = 0; i < r; i += 4)
+            for (int e = 0; e < 4; ++e) t4[e] += c[i + e] * q[i + e];
+          const double t = (t4[0] + t4[1]) + (t4[2] + t4[3]);
           for (int i = 0; i < r; ++i) q[i] -= t * c[i];
         }
       double nn = 0.0;
