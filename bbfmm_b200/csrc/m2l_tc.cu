@@ -864,6 +864,13 @@ __device__ __forceinline__ void pair_bar(int q) {  // the two epilogue warps of 
   asm volatile("bar.sync %0, 64;" ::"r"(1 + q) : "memory");
 }
 
+// The [hi | lo] BF16 split of x at element e of the two planes.
+__device__ __forceinline__ void split_to(__nv_bfloat16 *__restrict__ hi, __nv_bfloat16 *__restrict__ lo, int64_t e, double x) {
+  const __nv_bfloat16 h = __double2bfloat16(x);
+  hi[e] = h;
+  lo[e] = __double2bfloat16(x - (double)__bfloat162float(h));
+}
+
 template <bool UP>
 __global__ void __launch_bounds__(PD_THREADS, 1)
     proj_fused_kernel(const __grid_constant__ CUtensorMap mapAhi, const __grid_constant__ CUtensorMap mapAlo,
@@ -871,7 +878,8 @@ __global__ void __launch_bounds__(PD_THREADS, 1)
                       const double *__restrict__ Lfp, int ldl, const double *__restrict__ Dlead,
                       double *__restrict__ F, int ldf, int64_t rows, int level, int64_t row0, int kc0, int kc1,
                       const double *__restrict__ cs, double scale, int64_t ntiles, int col_skip,
-                      const int64_t *__restrict__ rowlist) {
+                      const int64_t *__restrict__ rowlist, __nv_bfloat16 *__restrict__ Shi = nullptr,
+                      __nv_bfloat16 *__restrict__ Slo = nullptr) {
   constexpr int ncb = UP ? 1 : 2;  // 256-column blocks: r = 256 outputs up, n3 = 512 down
   extern __shared__ uint8_t smem_raw[];
   const uint32_t raw = smem_u32(smem_raw);
@@ -1042,12 +1050,18 @@ __global__ void __launch_bounds__(PD_THREADS, 1)
 #pragma unroll
           for (int rr = 0; rr < 16; ++rr) {
             const int64_t o = UP ? __shfl_sync(0xffffffffu, orow, rr) : tq + 16 * h + rr;
-            F[o * ldf + n0 + lane] = sc * stg[(16 * h + rr) * PD_SROW + lane];
+            const double x = sc * stg[(16 * h + rr) * PD_SROW + lane];
+            F[o * ldf + n0 + lane] = x;
+            if (UP) split_to(Shi, Slo, o * ldf + n0 + lane, x);
           }
         } else {
           for (int rr = 0; rr < 16; ++rr) {
             const int64_t o = UP ? __shfl_sync(0xffffffffu, orow, rr) : tq + 16 * h + rr;
-            if (16 * h + rr < nrow) F[o * ldf + n0 + lane] = sc * stg[(16 * h + rr) * PD_SROW + lane];
+            if (16 * h + rr < nrow) {
+              const double x = sc * stg[(16 * h + rr) * PD_SROW + lane];
+              F[o * ldf + n0 + lane] = x;
+              if (UP) split_to(Shi, Slo, o * ldf + n0 + lane, x);
+            }
           }
         }
       }
@@ -1305,10 +1319,11 @@ int launch_proj_down(const void *pv, const void *Asplit, const double *Lfp, int6
 }
 
 // Up projection of `rows` Morton rows (row0 ..) of `level`: M[cpg(row0 + t)][j] = sum_l S'[t][l]
-// Bup[l][j] from the split S rows (Asplit, rows x n3), assigned for every j; the split operator
-// is zero for j < lead, whose FP64 values proj_narrow_kernel writes afterwards.
+// Bup[l][j] from the split S rows (Asplit, rows x n3), assigned for every j, with its BF16 split in
+// the planes Mhi and Mlo (what the tensor-core M2L reads); the split operator is zero for j < lead,
+// whose FP64 values and split proj_narrow_kernel writes afterwards.
 int launch_proj_up(const void *pv, const void *Asplit, int64_t rows, double *M, int level, int64_t row0,
-                   cudaStream_t s, const int64_t *rowlist) {
+                   cudaStream_t s, const int64_t *rowlist, void *Mhi, void *Mlo) {
   const TcProj *p = (const TcProj *)pv;
   if (!p) return bbfmm_set_error(BBFMM_ERR_STATE, "tensor-core projections not prepared");
   if (rows <= 0) return BBFMM_OK;
@@ -1329,7 +1344,7 @@ int launch_proj_up(const void *pv, const void *Asplit, int64_t rows, double *M, 
   const int grid = (int)(ntiles < 148 ? ntiles : 148);
   tc::proj_fused_kernel<true><<<grid, tc::PD_THREADS, tc::PD_SMEM, s>>>(
       ahi, alo, p->up_hi, p->up_lo, nullptr, 0, nullptr, M, p->r, rows, level, row0, 0, p->n3 / tc::BK, nullptr, 1.0,
-      ntiles, 0, rowlist);
+      ntiles, 0, rowlist, (__nv_bfloat16 *)Mhi, (__nv_bfloat16 *)Mlo);
   return bbfmm_set_cuda_error(cudaGetLastError(), "proj_up", __FILE__, __LINE__);
 }
 
@@ -1344,12 +1359,9 @@ int tc_split_rows(int64_t rows, int K, const double *src, int gather, int level,
   return bbfmm_set_cuda_error(cudaGetLastError(), "split", __FILE__, __LINE__);
 }
 
-// Msplit = [hi plane | lo plane], each ncell_total * r bf16, same cell order as M.
-int tc_split_multipoles(int r, int64_t ncell, const double *M, int lead, void *Msplit, cudaStream_t s) {
-  (void)lead;
-  __nv_bfloat16 *hi = (__nv_bfloat16 *)Msplit;
-  __nv_bfloat16 *lo = hi + (size_t)ncell * r;
-  tc::split_kernel<<<148 * 8, 256, 0, s>>>(ncell * r, M, hi, lo, 0, 0, 0);
+// The [hi | lo] BF16 split of `count` multipole values (levels that the FP64 projection wrote).
+int tc_split_multipoles(int64_t count, const double *M, void *hi, void *lo, cudaStream_t s) {
+  tc::split_kernel<<<148 * 8, 256, 0, s>>>(count, M, (__nv_bfloat16 *)hi, (__nv_bfloat16 *)lo, 0, 0, 0);
   return bbfmm_set_cuda_error(cudaGetLastError(), "split multipoles", __FILE__, __LINE__);
 }
 

@@ -6,6 +6,8 @@
 // C[out(m)][n] = scale * cs[n] * sum_k A[in(m)][k] B[k][n] with rows remapped between
 // Morton and cpg order. CTA tile 64 rows x BN columns (256 or 64), K-chunks of 16 in a
 // four-stage cp.async ring, 8 warps in a 2 x 4 grid of 32 x BN / 4 warp tiles.
+#include <cuda_bf16.h>
+
 #include "common.cuh"
 
 namespace bbfmm {
@@ -133,7 +135,8 @@ __global__ void __launch_bounds__(256, 1) proj_dmma_kernel(int64_t M, int K, int
 
 // Narrow form for the FP64 leading columns of the mixed-mode up projection:
 // C[out(m)][0:16] = sum_k A[m][k] B[k][0:16], CTA tile 128 rows x 16 columns, 8 warps of
-// 16 rows, K-chunks of 16 double-buffered with cp.async; rows of C ldc apart.
+// 16 rows, K-chunks of 16 double-buffered with cp.async; rows of C ldc apart. The BF16 split of the
+// values goes to the planes Chi and Clo.
 namespace nw {
 constexpr int BM = 128, BN = 16, BK = 16, AST = BK + 4, BST = BN + 8;
 constexpr int STAGE = BM * AST + BK * BST;
@@ -143,7 +146,9 @@ constexpr int SMEM_BYTES = 2 * STAGE * 8;
 __global__ void __launch_bounds__(256) proj_narrow_kernel(int64_t M, int K, const double *__restrict__ A,
                                                           const double *__restrict__ B, double *__restrict__ C,
                                                           int ldc, int level, int mapmode, int64_t row0,
-                                                          const int64_t *__restrict__ rows) {
+                                                          const int64_t *__restrict__ rows,
+                                                          __nv_bfloat16 *__restrict__ Chi,
+                                                          __nv_bfloat16 *__restrict__ Clo) {
   extern __shared__ __align__(16) double smem[];
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, r8 = lane >> 2, c4 = lane & 3;
   const int64_t m0 = (int64_t)blockIdx.x * nw::BM;
@@ -202,17 +207,24 @@ __global__ void __launch_bounds__(256) proj_narrow_kernel(int64_t M, int K, cons
   for (int mf = 0; mf < 2; ++mf) {
     const int64_t m = m0 + warp * 16 + mf * 8 + r8;
     if (m >= M) continue;
-    double *dst = C + remap(m, row0, rows, level, mapmode == MAP_OUT_CPG) * ldc;
+    const int64_t at = remap(m, row0, rows, level, mapmode == MAP_OUT_CPG) * ldc;
 #pragma unroll
-    for (int nf = 0; nf < NF; ++nf)
-      *reinterpret_cast<double2 *>(dst + nf * 8 + 2 * c4) = make_double2(acc[mf][nf][0], acc[mf][nf][1]);
+    for (int nf = 0; nf < NF; ++nf) {
+      const int64_t e = at + nf * 8 + 2 * c4;
+      const double x = acc[mf][nf][0], y = acc[mf][nf][1];
+      *reinterpret_cast<double2 *>(C + e) = make_double2(x, y);
+      const __nv_bfloat16 hx = __double2bfloat16(x), hy = __double2bfloat16(y);
+      *reinterpret_cast<__nv_bfloat162 *>(Chi + e) = __nv_bfloat162(hx, hy);
+      *reinterpret_cast<__nv_bfloat162 *>(Clo + e) = __nv_bfloat162(__double2bfloat16(x - (double)__bfloat162float(hx)),
+                                                                    __double2bfloat16(y - (double)__bfloat162float(hy)));
+    }
   }
 }
 
 }  // namespace pj
 
 int launch_proj_narrow(int64_t M, int K, const double *A, const double *B, double *C, int ldc, int level,
-                       int mapmode, cudaStream_t s, int64_t row0, const int64_t *rows) {
+                       int mapmode, cudaStream_t s, int64_t row0, const int64_t *rows, void *Chi, void *Clo) {
   if (K % pj::nw::BK) return bbfmm_set_error(BBFMM_ERR_ARG, "narrow projection: K must be a multiple of 16");
   if (M <= 0) return BBFMM_OK;
   static bool attr = false;  // 47 KB of dynamic shared memory
@@ -223,7 +235,7 @@ int launch_proj_narrow(int64_t M, int K, const double *A, const double *B, doubl
     attr = true;
   }
   pj::proj_narrow_kernel<<<(unsigned)((M + pj::nw::BM - 1) / pj::nw::BM), 256, pj::nw::SMEM_BYTES, s>>>(
-      M, K, A, B, C, ldc, level, mapmode, row0, rows);
+      M, K, A, B, C, ldc, level, mapmode, row0, rows, (__nv_bfloat16 *)Chi, (__nv_bfloat16 *)Clo);
   return bbfmm_set_cuda_error(cudaGetLastError(), "proj_narrow", __FILE__, __LINE__);
 }
 

@@ -305,6 +305,7 @@ int Solver<T>::alloc_work() {
     unsigned char *p = nullptr;
     TRY(dalloc(&p, tc_split_bytes(r, tot / r)));
     Msplit = p;
+    BBFMM_CUDA_OK(cudaMemsetAsync(Msplit, 0, tc_split_bytes(r, tot / r), stream));  // as Mall
   }
   return BBFMM_OK;
 }
@@ -468,10 +469,11 @@ int Solver<T>::upward(const void *q_dev, int q_is_double) {
     TRY(proj_up(count(l), S[l & 1], l, 0, false, local_solve ? src_list[l] : nullptr));
     mark(ST_PROJ_UP);
   }
-  if (mode == MODE_MIXED && tcops) {
-    TRY(tc_split_multipoles(r, Mcells(), (const double *)Mall, lead, Msplit, stream));
-    mark(ST_PROJ_UP);
-  }
+  for (int l = lowest; l <= maxlev; ++l)
+    if (split_later[l]) {
+      TRY(tc_split_multipoles(cells(l) * r, (const double *)(Mall + Moff[l]), msplit_hi(l), msplit_lo(l), stream));
+      mark(ST_PROJ_UP);
+    }
   return BBFMM_OK;
 }
 
@@ -505,15 +507,17 @@ int Solver<T>::proj_up(int64_t rows, const T *S_rows, int level, int64_t row0, b
   T *Mdst = Mall + Moff[level];
   if (r == 32) return launch_proj_r32<T>(true, rows, S_rows, P32, nullptr, (T)1, Mdst, level, row0, rowlist, stream);
   msym[level] = sym_level(level);
+  split_later[level] = mode == MODE_MIXED && tcops && !msym[level] && (!proj_tc() || rows > Ssplit_rows);
   if (!proj_tc() || rows > Ssplit_rows || msym[level])
     return launch_proj_dmma<T>(rows, n3, r, S_rows, msym[level] ? Bup_sym : Bup, nullptr, (T)1, Mdst, level, MAP_OUT_CPG,
                                stream, row0, 0, rowlist);
   // the tensor cores write all r columns (zero for j < PROJ_LEAD: those operator rows are
   // zero in the split copy), then the FP64 pass overwrites the leading columns
   if (!presplit) TRY(tc_split_rows(rows, n3, (const double *)S_rows, 0, level, row0, Ssplit, stream));
-  TRY(launch_proj_up(tcproj, Ssplit, rows, (double *)Mdst, level, row0, stream, rowlist));
+  TRY(launch_proj_up(tcproj, Ssplit, rows, (double *)Mdst, level, row0, stream, rowlist, msplit_hi(level),
+                     msplit_lo(level)));
   return launch_proj_narrow(rows, n3, (const double *)S_rows, (const double *)Bup_lead, (double *)Mdst, r, level,
-                            MAP_OUT_CPG, stream, row0, rowlist);
+                            MAP_OUT_CPG, stream, row0, rowlist, msplit_hi(level), msplit_lo(level));
 }
 
 // Down projection of the level's M2L output (Lbuf, cpg) into `rows` F rows (Morton cells

@@ -99,7 +99,7 @@ int launch_proj_dmma(int64_t M, int K, int N, const T *A, const T *B, const T *c
                      cudaStream_t s, int64_t row0 = 0, int lda = 0, const int64_t *rows = nullptr);
 // C[out(m)][0:32] = sum_k A[m][k] B[k][0:32] on the FP64 tensor path (B: K x 32 contiguous).
 int launch_proj_narrow(int64_t M, int K, const double *A, const double *B, double *C, int ldc, int level,
-                       int mapmode, cudaStream_t s, int64_t row0, const int64_t *rows = nullptr);
+                       int mapmode, cudaStream_t s, int64_t row0, const int64_t *rows, void *Chi, void *Clo);
 int launch_direct_fp64(int N, const double *xyz, const double *q, int nt, const int *targets, double *out, cudaStream_t s);
 int launch_direct_field_fp64(int N, const double *xyz, const double *q, int nt, const int *targets, double *pot,
                              double *fld, cudaStream_t s);
@@ -111,7 +111,7 @@ struct TcOperators;
 int tc_supported();
 int tc_prepare_operators(int r, const double *Ert, int lead, int lead_rows, void **out, cudaStream_t s);
 void tc_free_operators(void *ops);
-int tc_split_multipoles(int r, int64_t ncell, const double *M, int lead, void *Msplit, cudaStream_t s);
+int tc_split_multipoles(int64_t count, const double *M, void *hi, void *lo, cudaStream_t s);
 size_t tc_split_bytes(int r, int64_t ncell);
 // nprod: 3 = hi*hi + hi*lo + lo*hi (split BF16) for every term, 1 = hi*hi only (plain BF16
 // products), 0 = adaptive: the three products for components j < 32 TC_SPLIT_CHUNKS and
@@ -144,7 +144,7 @@ int launch_proj_down(const void *p, const void *Asplit, const double *Lfp, int64
                      int64_t row0, const double *cs, double scale, cudaStream_t s, int rank = 0,
                      const int64_t *rowlist = nullptr);
 int launch_proj_up(const void *p, const void *Asplit, int64_t rows, double *M, int level, int64_t row0, cudaStream_t s,
-                   const int64_t *rowlist = nullptr);
+                   const int64_t *rowlist, void *Mhi, void *Mlo);
 // rowlist (optional): the pass's Morton rows, row t being rowlist[t] instead of row0 + t
 int tc_split_rows(int64_t rows, int K, const double *src, int gather, int level, int64_t row0, void *dst,
                   cudaStream_t s, int zlead = 0, const int64_t *rowlist = nullptr);
@@ -235,6 +235,11 @@ struct Solver {
   // pass are in the rotated basis
   bool sym_level(int l) const { return sym_on() && !tc_m2l(l); }
   bool msym[11] = {};
+  // Msplit of a level: the BF16 planes that the up projection writes beside M; split_later: the level
+  // was projected in FP64 and is split at the end of the upward pass
+  void *msplit_hi(int l) const { return (char *)Msplit + 2 * Moff[l]; }
+  void *msplit_lo(int l) const { return (char *)Msplit + 2 * (Moff[l] + Mcells() * r); }
+  bool split_later[11] = {};
   int m2l_groups(int l) const {  // offset (or step) groups of the level's FP64 / FP32 M2L
     // (of a target region's short block lists: up to 8, the scratch of small levels only)
     if (region_boxes[l] && sym_on() && cells(l) <= 4096) return 8;
