@@ -23,12 +23,12 @@
 // 12 doubles and the B fragments (the operators in step order, 27 KB a step, by cp.async) are both
 // read without bank conflicts, and double-buffered with one barrier a step.
 //
-// Bound by the FP64 tensor path (37 TFLOP/s measured; its pipe is active 45% of the time) and the
-// latency of a step with three warps per scheduler: offsets and validity come from small shared
-// tables, because the integer work of finding eight sources was the larger part of a step's
-// instructions (262,144 particles, depth 5: 16.1 -> 13.75 ms of M2L with the tables; the unfolded
-// FP64 M2L takes 57.6 ms there). Letting some warps multiply first and form tiles afterwards made
-// no difference (13.76 ms) and is not done.
+// Bound by the FP64 tensor path (37 TFLOP/s measured) and the latency of a step with three warps per
+// scheduler: the path is busy about half of the time. Offsets and validity come from small shared
+// tables, because finding eight sources by integer arithmetic was the larger part of a step's
+// instructions. M2L of 262,144 particles, depth 5: unfolded FP64 57.6 ms, folded 16.1 ms, with the
+// tables 12.8 ms. Warps that multiply first and form tiles afterwards (13.8 ms) and twice the warps
+// with half the targets each (15.8 ms) were slower.
 #include <cmath>
 #include <cstring>
 #include <vector>
