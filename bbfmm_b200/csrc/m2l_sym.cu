@@ -475,11 +475,14 @@ static bool sym_basis(int n, int r, const T *U, std::vector<double> &Q, int *cst
         const double *v = V.data() + (size_t)a * r;
         for (int i = 0; i < r; ++i) q[i] += v[k] * v[i];
       }
-      for (int pass = 0; pass < 2; ++pass)  // against every earlier column: Q is orthogonal to rounding
-        for (const auto &c : cols) {
+      // against the class's earlier columns, then against every earlier one (the classes are
+      // orthogonal to about 1e-13 as they are; after that to rounding)
+      for (int pass = 0; pass < 2; ++pass)
+        for (size_t e = pass == 0 ? cstart[p] : 0; e < cols.size(); ++e) {
+          const std::vector<double> &c = cols[e];
           double t4[4] = {};
           for (int i = 0; i < r; i += 4)
-            for (int e = 0; e < 4; ++e) t4[e] += c[i + e] * q[i + e];
+            for (int k4 = 0; k4 < 4; ++k4) t4[k4] += c[i + k4] * q[i + k4];
           const double t = (t4[0] + t4[1]) + (t4[2] + t4[3]);
           for (int i = 0; i < r; ++i) q[i] -= t * c[i];
         }

@@ -200,9 +200,9 @@ __global__ void __launch_bounds__(128) p2m_join_kernel(const int4 *__restrict__ 
   p2m_store<T, NN>(acc, prefac * prefac * prefac, lane, h.x - m0, count, S, Ssplit);
 }
 
-// The leaves (rows of a pass: cells, or the cells of a row list) above `cap` particles: with items
-// null only counts (counts[0] items of at most cap particles, counts[1] leaves), else writes
-// items (row, p0, p1, cell) and heavy (row, first item, items, cell), in no particular order of leaves.
+// The leaves (rows of a pass: cells, or the cells of a row list) above `cap` particles: items of at
+// most cap particles (row, p0, p1, cell) and heavy (row, first item, items, cell), in no particular
+// order of leaves; counts: how many of each.
 __global__ void heavy_kernel(const int *__restrict__ leaf_start, const int64_t *__restrict__ rows, int64_t count, int cap,
                              int *counts, int4 *items, int4 *heavy) {
   for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < count; t += (int64_t)gridDim.x * blockDim.x) {
@@ -211,7 +211,6 @@ __global__ void heavy_kernel(const int *__restrict__ leaf_start, const int64_t *
     if (p1 - p0 <= cap) continue;
     const int n = (p1 - p0 + cap - 1) / cap;
     const int i0 = atomicAdd(&counts[0], n), h = atomicAdd(&counts[1], 1);
-    if (!items) continue;
     heavy[h] = make_int4((int)t, i0, n, (int)m);
     for (int i = 0; i < n; ++i)
       items[i0 + i] = make_int4((int)t, p0 + i * cap, min(p1, p0 + (i + 1) * cap), (int)m);

@@ -174,12 +174,11 @@ int Solver<T>::set_operators(const T *U, const T *E) {
   BBFMM_CUDA_OK(cudaDeviceSynchronize());
   transpose_blocks_kernel<T><<<dim3(r / 32, r / 32, BBFMM_NUM_OFFSETS), dim3(32, 8), 0, stream>>>(r, Ecol, Ert);
   BBFMM_CUDA_OK(cudaGetLastError());
-  BBFMM_CUDA_OK(cudaStreamSynchronize(stream));
   if (r == 32) {
     if (!B32) TRY(dalloc(&B32, r32_pack_doubles()));
     TRY(r32_pack<T>(Ecol, B32, stream));
-    BBFMM_CUDA_OK(cudaStreamSynchronize(stream));
   }
+  BBFMM_CUDA_OK(cudaStreamSynchronize(stream));
   if (symops) sym_free(symops);
   symops = nullptr;
   if (fold && U && r == 256) {
@@ -342,8 +341,8 @@ int Solver<T>::set_particles_global(int nsets_, int N_, const int *perm_h, const
   if (N > 0) BBFMM_CUDA_OK(cudaMemcpy(perm, perm_h, sizeof(int) * N, cudaMemcpyHostToDevice));
   BBFMM_CUDA_OK(cudaMemcpy(leaf_start, leaf_start_h, sizeof(int) * (nl + 1), cudaMemcpyHostToDevice));
   BBFMM_CUDA_OK(cudaDeviceSynchronize());
+  TRY(build_near_work());  // refuses offsets out of order
   TRY(build_heavy());
-  TRY(build_near_work());
   if (N > 0) {
     T *xyz_d = nullptr;
     TRY(dalloc(&xyz_d, 3 * (size_t)Nxyz));
@@ -402,8 +401,8 @@ int Solver<T>::set_particles_sets_device(int nsets_, const int *off_h, const int
   TRY(dalloc(&pos4, 4 * (size_t)(N > 0 ? N : 1)));
   TRY(dalloc(&phis, N > 0 ? N : 1));
   TRY(build_tree_device_sets<T>(nsets, off_h, count_h, xyz_d, (T)L, maxlev, perm, leaf_start, stream));
+  TRY(build_near_work());  // refuses offsets out of order
   TRY(build_heavy());
-  TRY(build_near_work());
   if (N > 0) TRY((launch_gather<T, T>(N, perm, xyz_d, nullptr, pos4, stream)));
   TRY(alloc_work());
   BBFMM_CUDA_OK(cudaStreamSynchronize(stream));
@@ -746,8 +745,8 @@ int Solver<T>::set_target_region(int level, const unsigned char *active_host) {
   if (pos4) TRY(alloc_partials());
   TRY(build_local());
   if (!pos4) return BBFMM_OK;
-  TRY(build_heavy());
-  return build_near_work();
+  TRY(build_near_work());
+  return build_heavy();
 }
 
 template <typename T>
@@ -770,59 +769,46 @@ void Solver<T>::free_local() {
 
 template <typename T>
 void Solver<T>::free_heavy() {
-  for (HeavyLeaves *h : {&heavy_up, &heavy_down}) {
-    if (h->part) cudaFree(h->part);
-    if (h == &heavy_up || h->items != heavy_up.items) {
-      if (h->items) cudaFree(h->items);
-      if (h->heavy) cudaFree(h->heavy);
-    }
-  }
+  for (void *p : {(void *)heavy_mem[0], (void *)heavy_mem[1], heavy_up.part})
+    if (p) cudaFree(p);
+  heavy_mem[0] = heavy_mem[1] = nullptr;
   heavy_up = heavy_down = HeavyLeaves();
 }
 
 // Lists of the leaves of more than `cap` particles among the rows of P2M and of L2P (the same rows
-// unless the solve is local). cap: 64 (measured: a warp takes about 10 us for that), more above a
-// million particles so that the partial sums stay below 16,384 + N / cap rows.
+// unless the solve is local). cap: 64 (a warp takes about 10 us for that), more above a million
+// particles so that the partial sums stay below 16,384 + N / cap rows. A leaf of n > cap particles
+// has at most 2 n / cap chunks, which bounds the lists before they are counted.
 template <typename T>
 int Solver<T>::build_heavy() {
   free_heavy();
-  const int cap = 64 * (int)(((int64_t)N + (1 << 20) - 1) / (1 << 20) > 1 ? ((int64_t)N + (1 << 20) - 1) / (1 << 20) : 1);
-  int *counts = nullptr;
-  TRY(dalloc(&counts, 2));
-  auto list = [&](HeavyLeaves &h, const int64_t *rows, int64_t count, bool parts) -> int {
-    int c[2] = {0, 0};
-    BBFMM_CUDA_OK(cudaMemsetAsync(counts, 0, 8, stream));
-    TRY(launch_heavy(leaf_start, rows, count, cap, counts, nullptr, nullptr, stream));
-    BBFMM_CUDA_OK(cudaMemcpyAsync(c, counts, 8, cudaMemcpyDeviceToHost, stream));
-    BBFMM_CUDA_OK(cudaStreamSynchronize(stream));
+  const int64_t mega = ((int64_t)N + (1 << 20) - 1) >> 20;
+  const int cap = 64 * (int)(mega > 1 ? mega : 1);
+  const size_t nh = (size_t)N / cap + 1, ni = 2 * nh;
+  auto list = [&](HeavyLeaves &h, int4 **mem, const int64_t *rows, int64_t count) -> int {
+    TRY(dalloc(mem, 1 + ni + nh));  // counts, items, leaves
+    int c[2] = {0, 0}, *counts = (int *)*mem;
     h.cap = cap;
-    if (c[0] == 0) return BBFMM_OK;
-    TRY(dalloc(&h.items, c[0]));
-    TRY(dalloc(&h.heavy, c[1]));
-    if (parts) {
-      T *p = nullptr;
-      TRY(dalloc(&p, (size_t)c[0] * n3));
-      h.part = p;
-    }
+    h.items = *mem + 1;
+    h.heavy = h.items + ni;
     BBFMM_CUDA_OK(cudaMemsetAsync(counts, 0, 8, stream));
     TRY(launch_heavy(leaf_start, rows, count, cap, counts, h.items, h.heavy, stream));
+    BBFMM_CUDA_OK(cudaMemcpyAsync(c, counts, 8, cudaMemcpyDeviceToHost, stream));
+    BBFMM_CUDA_OK(cudaStreamSynchronize(stream));
     h.nitems = c[0];
     h.nheavy = c[1];
     return BBFMM_OK;
   };
-  int rc = local_solve ? list(heavy_up, src_list[maxlev], n_src[maxlev], true) : list(heavy_up, nullptr, cells(maxlev), true);
-  if (rc == BBFMM_OK) {
-    if (local_solve) {
-      rc = list(heavy_down, tgt_list[maxlev], n_tgt[maxlev], false);
-    } else {
-      heavy_down = heavy_up;
-      heavy_down.part = nullptr;
-    }
+  TRY(list(heavy_up, &heavy_mem[0], local_solve ? src_list[maxlev] : nullptr, local_solve ? n_src[maxlev] : cells(maxlev)));
+  if (heavy_up.nitems > 0) {
+    T *p = nullptr;
+    TRY(dalloc(&p, (size_t)heavy_up.nitems * n3));
+    heavy_up.part = p;
   }
-  if (rc == BBFMM_OK) rc = bbfmm_set_cuda_error(cudaStreamSynchronize(stream), "heavy leaves", __FILE__, __LINE__);
-  cudaFree(counts);
-  if (rc != BBFMM_OK) free_heavy();
-  return rc;
+  heavy_down = heavy_up;
+  heavy_down.part = nullptr;
+  if (local_solve) TRY(list(heavy_down, &heavy_mem[1], tgt_list[maxlev], n_tgt[maxlev]));
+  return BBFMM_OK;
 }
 
 // Runs of the region cells (tgt) and of those with their neighbours (src) at region_level,
@@ -941,19 +927,15 @@ int Solver<T>::build_region_tiles() {
 // synchronisation: the item count sizes the launch).
 template <typename T>
 int Solver<T>::build_near_work() {
-  if (!near_work) TRY(dalloc((unsigned char **)&near_work, near_work_bytes(N, maxlev, nsets)));
+  if (!near_work) TRY(dalloc((unsigned char **)&near_work, near_work_bytes(N, maxlev, nsets) + near_order_bytes(N)));
   int flag = 0;
   TRY(near_work_build(N, leaf_start, maxlev, nsets, tune.p2p_threads, near_work, stream, &near_items, &flag,
                       region_mask, region_level));
   if (flag) return bbfmm_set_error(BBFMM_ERR_ARG, "leaf offsets must rise from 0 to N without decreasing");
   near_threads = tune.p2p_threads;
-  if (near_items < 2) return BBFMM_OK;
-  unsigned char *tmp = nullptr;  // longest items first
-  TRY(dalloc(&tmp, near_order_bytes(near_items)));
-  int rc = near_order(N, leaf_start, maxlev, nsets, near_threads, near_work, near_items, tmp, stream);
-  if (rc == BBFMM_OK) rc = bbfmm_set_cuda_error(cudaStreamSynchronize(stream), "near order", __FILE__, __LINE__);
-  cudaFree(tmp);
-  return rc;
+  // longest items first, through scratch behind the list
+  return near_order(N, leaf_start, maxlev, nsets, near_threads, near_work, near_items,
+                    (char *)near_work + near_work_bytes(N, maxlev, nsets), stream);
 }
 
 // pot[i] = sum_j q_j / r_ij and fld[i] = grad pot at x_i (FMM), caller's order, no target

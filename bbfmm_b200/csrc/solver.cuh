@@ -125,7 +125,8 @@ constexpr int TC_SPLIT_CHUNKS = 2, TC_SPLIT_ROWS = 64;
 // boxes (nboxes entries of set, x0, y0, z0): run only the targets of these blocks of parent
 // cells, of 2^lx x 2^ly x 2^lz cells (lgeom = lx | ly << 4 | lz << 8, 8 to 256 cells, origins
 // multiples of the extents), 256 / cells per tile; the outputs of the other cells are not
-// written.
+// written. part (part_elems doubles), ngroups: the two-box kernel's offsets split over ngroups CTAs
+// per tile through slices of part, where they fit and the leading block is inside the kernel.
 int launch_m2l_tc(int r, const void *Msplit, int64_t ncell_total, int64_t cell_offset, const void *ops, double *Lacc,
                   int level, const int4 *offs, cudaStream_t s, int nsets = 1, int nprod = 3, int rank = 0,
                   const double *Mlead = nullptr, const double *Erow = nullptr, void *Lsplit = nullptr,
@@ -341,6 +342,7 @@ struct Solver {
   int set_target_region(int level, const unsigned char *active_host);  // level < 0 clears
   int set_m2l_first(int level);                                        // m2l_first, then the runs
   HeavyLeaves heavy_up, heavy_down;  // of the rows that P2M and L2P run over
+  int4 *heavy_mem[2] = {};           // their lists
   int build_heavy();
   void free_heavy();
   int build_local();                                                   // runs and row lists
