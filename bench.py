@@ -41,8 +41,6 @@ TC_DRAM_BYTES_PER_CELL = (885159936 + 299155712) / 262144
 SMS, MAX_SM_MHZ = 148, 1965.0
 # FP64 tensor (DMMA) peak: 128 FP64 flops per clock per SM (profiles/m2l_lead_n8_level5.md)
 DMMA_TFLOPS = SMS * 128 * MAX_SM_MHZ * 1e6 / 1e12
-# FP32 SIMT peak (an FMA as two flops per lane, 128 lanes per SM)
-FP32_TFLOPS = SMS * 256 * MAX_SM_MHZ * 1e6 / 1e12
 # Near-field roof: min(FP32 issue / 7 FP32 operations per pair, reciprocal
 # square roots at 16 per clock per SM), in pairs/s at the maximum SM clock
 P2P_ROOF_PAIRS = min(SMS * 128 * MAX_SM_MHZ * 1e6 / 7, SMS * 16 * MAX_SM_MHZ * 1e6)
@@ -1048,15 +1046,14 @@ def main():
                 "traffic_note": "ncu DRAM bytes of the level-6 launch (split rows written) scaled by cells",
                 "flop_per_launch": exec_flop, "launch_ms": m2l_ms}
     else:
-        flop = 2.0 * r * r * I_leaf
+        # n = 8: the 189 products of a cell fold to 39.5 (mirrored offsets); n = 4: 2 r^2 per pair.
+        # Both run on the FP64 tensor path in either precision.
+        flop = 2.0 * r * r * (39.5 * 8 ** lev if r == 256 else I_leaf)
         achieved = flop / (m2l_ms / 1e3) / 1e12
-        fp64 = args.mode == "d" and r == 256
-        peak = DMMA_TFLOPS if fp64 else FP32_TFLOPS
-        roof = {"kernel": "m2l_dmma_kernel (leaf level)" if fp64 else "m2l_simt_kernel (leaf level)",
-                "bound": "tensor" if fp64 else "fp32", "achieved": achieved, "peak": peak, "unit": "TFLOP/s",
-                "frac": achieved / peak,
-                "peak_source": "FP64 tensor (DMMA) rate, 128 flops/clock/SM at 1965 MHz" if fp64 else
-                               "FP32 FMA rate, 128 lanes/SM at 1965 MHz",
+        roof = {"kernel": "m2l_sym_kernel (leaf level)" if r == 256 else "m2l_r32_kernel (leaf level)",
+                "bound": "tensor", "achieved": achieved, "peak": DMMA_TFLOPS, "unit": "TFLOP/s",
+                "frac": achieved / DMMA_TFLOPS,
+                "peak_source": "FP64 tensor (DMMA) rate, 128 flops/clock/SM at 1965 MHz",
                 "traffic": None, "flop_per_launch": flop, "launch_ms": m2l_ms}
     # near field and passes: pairs exact from the tree, bytes of the passes
     counts = leaf_counts(x, lev)
