@@ -611,16 +611,15 @@ int sym_prepare(int n, int r, const T *U, const T *Ecol, double tol, const T *Bu
   return cleanup(BBFMM_OK);
 }
 
-// dst[c][i] = sum_i' Q(i, i') src[c][i'] for `cells` rows of r: rows of the rotated basis back in
-// the given one.
+// `cells` rows of r (a multiple of 64) from the rotated basis to the given one, dst[c][i] =
+// sum_i' Q(i, i') src[c][i'], or the other way, dst[c][i'] = sum_i Q(i, i') src[c][i].
 template <typename T>
-int sym_to_given(const void *op, int64_t cells, const T *src, T *dst, cudaStream_t s) {
+int sym_rotate(const void *op, bool to_given, int64_t cells, const T *src, T *dst, cudaStream_t s) {
   const SymOps *o = (const SymOps *)op;
   const int r = sy::R;
-  // rows in blocks of 64 (levels hold 64 or more cells)
-  sy::gemm_kernel<T, double, T><<<dim3((unsigned)(cells / 64), r / 64, 1), 256, 0, s>>>(r, src, r, 1, 0, o->Q, 1, r, 0, dst,
-                                                                                     r, 1, 0);
-  return bbfmm_set_cuda_error(cudaGetLastError(), "sym_to_given", __FILE__, __LINE__);
+  sy::gemm_kernel<T, double, T><<<dim3((unsigned)(cells / 64), r / 64, 1), 256, 0, s>>>(
+      r, src, r, 1, 0, o->Q, to_given ? 1 : r, to_given ? r : 1, 0, dst, r, 1, 0);
+  return bbfmm_set_cuda_error(cudaGetLastError(), "sym_rotate", __FILE__, __LINE__);
 }
 
 static int64_t sym_tiles(int level, int nsets) {
@@ -686,7 +685,7 @@ int launch_m2l_sym(const void *op, const T *M, T *Lout, int level, T *part, int6
 #define SYM_INST(T)                                                                                                   \
   template int sym_prepare<T>(int, int, const T *, const T *, double, const T *, const T *, T *, T *, void **,        \
                               cudaStream_t);                                                                          \
-  template int sym_to_given<T>(const void *, int64_t, const T *, T *, cudaStream_t);                                  \
+  template int sym_rotate<T>(const void *, bool, int64_t, const T *, T *, cudaStream_t);                              \
   template int launch_m2l_sym<T>(const void *, const T *, T *, int, T *, int64_t, cudaStream_t, int, int, const int4 *, int);
 SYM_INST(double)
 SYM_INST(float)

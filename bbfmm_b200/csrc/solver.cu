@@ -479,11 +479,11 @@ int Solver<T>::upward(const void *q_dev, int q_is_double) {
 // r = 32 and mirror-symmetric operators run on the FP64 tensor path in either precision, other
 // r = 256 operators there in FP64 and on CUDA cores in FP32.
 template <typename T>
-int Solver<T>::m2l_fp(const T *Ml, int level, int j0, int j1, int ni, const int4 *boxes, int nboxes) {
+int Solver<T>::m2l_fp(const T *Ml, int level, int j0, int j1, int ni, bool folded, const int4 *boxes, int nboxes) {
   if (r == 32)
     return launch_m2l_r32<T>(B32, Ml, Lbuf, level, offs, Lpart, Lpart_elems, stream, nsets, m2l_groups(level), boxes,
                              nboxes);
-  if (msym[level])
+  if (folded)
     return launch_m2l_sym<T>(symops, Ml, Lbuf, level, Lpart, Lpart_elems, stream, nsets, m2l_groups(level), boxes, nboxes);
   if (sizeof(T) == 8 && r == 256)
     return launch_m2l_dmma(r, (const double *)Ml, (const double *)Ecol, (double *)Lbuf, level, j0, j1, ni, offs,
@@ -622,10 +622,10 @@ int Solver<T>::m2l_post(int l) {
       // a target region: only the blocks above active cells run (one offset group), the rest
       // of the output is zero
       BBFMM_CUDA_OK(cudaMemsetAsync(Lbuf, 0, sizeof(T) * (size_t)cells(l) * r, stream));
-      TRY(m2l_fp(Ml, l, 0, rk(), rk(), region_boxes[l], region_nboxes[l]));
+      TRY(m2l_fp(Ml, l, 0, rk(), rk(), msym[l], region_boxes[l], region_nboxes[l]));
       mark(ST_M2L, 1);
     } else {
-      TRY(m2l_fp(Ml, l, 0, rk(), rk()));
+      TRY(m2l_fp(Ml, l, 0, rk(), rk(), msym[l]));
       int g = m2l_groups(l);
       if ((int64_t)g * cells(l) * r > Lpart_elems) g = 1;
       mark(ST_M2L, g > 1 ? 2 : 1);  // groups add the partial sum
@@ -668,7 +668,8 @@ int Solver<T>::solve(const void *q_dev, void *phi_dev, int io_double) {
 }
 
 // Re-runs the M2L of one level `reps` times between two events on the solver's stream
-// (multipoles of the last solve as input) and reports the mean time per launch group.
+// (multipoles of the last solve as input, in whichever basis they are: the time does not depend on
+// it) and reports the mean time per launch group.
 template <typename T>
 int Solver<T>::time_m2l(int level, int reps, float *ms) {
   if (level < BBFMM_MINLEV || level > maxlev || reps < 1) return bbfmm_set_error(BBFMM_ERR_ARG, "bad level/reps");
@@ -676,8 +677,7 @@ int Solver<T>::time_m2l(int level, int reps, float *ms) {
   BBFMM_CUDA_OK(cudaEventCreate(&a));
   BBFMM_CUDA_OK(cudaEventCreate(&b));
   const T *Ml = Mall + Moff[level];
-  const bool split = tc_m2l(level);
-  msym[level] = sym_level(level);  // the launch that the current tuning makes
+  const bool split = tc_m2l(level), folded = sym_level(level);  // the launch that the current choices make
   const bool fused = split && lead > 0 && tc_fuses_lead(tcops, tc_products, rk());
   // the launch as the solve makes it: a whole level with the mixed projections also writes
   // the split rows of the down projection (m2l_post)
@@ -688,7 +688,7 @@ int Solver<T>::time_m2l(int level, int reps, float *ms) {
   for (int part = 0; part < (split ? 2 : 1) && rc == BBFMM_OK; ++part) {
     cudaEventRecord(a, stream);
     for (int i = 0; i < reps && rc == BBFMM_OK; ++i) {
-      if (!split) rc = m2l_fp(Ml, level, 0, rk(), rk());
+      if (!split) rc = m2l_fp(Ml, level, 0, rk(), rk(), folded);
       else if (part == 0) rc = launch_m2l_tc(r, Msplit, Mcells(), Moff[level] / r, tcops, (double *)Lbuf, level, offs,
                                              stream, nsets, tc_products, rk(), fused ? (const double *)Ml : nullptr,
                                              fused ? (const double *)Ert : nullptr, presplit ? Lsplit : nullptr, nullptr,
@@ -1095,7 +1095,6 @@ int Solver<T>::autotune(const void *q_dev, int io_double) {
     g_tune_cache[key] = pick;
   }
   TRY(alloc_partials());
-  TRY(upward(q_dev, io_double));  // multipoles in the bases that the choices take
   // near field: threads per block
   char key[96];
   snprintf(key, sizeof(key), "p2p/%d/%d/%d", mode, bucket(N), bucket(cells(maxlev)));
@@ -1152,7 +1151,7 @@ int Solver<T>::copy_rows_morton(const T *rows, int level, T *host_out) {
   int rc = launch_morton_cpg<T>(level, r, rows, tmp, 1, stream);
   if (rc == BBFMM_OK && msym[level]) {
     rc = dalloc(&given, (size_t)pow8i(level) * r);
-    if (rc == BBFMM_OK) rc = sym_to_given<T>(symops, pow8i(level), tmp, given, stream);
+    if (rc == BBFMM_OK) rc = sym_rotate<T>(symops, true, pow8i(level), tmp, given, stream);
   }
   if (rc == BBFMM_OK) {
     cudaError_t e = cudaMemcpyAsync(host_out, given ? given : tmp, sizeof(T) * pow8i(level) * r, cudaMemcpyDeviceToHost,
@@ -1172,6 +1171,30 @@ int Solver<T>::copy_multipoles_morton(int level, T *host_out) {
   return copy_rows_morton(Mall + Moff[level], level, host_out);
 }
 
+// Brings the stored multipoles of a level to the basis (and, for the tensor cores, the split) that
+// the current choices take, where the rank or the M2L kind has changed since they were projected.
+template <typename T>
+int Solver<T>::stored_basis(int level) {
+  if (!symops || msym[level] == sym_level(level)) return BBFMM_OK;
+  const int64_t n = cells(level), block = n < 4096 ? n : 4096;
+  T *tmp = nullptr, *Ml = Mall + Moff[level];
+  TRY(dalloc(&tmp, (size_t)block * r));
+  int rc = BBFMM_OK;
+  for (int64_t a = 0; a < n && rc == BBFMM_OK; a += block) {  // every block a multiple of 64, as n
+    const int64_t c = n - a < block ? n - a : block;
+    rc = sym_rotate<T>(symops, msym[level], c, Ml + a * r, tmp, stream);
+    if (rc == BBFMM_OK)
+      rc = bbfmm_set_cuda_error(cudaMemcpyAsync(Ml + a * r, tmp, sizeof(T) * c * r, cudaMemcpyDeviceToDevice, stream),
+                                "rotate multipoles", __FILE__, __LINE__);
+  }
+  cudaFree(tmp);  // waits for the copies
+  TRY(rc);
+  msym[level] = !msym[level];
+  if (Msplit && tcops && !msym[level])
+    TRY(tc_split_multipoles(n * r, (const double *)Ml, msplit_hi(level), msplit_lo(level), stream));
+  return BBFMM_OK;
+}
+
 // The M2L output of one level (L = sum E_k M over the interaction lists, before the post-M2L
 // projection and its scale), recomputed from the multipoles of the last solve with the launch
 // choices of the solve (the mixed mode's tensor-core kernel writing its full FP64 output), r
@@ -1181,8 +1204,9 @@ int Solver<T>::copy_m2l_morton(int level, T *host_out) {
   if (level < BBFMM_MINLEV || level > maxlev) return bbfmm_set_error(BBFMM_ERR_ARG, "level out of range");
   if (nsets != 1) return bbfmm_set_error(BBFMM_ERR_UNSUPPORTED, "M2L copies are per single-set solver");
   if (!pos4 || !Lbuf) return bbfmm_set_error(BBFMM_ERR_STATE, "particles not set");
+  TRY(stored_basis(level));
   const T *Ml = Mall + Moff[level];
-  const bool split = tc_m2l(level) && !msym[level];
+  const bool split = tc_m2l(level);
   if (split) {
     const bool fused = lead > 0 && tc_fuses_lead(tcops, tc_products, rk());
     if (lead > 0 && !fused) TRY(m2l_fp(Ml, level, 0, lead, lead_rows));
@@ -1190,7 +1214,7 @@ int Solver<T>::copy_m2l_morton(int level, T *host_out) {
                       tc_products, rk(), fused ? (const double *)Ml : nullptr, fused ? (const double *)Ert : nullptr, nullptr,
                       nullptr, 0, 0x111, (double *)Lpart, Lpart_elems, tc_groups(level)));
   } else {
-    TRY(m2l_fp(Ml, level, 0, rk(), rk()));
+    TRY(m2l_fp(Ml, level, 0, rk(), rk(), msym[level]));
   }
   return copy_rows_morton(Lbuf, level, host_out);
 }

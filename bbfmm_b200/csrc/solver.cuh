@@ -88,7 +88,7 @@ int sym_prepare(int n, int r, const T *U, const T *Ecol, double tol, const T *Bu
                 void **out, cudaStream_t s);
 void sym_free(void *ops);
 template <typename T>
-int sym_to_given(const void *ops, int64_t cells, const T *src, T *dst, cudaStream_t s);
+int sym_rotate(const void *ops, bool to_given, int64_t cells, const T *src, T *dst, cudaStream_t s);
 int sym_default_groups(int level, int nsets);
 template <typename T>
 int launch_m2l_sym(const void *ops, const T *M, T *Lout, int level, T *part, int64_t part_elems, cudaStream_t s,
@@ -232,10 +232,12 @@ struct Solver {
   T *Bup_sym = nullptr, *Bdn_sym = nullptr;
   double *B32 = nullptr, *P32 = nullptr;  // r = 32: operators and projections in fragment order
   bool sym_on() const { return symops && rank_eff == 0; }
-  // whether the level's solve runs the folded M2L, and whether its multipoles of the last upward
-  // pass are in the rotated basis
+  // whether the level's solve runs the folded M2L under the current choices, and whether the
+  // multipoles stored for it are in the rotated basis (set where they are written: by the up
+  // projection, and by stored_basis, which brings them to the choices' basis)
   bool sym_level(int l) const { return sym_on() && !tc_m2l(l); }
   bool msym[11] = {};
+  int stored_basis(int level);
   // Msplit of a level: the BF16 planes that the up projection writes beside M; split_later: the level
   // was projected in FP64 and is split at the end of the upward pass
   void *msplit_hi(int l) const { return (char *)Msplit + 2 * Moff[l]; }
@@ -400,8 +402,8 @@ struct Solver {
   int copy_m2l_morton(int level, T *host_out);         // level's M2L output, recomputed, Morton order
   void mark(int stage, int launches = 1);
   int time_m2l(int level, int reps, float *ms);
-  int m2l_fp(const T *Ml, int level, int j0, int j1, int ni,  // FP64 (DMMA) / FP32 (SIMT) M2L part
-             const int4 *boxes = nullptr, int nboxes = 0);
+  int m2l_fp(const T *Ml, int level, int j0, int j1, int ni,  // FP64 (DMMA) / FP32 (SIMT) M2L part,
+             bool folded = false, const int4 *boxes = nullptr, int nboxes = 0);  // or the folded M2L
   void release();
 };
 

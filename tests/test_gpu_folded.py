@@ -141,3 +141,77 @@ def test_offset_groups_of_small_tensor_core_levels(lev, sets):
     for k in range(sets):
         a, e = int(off[k]), int(off[k + 1])
         assert rel_l2(out["mixed"][a:e], out["d"][a:e]) < 3e-7
+
+
+def _after_a_change(s, q, level, change):
+    """multipoles() and m2l_output() of a level before and after `change` and a timing call, with no
+    solve in between."""
+    import torch
+    s.solve(torch.as_tensor(q, dtype=s.dtype, device="cuda"))
+    before = s.multipoles(level), s.m2l_output(level)
+    change()
+    s.time_m2l(level, 1)
+    return before, (s.multipoles(level), s.m2l_output(level))
+
+
+@pytest.mark.parametrize("level,kinds", [(3, (0, 2)), (3, (2, 0)), (4, (0, 1)), (4, (1, 0))])
+def test_read_back_after_a_change_of_the_m2l_kind(level, kinds):
+    """Mixed mode, a level moved between the folded FP64 M2L and the tensor cores: the multipoles
+    stay those of the solve (1e-13: one rotation to the operators' basis) and the M2L output is
+    theirs under either kind (1e-6, the tolerance of the tensor-core M2L elsewhere)."""
+    from bbfmm_b200 import Solver
+    x, q = uniform_inputs(3000, seed=level)
+    s = Solver(8, 4, 1.0, mode="mixed")
+
+    def kind(k):
+        t = s.tuning()
+        t["m2l_kind"][level] = k
+        s.set_tuning(t)
+
+    kind(kinds[0])
+    s.set_particles(x)
+    (m0, l0), (m1, l1) = _after_a_change(s, q, level, lambda: kind(kinds[1]))
+    assert rel_l2(m1, m0) < 1e-13
+    assert rel_l2(l1.ravel(), l0.ravel()) < 1e-6
+    s.close()
+
+
+@pytest.mark.parametrize("mode", ["d", "s"])
+@pytest.mark.parametrize("ranks", [(0, 160), (160, 0)])
+def test_read_back_after_a_change_of_the_rank(mode, ranks):
+    """The rank set (which takes the unfolded kernel, components below it) or cleared after the
+    solve: the multipoles stay, and the M2L output is that of the rank in force."""
+    from bbfmm_b200 import _lib
+    from bbfmm_b200 import operators as ops
+    level, r = 3, 256
+    x, q = uniform_inputs(3000, seed=9)
+    U, E = _ops(8, single=mode == "s")
+    from bbfmm_b200 import Solver
+    s = Solver(8, 3, 1.0, mode=mode, operators=(U, E))
+    rank = lambda k: _lib.check(_lib.lib().bbfmm_b200_set_rank(s.h, k))
+    rank(ranks[0])
+    s.set_particles(x)
+    (m0, _), (m1, l1) = _after_a_change(s, q, level, lambda: rank(ranks[1]))
+    tol = 1e-12 if mode == "d" else 2e-5
+    assert rel_l2(m1.astype(float), m0.astype(float)) < (1e-13 if mode == "d" else 1e-6)
+    k = ranks[1] or r
+    if k != r:
+        U, E = ops.truncate_operators(8, U, E, k)
+    cells = np.arange(0, 8 ** level, 37)
+    want = Oracle("d").m2l_sample(level, r, E.astype(float), m1.astype(float), cells)
+    assert rel_l2(l1[cells][:, :k].astype(float).ravel(), np.asarray(want).reshape(len(cells), r)[:, :k].ravel()) < tol
+    s.close()
+
+
+def test_autotune_leaves_the_multipoles_in_the_given_basis():
+    import torch
+    from bbfmm_b200 import Solver
+    x, q = uniform_inputs(4000, seed=2)
+    s = Solver(8, 4, 1.0, mode="mixed")
+    s.set_particles(x)
+    s.solve(torch.as_tensor(q, dtype=s.dtype, device="cuda"))
+    want = [s.multipoles(l) for l in (2, 3, 4)]
+    s.autotune(torch.as_tensor(q, dtype=s.dtype, device="cuda"))
+    for l, w in zip((2, 3, 4), want):
+        assert rel_l2(s.multipoles(l), w) < 3e-7
+    s.close()
