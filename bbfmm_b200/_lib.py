@@ -13,6 +13,7 @@ LIB_PATH = os.path.join(HERE, "lib", "libbbfmm_b200.so")
 
 MODE_D, MODE_S, MODE_MIXED = 0, 1, 2
 MODES = {"d": MODE_D, "s": MODE_S, "mixed": MODE_MIXED}
+M2L_FORMS = ["dense", "folded", "r32", "tensor"]
 STAGES = ["gather", "p2m", "m2m", "proj_up", "m2l", "proj_down", "l2l", "l2p", "p2p", "scatter"]
 
 ERRORS = {1: "argument", 2: "cuda", 3: "out of memory", 4: "unsupported", 5: "state"}
@@ -54,6 +55,7 @@ def lib() -> C.CDLL:
         L.bbfmm_b200_copy_m2l.argtypes = [vp, i, vp]
         L.bbfmm_b200_set_target_region.argtypes = [vp, i, vp]
         L.bbfmm_b200_set_first_m2l_level.argtypes = [vp, i]
+        L.bbfmm_b200_m2l_form.argtypes = [vp, i, ip]
         L.bbfmm_b200_time_m2l.argtypes = [vp, i, i, C.POINTER(C.c_float)]
         L.bbfmm_b200_direct.argtypes = [i, vp, vp, i, vp, vp, vp]
         L.bbfmm_b200_direct_field.argtypes = [i, vp, vp, i, vp, vp, vp, vp]

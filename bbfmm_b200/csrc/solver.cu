@@ -1425,6 +1425,14 @@ int bbfmm_b200_copy_m2l(bbfmm_b200_solver *h, int level, void *host_out) {
   return h->d->copy_m2l_morton(level, (double *)host_out);
 }
 
+int bbfmm_b200_m2l_form(const bbfmm_b200_solver *h, int level, int *form) {
+  if (!h || !form) return bbfmm_set_error(BBFMM_ERR_ARG, "null argument");
+  const int maxlev = h->f ? h->f->maxlev : h->d->maxlev;
+  if (level < BBFMM_MINLEV || level > maxlev) return bbfmm_set_error(BBFMM_ERR_ARG, "level out of range");
+  *form = h->f ? h->f->m2l_form(level) : h->d->m2l_form(level);
+  return BBFMM_OK;
+}
+
 int bbfmm_b200_time_m2l(bbfmm_b200_solver *h, int level, int reps, float *ms) {
   if (!h || !ms) return bbfmm_set_error(BBFMM_ERR_ARG, "null argument");
   return h->f ? h->f->time_m2l(level, reps, ms) : h->d->time_m2l(level, reps, ms);

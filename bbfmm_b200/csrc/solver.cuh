@@ -236,6 +236,10 @@ struct Solver {
   // multipoles stored for it are in the rotated basis (set where they are written: by the up
   // projection, and by stored_basis, which brings them to the choices' basis)
   bool sym_level(int l) const { return sym_on() && !tc_m2l(l); }
+  int m2l_form(int l) const {
+    return r == 32 ? BBFMM_B200_M2L_R32
+                   : (tc_m2l(l) ? BBFMM_B200_M2L_TENSOR : (sym_on() ? BBFMM_B200_M2L_FOLDED : BBFMM_B200_M2L_DENSE));
+  }
   bool msym[11] = {};
   int stored_basis(int level);
   // Msplit of a level: the BF16 planes that the up projection writes beside M; split_later: the level

@@ -258,6 +258,13 @@ class Solver:
         nl = _lib.lib().bbfmm_b200_stage_times(self.h, ms, len(_lib.STAGES))
         return dict(zip(_lib.STAGES, list(ms))), nl
 
+    def m2l_form(self, level: int) -> str:
+        """The form of the level's M2L under the current rank and tuning: "dense", "folded" (n = 8
+        operators with mirror symmetry), "r32" (n = 4) or "tensor" (mixed mode)."""
+        form = C.c_int()
+        _lib.check(_lib.lib().bbfmm_b200_m2l_form(self.h, int(level), C.byref(form)))
+        return _lib.M2L_FORMS[form.value]
+
     def time_m2l(self, level: int, reps: int = 3):
         ms = (C.c_float * 2)()
         _lib.check(_lib.lib().bbfmm_b200_time_m2l(self.h, level, reps, ms))

@@ -154,9 +154,18 @@ BBFMM_B200_API int bbfmm_b200_copy_multipoles(bbfmm_b200_solver *s, int level, v
 /* The M2L output of one level -- the level's slice of what the reference's m2l_drv writes
  * into L (m2l_drv.cu:14-19; PF of anotherFMMInteraction): L(F) = sum_{S in IL(F)} E_k M(S),
  * before the post-M2L projection and its (1/L_l)^homogeneity scale -- recomputed from the
- * multipoles of the last solve with that solve's kernels (MIXED: the tensor-core kernel with
- * its full FP64 output), r values per cell in the reference's Morton cell order. */
+ * multipoles of the last solve with the kernels of the current rank and tuning (MIXED: the
+ * tensor-core kernel with its full FP64 output), r values per cell in the reference's Morton cell order. */
 BBFMM_B200_API int bbfmm_b200_copy_m2l(bbfmm_b200_solver *s, int level, void *host_out);
+
+/* The form of one level's M2L under the current rank, tuning and operators: form[0] = one of the
+ * values below. Operators whose basis does not split into parity classes, or whose mirror images
+ * differ by more than their rounding, are never folded. */
+#define BBFMM_B200_M2L_DENSE 0  /* n = 8: every offset's product, FP64 on the FP64 tensor path or FP32 on CUDA cores */
+#define BBFMM_B200_M2L_FOLDED 1 /* n = 8: mirrored offsets folded, FP64 tensor path */
+#define BBFMM_B200_M2L_R32 2    /* n = 4, FP64 tensor path */
+#define BBFMM_B200_M2L_TENSOR 3 /* MIXED: split BF16 on the tensor cores */
+BBFMM_B200_API int bbfmm_b200_m2l_form(const bbfmm_b200_solver *s, int level, int *form);
 
 /* Re-run the M2L of one level `reps` times (inputs of the last solve), each launch as the
  * solve makes it, between CUDA events on the solver's stream: ms[0] = mean time of the main

@@ -215,3 +215,37 @@ def test_autotune_leaves_the_multipoles_in_the_given_basis():
     for l, w in zip((2, 3, 4), want):
         assert rel_l2(s.multipoles(l), w) < 3e-7
     s.close()
+
+
+def _forms(n, mode, lev=4, operators=None, **kw):
+    from bbfmm_b200 import Solver
+    s = Solver(n, lev, 1.0, mode=mode, operators=operators, **kw)
+    f = [s.m2l_form(l) for l in range(2, lev + 1)]
+    s.close()
+    return f
+
+
+def test_the_form_of_the_m2l():
+    """Which M2L runs: the tests above pass on the dense kernels too, so the form is stated here."""
+    assert _forms(8, "d") == _forms(8, "s") == ["folded"] * 3
+    assert _forms(8, "mixed") == ["folded", "folded", "tensor"]
+    for mode in ("d", "s", "mixed"):
+        assert _forms(4, mode) == ["r32"] * 3
+    # a rank cut, kernels odd in an axis or with a basis of mixed parity
+    assert _forms(8, "d", rank=128) == ["dense"] * 3
+    for kernel in ("laplacianforce", "oneoverr4"):
+        assert _forms(8, "d", kernel=kernel) == ["dense"] * 3
+
+
+def test_the_form_of_other_operators():
+    """The rotated basis of test_any_basis_of_the_same_span is folded, the operator changed in
+    test_operators_without_the_symmetry_take_the_general_path is not."""
+    r, n3 = 256, 512
+    U, E = _ops(8)
+    Q, _ = np.linalg.qr(np.random.default_rng(1).standard_normal((r, r)))
+    U2 = np.ascontiguousarray((U.reshape(r, n3).T @ Q).T.reshape(-1))
+    E2 = np.ascontiguousarray((Q.T @ E.reshape(316, r, r).transpose(0, 2, 1) @ Q).transpose(0, 2, 1).reshape(-1))
+    assert _forms(8, "d", operators=(U2, E2)) == ["folded"] * 3
+    E = E.copy()
+    E[5 * r * r:6 * r * r] *= 1.5
+    assert _forms(8, "d", operators=(U, E)) == ["dense"] * 3
