@@ -30,7 +30,7 @@
 // tables 12.8 ms. Warps that multiply first and form tiles afterwards (13.8 ms) and twice the warps
 // with half the targets each (15.8 ms) were slower.
 #include <cmath>
-#include <cstring>
+#include <limits>
 #include <vector>
 
 #include "solver.cuh"
@@ -363,36 +363,77 @@ __device__ __forceinline__ int class_of(const Classes &cl, int i) {
   while (i >= cl.cstart[p + 1]) ++p;
   return p;
 }
-__device__ __forceinline__ void atomic_max_nonneg(double *dst, double v) {  // v >= 0 (NaN counts as largest)
-  atomicMax((unsigned long long *)dst, (unsigned long long)__double_as_longlong(v));
+
+// One thread per component pair e = i r + j. Eavg[o] (row-major) = mean over the eight sign choices s
+// of S_s E'_{s a} S_s for each orbit o (words ax | ay << 2 | az << 4), E' row-major per offset;
+// off[e] = the pair's largest distance of an image from the mean (NaN is kept), mx the largest |E'|,
+// over all orbits.
+__global__ void __launch_bounds__(256) average_kernel(const double *__restrict__ Ep, const int *__restrict__ kt,
+                                                      const int *__restrict__ orbits, int norb, Classes cl,
+                                                      double *__restrict__ Eavg, double *__restrict__ off, double *mx) {
+  const int e = blockIdx.x * blockDim.x + threadIdx.x;
+  const int u = class_of(cl, e / R) ^ class_of(cl, e % R);
+  double most = 0.0, far = 0.0;
+  for (int o = 0; o < norb; ++o) {
+    const int w = orbits[o], a[3] = {w & 3, (w >> 2) & 3, (w >> 4) & 3};
+    double v[8], sum = 0.0;
+#pragma unroll
+    for (int s = 0; s < 8; ++s) {
+      const int x = s & 4 ? -a[0] : a[0], y = s & 2 ? -a[1] : a[1], z = s & 1 ? -a[2] : a[2];
+      const double t = Ep[(int64_t)kt[49 * (x + 3) + 7 * (y + 3) + z + 3] * R * R + e];
+      v[s] = __popc(s & u) & 1 ? -t : t;
+      sum += v[s];
+      most = fmax(most, fabs(t));
+    }
+    sum *= 0.125;
+#pragma unroll
+    for (int s = 0; s < 8; ++s) {
+      const double d = fabs(v[s] - sum);
+      if (d > far || d != d) far = d;
+    }
+    Eavg[(int64_t)o * R * R + e] = sum;
+  }
+  off[e] = far;
+  __shared__ double s_most[256];
+  s_most[threadIdx.x] = most;
+  __syncthreads();
+  for (int h = 128; h > 0; h >>= 1) {
+    if (threadIdx.x < h) s_most[threadIdx.x] = fmax(s_most[threadIdx.x], s_most[threadIdx.x + h]);
+    __syncthreads();
+  }
+  if (threadIdx.x == 0) atomicMax((unsigned long long *)mx, (unsigned long long)__double_as_longlong(s_most[0]));
 }
 
-// Eavg[o] (row-major) = mean over the eight sign choices s of S_s E'_{s a} S_s for orbit o (words
-// ax | ay << 2 | az << 4), E' row-major per offset; mx[0] = largest |E'|, mx[1] = largest distance
-// of an image from the mean.
-__global__ void average_kernel(const double *__restrict__ Ep, const int *__restrict__ kt, const int *__restrict__ orbits,
-                               Classes cl, double *__restrict__ Eavg, double *mx) {
-  const int w = orbits[blockIdx.y];
-  const int a[3] = {w & 3, (w >> 2) & 3, (w >> 4) & 3};
-  const int e = blockIdx.x * blockDim.x + threadIdx.x;  // i r + j
-  const int u = class_of(cl, e / R) ^ class_of(cl, e % R);
-  double v[8], sum = 0.0, big = 0.0, off = 0.0;
-  for (int s = 0; s < 8; ++s) {
-    const int x = s & 4 ? -a[0] : a[0], y = s & 2 ? -a[1] : a[1], z = s & 1 ? -a[2] : a[2];
-    const int k = kt[49 * (x + 3) + 7 * (y + 3) + z + 3];
-    const double t = Ep[(int64_t)k * R * R + e];
-    v[s] = __popc(s & u) & 1 ? -t : t;
-    sum += v[s];
-    big = fmax(big, fabs(t));
+// sq[i r + j] = the largest E_k(i, j)^2 of the 316 offsets (E_k(i, j) at i + j r).
+template <typename T>
+__global__ void __launch_bounds__(256) largest_kernel(const T *__restrict__ Ecol, double *__restrict__ sq) {
+  const int e = blockIdx.x * blockDim.x + threadIdx.x;
+  double most = 0.0;
+  for (int k = 0; k < BBFMM_NUM_OFFSETS; ++k) {
+    const double v = (double)Ecol[(int64_t)k * R * R + e];
+    most = fmax(most, v * v);
   }
-  sum *= 0.125;
-  for (int s = 0; s < 8; ++s) {
-    const double d = fabs(v[s] - sum);
-    if (!(d <= off)) off = d;  // NaN is kept
+  sq[(e % R) * R + e / R] = most;
+}
+
+// out = (Q o Q)^T in, or in (Q o Q): the squares that rotation from the left or the right adds up.
+__global__ void __launch_bounds__(256) rotate_squares_kernel(const double *__restrict__ Q, const double *__restrict__ in,
+                                                             int left, double *__restrict__ out) {
+  const int e = blockIdx.x * blockDim.x + threadIdx.x, i = e / R, j = e % R;
+  double sum = 0.0;
+  for (int k = 0; k < R; ++k) {
+    const double q = left ? Q[k * R + i] : Q[k * R + j];
+    sum += q * q * (left ? in[k * R + j] : in[i * R + k]);
   }
-  Eavg[(int64_t)blockIdx.y * R * R + e] = sum;
-  atomic_max_nonneg(mx, big);
-  atomic_max_nonneg(mx + 1, fabs(off));
+  out[e] = sum;
+}
+
+// *bad = 1 where a pair's images differ by more than rel of its rotated root-sum-square entry and base
+// of the largest of all, or are not finite.
+__global__ void __launch_bounds__(256) symmetric_kernel(const double *__restrict__ sq, const double *__restrict__ off,
+                                                        const double *__restrict__ mx, double rel, double base, int *bad) {
+  const int e = blockIdx.x * blockDim.x + threadIdx.x;
+  if (__syncthreads_or(!(off[e] <= rel * sqrt(sq[e]) + base * *mx)) && threadIdx.x == 0) *bad = 1;
 }
 
 // Bsteps[step][ks][f][lane] = E_a(i, j) for component j = 12 chunk + 4 ks + (lane & 3) of class
@@ -435,8 +476,12 @@ void sym_free(void *p) {
 // the given components (the largest singular values first): for class p the rows of U folded over
 // the eight mirror images of a node with the class's signs span the class's part of U, and the
 // columns of its Gram matrix, taken in order with a pivot of at least half the largest that
-// remains, are orthonormalised. False when the classes do not add up to r (the span of U is not
-// invariant) or a class is larger than the kernel's tiles.
+// remains, are orthonormalised. A component of a parity of its own is then a column with one entry,
+// and only components of equal singular values mix; the entries that the rounding of U leaves
+// elsewhere are cleared (below 32 roundings), because each would carry the largest operator entries
+// into the smallest: in FP32 it left 3e-9 of the largest entry in pairs of 1e-10 of it. False when the
+// classes do not add up to r (the span of U is not invariant) or a class is larger than the kernel's
+// tiles.
 template <typename T>
 static bool sym_basis(int n, int r, const T *U, std::vector<double> &Q, int *cstart) {
   const int n3 = n * n * n, h = n / 2, hh = h * h * h;
@@ -497,6 +542,28 @@ static bool sym_basis(int n, int r, const T *U, std::vector<double> &Q, int *cst
   }
   cstart[8] = (int)cols.size();
   if (cstart[8] != r) return false;
+  const double none = 16.0 * std::numeric_limits<T>::epsilon();
+  std::vector<int> at;
+  for (size_t j = 0; j < cols.size(); ++j) {  // cleared, then orthonormal again
+    std::vector<double> &c = cols[j];
+    for (int i = 0; i < r; ++i)
+      if (std::fabs(c[i]) < none) c[i] = 0.0;
+    for (int pass = 0; pass < 2; ++pass) {
+      at.clear();  // the entries left (one or three, but every one of a basis given in another mix)
+      for (int i = 0; i < r; ++i)
+        if (c[i] != 0.0) at.push_back(i);
+      for (size_t e = 0; e < j; ++e) {
+        double t = 0.0;
+        for (int i : at) t += cols[e][i] * c[i];
+        if (t != 0.0)
+          for (int i = 0; i < r; ++i) c[i] -= t * cols[e][i];
+      }
+    }
+    double nn = 0.0;
+    for (int i = 0; i < r; ++i) nn += c[i] * c[i];
+    nn = 1.0 / std::sqrt(nn);
+    for (int i = 0; i < r; ++i) c[i] *= nn;
+  }
   Q.resize((size_t)r * r);
   for (int j = 0; j < r; ++j)
     for (int i = 0; i < r; ++i) Q[(size_t)i * r + j] = cols[j][i];
@@ -506,10 +573,16 @@ static bool sym_basis(int n, int r, const T *U, std::vector<double> &Q, int *cst
 // The folded M2L's operators from U (host, column-major n^3 x r) and E (device, [316][r][r]
 // column-major), and the projections' U operators in the rotated basis: Bup (n^3 x r) and Bdn
 // (r x n^3) from the given ones (all on the device). *out stays null when the operators do not
-// have the mirror symmetry: an image further than `tol` of the largest entry from the mean of its
-// orbit, or a basis that does not split into parity classes.
+// have the mirror symmetry: a basis that does not split into parity classes, or a component pair with
+// an image further from the mean of its orbit than the rounding of its entries carries there: 8
+// roundings of the given operators' entries, each at the largest of its pair and rotated as errors add
+// up (root of the sum of squares), and 64 FP64 roundings of the largest entry of all for the arithmetic
+// that made them. Measured beyond the first term: 4 of those in FP32 and FP64, 30 in FP64 for a random
+// basis of the same span; entries changed by two roundings need 4 of the 8. The entries of the high
+// components are 1e-10 of the largest, so that a bound by the largest entry alone would let them differ
+// by any factor.
 template <typename T>
-int sym_prepare(int n, int r, const T *U, const T *Ecol, double tol, const T *Bup, const T *Bdn, T *Bup_sym, T *Bdn_sym,
+int sym_prepare(int n, int r, const T *U, const T *Ecol, const T *Bup, const T *Bdn, T *Bup_sym, T *Bdn_sym,
                 void **out, cudaStream_t s) {
   *out = nullptr;
   if (r != sy::R) return BBFMM_OK;
@@ -562,10 +635,10 @@ int sym_prepare(int n, int r, const T *U, const T *Ecol, double tol, const T *Bu
     orbits.push_back(w);
   }
   o->nsteps = (int)steps.size();
-  double *tmp = nullptr, *Ep = nullptr, *Eavg = nullptr, *mx = nullptr;
+  double *tmp = nullptr, *Ep = nullptr, *Eavg = nullptr, *chk = nullptr;  // chk: largest entry, flag, off, squares
   int *ktd = nullptr;
   auto cleanup = [&](int rc) {
-    for (void *p : {(void *)tmp, (void *)Ep, (void *)Eavg, (void *)mx, (void *)ktd})
+    for (void *p : {(void *)tmp, (void *)Ep, (void *)Eavg, (void *)chk, (void *)ktd})
       if (p) cudaFree(p);
     if (rc != BBFMM_OK || !*out) sym_free(o);
     return rc;
@@ -579,7 +652,7 @@ int sym_prepare(int n, int r, const T *U, const T *Ecol, double tol, const T *Bu
   SYM_OK(cudaMalloc(&tmp, BBFMM_NUM_OFFSETS * rr * 8));
   SYM_OK(cudaMalloc(&Ep, BBFMM_NUM_OFFSETS * rr * 8));
   SYM_OK(cudaMalloc(&Eavg, orbits.size() * rr * 8));
-  SYM_OK(cudaMalloc(&mx, 16));
+  SYM_OK(cudaMalloc(&chk, (2 + 3 * rr) * 8));
   SYM_OK(cudaMalloc(&ktd, kt.size() * 4));
   SYM_OK(cudaMalloc(&o->Q, rr * 8));
   SYM_OK(cudaMalloc(&o->orbits, orbits.size() * 4));
@@ -589,17 +662,25 @@ int sym_prepare(int n, int r, const T *U, const T *Ecol, double tol, const T *Bu
   SYM_OK(cudaMemcpyAsync(ktd, kt.data(), kt.size() * 4, cudaMemcpyHostToDevice, s));
   SYM_OK(cudaMemcpyAsync(o->orbits, orbits.data(), orbits.size() * 4, cudaMemcpyHostToDevice, s));
   SYM_OK(cudaMemcpyAsync(o->steps, steps.data(), steps.size() * sizeof(sy::Step), cudaMemcpyHostToDevice, s));
-  SYM_OK(cudaMemsetAsync(mx, 0, 16, s));
+  SYM_OK(cudaMemsetAsync(chk, 0, 16, s));
   const dim3 g316(r / 64, r / 64, BBFMM_NUM_OFFSETS);
   // E'_k = Q^T (E_k Q), row-major; E_k(i, j) at i + j r
   sy::gemm_kernel<T, double, double><<<g316, 256, 0, s>>>(r, Ecol, 1, r, (int64_t)rr, o->Q, r, 1, 0, tmp, r, 1, (int64_t)rr);
   sy::gemm_kernel<double, double, double><<<g316, 256, 0, s>>>(r, o->Q, 1, r, 0, tmp, r, 1, (int64_t)rr, Ep, r, 1,
                                                               (int64_t)rr);
-  sy::average_kernel<<<dim3((unsigned)(rr / 256), (unsigned)orbits.size()), 256, 0, s>>>(Ep, ktd, o->orbits, cl, Eavg, mx);
-  double h[2];
-  SYM_OK(cudaMemcpyAsync(h, mx, 16, cudaMemcpyDeviceToHost, s));
+  const unsigned grr = (unsigned)(rr / 256);
+  double *off = chk + 2, *sq = off + rr, *sq2 = sq + rr;
+  sy::average_kernel<<<grr, 256, 0, s>>>(Ep, ktd, o->orbits, (int)orbits.size(), cl, Eavg, off, chk);
+  sy::largest_kernel<T><<<grr, 256, 0, s>>>(Ecol, sq);
+  sy::rotate_squares_kernel<<<grr, 256, 0, s>>>(o->Q, sq, 1, sq2);
+  sy::rotate_squares_kernel<<<grr, 256, 0, s>>>(o->Q, sq2, 0, sq);
+  int bad = 0;
+  sy::symmetric_kernel<<<grr, 256, 0, s>>>(sq, off, chk, 4.0 * std::numeric_limits<T>::epsilon(), 64.0 * 0x1p-53,
+                                           (int *)(chk + 1));
+  SYM_OK(cudaGetLastError());
+  SYM_OK(cudaMemcpyAsync(&bad, chk + 1, 4, cudaMemcpyDeviceToHost, s));
   SYM_OK(cudaStreamSynchronize(s));
-  if (!(h[1] <= tol * h[0])) return cleanup(BBFMM_OK);  // not mirror-symmetric (or not finite)
+  if (bad) return cleanup(BBFMM_OK);
   sy::pack_steps_kernel<<<o->nsteps, 256, 0, s>>>(Eavg, o->steps, cl, o->Bsteps);
   sy::gemm_kernel<T, double, T><<<dim3(n3 / 64, r / 64, 1), 256, 0, s>>>(r, Bup, r, 1, 0, o->Q, r, 1, 0, Bup_sym, r, 1, 0);
   sy::gemm_kernel<double, T, T><<<dim3(r / 64, n3 / 64, 1), 256, 0, s>>>(r, o->Q, 1, r, 0, Bdn, n3, 1, 0, Bdn_sym, n3, 1,
@@ -683,8 +764,7 @@ int launch_m2l_sym(const void *op, const T *M, T *Lout, int level, T *part, int6
 }
 
 #define SYM_INST(T)                                                                                                   \
-  template int sym_prepare<T>(int, int, const T *, const T *, double, const T *, const T *, T *, T *, void **,        \
-                              cudaStream_t);                                                                          \
+  template int sym_prepare<T>(int, int, const T *, const T *, const T *, const T *, T *, T *, void **, cudaStream_t);    \
   template int sym_rotate<T>(const void *, bool, int64_t, const T *, T *, cudaStream_t);                              \
   template int launch_m2l_sym<T>(const void *, const T *, T *, int, T *, int64_t, cudaStream_t, int, int, const int4 *, int);
 SYM_INST(double)

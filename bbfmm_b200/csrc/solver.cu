@@ -186,8 +186,7 @@ int Solver<T>::set_operators(const T *U, const T *E) {
       TRY(dalloc(&Bup_sym, (size_t)n3 * r));
       TRY(dalloc(&Bdn_sym, (size_t)r * n3));
     }
-    // images of an operator agree to the rounding of its entries
-    TRY(sym_prepare<T>(n, r, U, Ecol, sizeof(T) == 8 ? 1e-13 : 4e-6, Bup, Bdn, Bup_sym, Bdn_sym, &symops, stream));
+    TRY(sym_prepare<T>(n, r, U, Ecol, Bup, Bdn, Bup_sym, Bdn_sym, &symops, stream));
   }
   if (mode == MODE_MIXED && r == 256) {  // r = 32 (n = 4): the M2L stays in FP64 on CUDA cores
     if (!tc_supported()) return bbfmm_set_error(BBFMM_ERR_UNSUPPORTED, "mixed mode needs an sm_100 GPU");

@@ -84,7 +84,7 @@ int dmma_default_groups(int level, int nsets);
 // M2L folded over mirrored offsets (m2l_sym.cu): n = 8 operators whose basis splits into parity
 // classes. U is on the host, the rest on the device; *out stays null without the symmetry.
 template <typename T>
-int sym_prepare(int n, int r, const T *U, const T *Ecol, double tol, const T *Bup, const T *Bdn, T *Bup_sym, T *Bdn_sym,
+int sym_prepare(int n, int r, const T *U, const T *Ecol, const T *Bup, const T *Bdn, T *Bup_sym, T *Bdn_sym,
                 void **out, cudaStream_t s);
 void sym_free(void *ops);
 template <typename T>

@@ -249,3 +249,59 @@ def test_the_form_of_other_operators():
     E = E.copy()
     E[5 * r * r:6 * r * r] *= 1.5
     assert _forms(8, "d", operators=(U, E)) == ["dense"] * 3
+
+
+def _output_by_components(U, E, mode):
+    """The M2L output of level 3 against the oracle's from the same multipoles and operators, per 64
+    components (their operators fall from 1 to 1e-10 of the largest entry): relative errors."""
+    import torch
+    from bbfmm_b200 import Solver
+    x, q = uniform_inputs(3000, seed=6)
+    s = Solver(8, 3, 1.0, mode=mode, operators=(U, E))
+    form = s.m2l_form(3)
+    s.set_particles(x)
+    s.solve(torch.as_tensor(q, dtype=s.dtype, device="cuda"))
+    cells = np.arange(0, 512, 5)
+    got = s.m2l_output(3)[cells].astype(float)
+    want = Oracle("d").m2l_sample(3, 256, np.asarray(E, float), s.multipoles(3).astype(float), cells).reshape(-1, 256)
+    s.close()
+    return form, [rel_l2(got[:, a:a + 64].ravel(), want[:, a:a + 64].ravel()) for a in range(0, 256, 64)]
+
+
+# components of FP32 output are rounded and summed as those of the solve (2e-5); in FP64 the folded
+# operators are off the given ones by at most 64 roundings (7e-15) of the largest entry, against
+# entries of 1e-3, 1e-6, 2e-8 and 1e-9 of it
+BY_COMPONENT = {"s": [2e-5] * 4, "d": [1e-11, 1e-8, 1e-6, 1e-5]}
+
+
+@pytest.mark.parametrize("mode", ["d", "s"])
+def test_high_components_keep_their_precision(mode):
+    U, E = _ops(8, single=mode == "s")
+    form, err = _output_by_components(U, E, mode)
+    assert form == "folded"
+    assert all(e < t for e, t in zip(err, BY_COMPONENT[mode])), err
+
+
+@pytest.mark.parametrize("mode,rows,factor", [("s", 64, 1.5), ("s", 128, 1.01), ("s", 192, 1.01), ("d", 128, 1.001),
+                                              ("d", 240, 1.001)])
+def test_operators_that_differ_beyond_their_rounding_are_not_folded(mode, rows, factor):
+    """The high components of one offset's operator changed: far below a rounding of the largest
+    entry, and the M2L still follows the operators given."""
+    U, E = _ops(8, single=mode == "s")
+    E = E.reshape(316, 256, 256).copy()
+    k = 202  # offset (1, 1, 2)
+    E[k, :, rows:] *= E.dtype.type(factor)
+    form, err = _output_by_components(U, E.reshape(-1), mode)
+    assert form == "dense"
+    assert max(err) < (2e-5 if mode == "s" else 1e-12), err
+
+
+@pytest.mark.parametrize("mode", ["d", "s"])
+def test_operators_that_differ_by_their_rounding_are_folded(mode):
+    """Every entry changed by up to two roundings of its own."""
+    U, E = _ops(8, single=mode == "s")
+    u = np.finfo(E.dtype).eps / 2
+    E2 = (E * (1 + 2 * u * np.random.default_rng(3).uniform(-1, 1, E.size))).astype(E.dtype)
+    form, err = _output_by_components(U, E2, mode)
+    assert form == "folded"
+    assert all(e < t for e, t in zip(err, BY_COMPONENT[mode])), err
