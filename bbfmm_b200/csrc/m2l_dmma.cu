@@ -328,16 +328,27 @@ __global__ void __launch_bounds__(256) m2l_lead_kernel(const double *__restrict_
   }
 }
 
-// Lout[e] = sum_g part[g][e], in a fixed order.
-__global__ void sum_parts_kernel(int64_t count, int ng, const double *__restrict__ part, double *__restrict__ Lout) {
+// Lout[e] = sum_g part[g][e], in a fixed order, in FP64 whatever T is.
+template <typename T>
+__global__ void sum_parts_kernel(int64_t count, int ng, const double *__restrict__ part, T *__restrict__ Lout) {
   for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < count; e += (int64_t)gridDim.x * blockDim.x) {
     double v = 0.0;
     for (int g = 0; g < ng; ++g) v += part[(int64_t)g * count + e];
-    Lout[e] = v;
+    Lout[e] = (T)v;
   }
 }
 
 }  // namespace dm
+
+// The partial sums of a whole level's offset (or step) groups added up: `count` values a group.
+template <typename T>
+int launch_sum_parts(int64_t count, int ng, const double *part, T *Lout, cudaStream_t s) {
+  const int64_t sg = (count + 255) / 256;
+  dm::sum_parts_kernel<T><<<(unsigned)(sg < 148 * 16 ? sg : 148 * 16), 256, 0, s>>>(count, ng, part, Lout);
+  return bbfmm_set_cuda_error(cudaGetLastError(), "M2L parts", __FILE__, __LINE__);
+}
+template int launch_sum_parts<double>(int64_t, int, const double *, double *, cudaStream_t);
+template int launch_sum_parts<float>(int64_t, int, const double *, float *, cudaStream_t);
 
 // Target tiles (CTAs) of the full FP64 M2L of one level.
 static int64_t dmma_tiles(int level, int nsets) {
@@ -415,8 +426,7 @@ int launch_m2l_dmma(int r, const double *M, const double *Ecol, double *Lout, in
                                                                    nsets);
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return bbfmm_set_cuda_error(e, "m2l_dmma", __FILE__, __LINE__);
-    dm::sum_parts_kernel<<<(int)((count + 255) / 256), 256, 0, s>>>(count, ng, part, Lout);
-    return bbfmm_set_cuda_error(cudaGetLastError(), "m2l_dmma parts", __FILE__, __LINE__);
+    return launch_sum_parts<double>(count, ng, part, Lout, s);
   }
   dm::m2l_dmma_kernel<<<boxes ? 8 * ((nboxes + 7) / 8) : grid, 256, dm::SMEM_BYTES, s>>>(M, Ecol, Lout, level, j0, j1,
                                                                                         ni, offs, boxes, nboxes, nsets);

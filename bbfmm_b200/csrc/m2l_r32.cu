@@ -47,11 +47,11 @@ __device__ __forceinline__ double get8(const Eight<float> &e, int k) {
 }
 
 // Grid: x = 8 classes x tiles of 16 blocks (class fastest: the resident CTAs share one source
-// region), y = groups of the 189 offsets, each with its own slice of Lout.
+// region), y = groups of the 189 offsets; several write their sums to slices of part, in FP64 whatever T is.
 template <typename T>
 __global__ void __launch_bounds__(THREADS, 2)
-    m2l_r32_kernel(const T *__restrict__ M, const double *__restrict__ Bpack, T *__restrict__ Lout, int level,
-                   const int4 *__restrict__ offs, const int4 *__restrict__ boxes, int nblocks, int nsets) {
+    m2l_r32_kernel(const T *__restrict__ M, const double *__restrict__ Bpack, T *__restrict__ Lout,
+                   double *__restrict__ part, int level, const int4 *__restrict__ offs, const int4 *__restrict__ boxes, int nblocks, int nsets) {
   __shared__ __align__(16) double Bs[STAGES][B_DOUBLES];
   const int P = 1 << (level - 1), P3 = P * P * P;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -84,7 +84,7 @@ __global__ void __launch_bounds__(THREADS, 2)
     sb[m] = o.x * 8 * P3;
   }
   const int o0 = (189 * blockIdx.y) / gridDim.y, o1 = (189 * (blockIdx.y + 1)) / gridDim.y;
-  Lout += (int64_t)blockIdx.y * 8 * nsets * P3 * R;
+  part += (int64_t)blockIdx.y * 8 * nsets * P3 * R;
 
   auto load_b = [&](int o) {
     if (o < o1) {
@@ -144,21 +144,17 @@ __global__ void __launch_bounds__(THREADS, 2)
 #pragma unroll
   for (int m = 0; m < 2; ++m) {
     if (!live[m]) continue;
-    T *dst = Lout + (int64_t)(sb[m] + c * P3 + (z0[m] * P + y0[m]) * P + x0[m]) * R + 2 * (lane & 3);
+    const int64_t at = (int64_t)(sb[m] + c * P3 + (z0[m] * P + y0[m]) * P + x0[m]) * R + 2 * (lane & 3);
 #pragma unroll
     for (int f = 0; f < 4; ++f) {
-      dst[8 * f] = (T)acc[m][f][0];
-      dst[8 * f + 1] = (T)acc[m][f][1];
+      if (gridDim.y > 1) {
+        part[at + 8 * f] = acc[m][f][0];
+        part[at + 8 * f + 1] = acc[m][f][1];
+      } else {
+        Lout[at + 8 * f] = (T)acc[m][f][0];
+        Lout[at + 8 * f + 1] = (T)acc[m][f][1];
+      }
     }
-  }
-}
-
-template <typename T>
-__global__ void sum_parts_kernel(int64_t count, int ng, const T *__restrict__ part, T *__restrict__ Lout) {
-  for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < count; e += (int64_t)gridDim.x * blockDim.x) {
-    T v = 0;
-    for (int g = 0; g < ng; ++g) v += part[(int64_t)g * count + e];
-    Lout[e] = v;
   }
 }
 
@@ -289,7 +285,7 @@ int r32_default_groups(int level, int nsets) {
 // Writes Lout for every cell of the level (assign), or with a list of 2 x 2 x 2 blocks of parent
 // cells (set, x0, y0, z0) for their cells only, in one group.
 template <typename T>
-int launch_m2l_r32(const double *Bpack, const T *M, T *Lout, int level, const int4 *offs, T *part, int64_t part_elems,
+int launch_m2l_r32(const double *Bpack, const T *M, T *Lout, int level, const int4 *offs, double *part, int64_t part_elems,
                    cudaStream_t s, int nsets, int ngroups, const int4 *boxes, int nboxes) {
   const int64_t all = r32_blocks(level, nsets), count = all * 64 * r32::R;
   if (boxes && (nboxes < 0 || nboxes > all)) return bbfmm_set_error(BBFMM_ERR_ARG, "box list longer than the level");
@@ -301,13 +297,11 @@ int launch_m2l_r32(const double *Bpack, const T *M, T *Lout, int level, const in
   if (ng < 1) ng = 1;
   const int64_t nb = boxes ? nboxes : all;
   const int64_t tiles = 8 * ((nb + r32::BLOCKS - 1) / r32::BLOCKS);
-  r32::m2l_r32_kernel<T><<<dim3((unsigned)tiles, ng), r32::THREADS, 0, s>>>(M, Bpack, ng > 1 ? part : Lout, level, offs,
-                                                                         boxes, (int)nb, nsets);
+  r32::m2l_r32_kernel<T><<<dim3((unsigned)tiles, ng), r32::THREADS, 0, s>>>(M, Bpack, Lout, part, level, offs, boxes,
+                                                                         (int)nb, nsets);
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess || ng == 1) return bbfmm_set_cuda_error(e, "m2l_r32", __FILE__, __LINE__);
-  const int64_t sg = (count + 255) / 256;
-  r32::sum_parts_kernel<T><<<(unsigned)(sg < 148 * 16 ? sg : 148 * 16), 256, 0, s>>>(count, ng, part, Lout);
-  return bbfmm_set_cuda_error(cudaGetLastError(), "m2l_r32 parts", __FILE__, __LINE__);
+  return launch_sum_parts<T>(count, ng, part, Lout, s);
 }
 
 #define R32_INST(T)                                                                                                  \
@@ -315,7 +309,7 @@ int launch_m2l_r32(const double *Bpack, const T *M, T *Lout, int level, const in
   template int r32_pack_proj<T>(const T *, const T *, double *, cudaStream_t);                                       \
   template int launch_proj_r32<T>(bool, int64_t, const T *, const double *, const T *, T, T *, int, int64_t,         \
                                   const int64_t *, cudaStream_t);                                                    \
-  template int launch_m2l_r32<T>(const double *, const T *, T *, int, const int4 *, T *, int64_t, cudaStream_t, int, int, \
+  template int launch_m2l_r32<T>(const double *, const T *, T *, int, const int4 *, double *, int64_t, cudaStream_t, int, int, \
                                  const int4 *, int);
 R32_INST(double)
 R32_INST(float)

@@ -73,7 +73,8 @@ __device__ __forceinline__ void dmma(double &d0, double &d1, double a, double b)
 template <typename T>
 __global__ void __launch_bounds__(THREADS, 1)
     m2l_sym_kernel(const T *__restrict__ M, const double *__restrict__ Bsteps, const Step *__restrict__ steps, int nsteps,
-                   const int *__restrict__ orbits, T *__restrict__ Lout, int level, const __grid_constant__ Classes cl,
+                   const int *__restrict__ orbits, T *__restrict__ Lout, double *__restrict__ part, int level,
+                   const __grid_constant__ Classes cl,
                    const int4 *__restrict__ boxes, int nboxes, int nsets) {
   extern __shared__ __align__(16) double smem[];
   double *const Bs = smem + 2 * A_DOUBLES;  // A tiles of two steps, then B tiles of two
@@ -126,7 +127,7 @@ __global__ void __launch_bounds__(THREADS, 1)
   __syncthreads();
   const int og = blockIdx.y, ng = gridDim.y;
   const int s0 = (int)((int64_t)nsteps * og / ng), s1 = (int)((int64_t)nsteps * (og + 1) / ng);
-  Lout += (int64_t)og * 8 * nsets * P3 * R;
+  part += (int64_t)og * 8 * nsets * P3 * R;  // used with several groups: FP64 whatever T is
 
   // the two elements of the A tiles this thread forms: component tid % 12 of targets tid / 12 and
   // 32 + tid / 12 (a warp's loads are runs of 12 consecutive components); target t is cell t & 7 of
@@ -283,27 +284,22 @@ __global__ void __launch_bounds__(THREADS, 1)
     for (int f = 0; f < FW; ++f) {
       const int c0 = cl.cstart[fc[f]], n = cl.cstart[fc[f] + 1] - c0;
       const int col = cl.fcol[warp * FW + f] + 2 * (lane & 3);
-      T *dst = Lout + cell * R + c0 + col;
-      if (col < n) dst[0] = (T)acc[m][f][0];
-      if (col + 1 < n) dst[1] = (T)acc[m][f][1];
+      const int64_t at = cell * R + c0 + col;
+      if (ng > 1) {
+        if (col < n) part[at] = acc[m][f][0];
+        if (col + 1 < n) part[at + 1] = acc[m][f][1];
+      } else {
+        if (col < n) Lout[at] = (T)acc[m][f][0];
+        if (col + 1 < n) Lout[at + 1] = (T)acc[m][f][1];
+      }
     }
   }
 }
 
-// Lout[e] = sum_g part[g][e], in a fixed order.
-template <typename T>
-__global__ void sym_sum_parts_kernel(int64_t count, int ng, const T *__restrict__ part, T *__restrict__ Lout) {
-  for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < count; e += (int64_t)gridDim.x * blockDim.x) {
-    T v = 0;
-    for (int g = 0; g < ng; ++g) v += part[(int64_t)g * count + e];
-    Lout[e] = v;
-  }
-}
-
-// The same for the 64 cells (8 classes x 2 x 2 x 2) of each listed block of parent cells.
+// Lout[e] = sum_g part[g][e], in a fixed order, for the 64 cells (8 classes x 2 x 2 x 2) of each listed block of parent cells.
 template <typename T>
 __global__ void __launch_bounds__(256) sym_sum_boxes_kernel(int64_t count, int ng, int P, const int4 *__restrict__ boxes,
-                                                            const T *__restrict__ part, T *__restrict__ Lout) {
+                                                            const double *__restrict__ part, T *__restrict__ Lout) {
   const int4 b = boxes[blockIdx.x];
   const int64_t P3 = (int64_t)P * P * P;
   for (int e = threadIdx.x; e < 64 * R; e += blockDim.x) {
@@ -311,9 +307,9 @@ __global__ void __launch_bounds__(256) sym_sum_boxes_kernel(int64_t count, int n
     const int64_t cell = (int64_t)(b.x * 8 + (t >> 3)) * P3 +
                          ((int64_t)(b.w + ((t >> 2) & 1)) * P + b.z + ((t >> 1) & 1)) * P + b.y + (t & 1);
     const int64_t at = cell * R + e % R;
-    T v = 0;
+    double v = 0.0;
     for (int g = 0; g < ng; ++g) v += part[(int64_t)g * count + at];
-    Lout[at] = v;
+    Lout[at] = (T)v;
   }
 }
 
@@ -730,7 +726,7 @@ int sym_default_groups(int level, int nsets) { return sym_groups(sym_tiles(level
 // blocks of parent cells (set, x0, y0, z0) for their cells only. ngroups: step groups of a whole
 // level (0: the default); a list takes as many as its tiles want and the scratch holds.
 template <typename T>
-int launch_m2l_sym(const void *op, const T *M, T *Lout, int level, T *part, int64_t part_elems, cudaStream_t s, int nsets,
+int launch_m2l_sym(const void *op, const T *M, T *Lout, int level, double *part, int64_t part_elems, cudaStream_t s, int nsets,
                    int ngroups, const int4 *boxes, int nboxes) {
   const SymOps *o = (const SymOps *)op;
   const int64_t P = (int64_t)1 << (level - 1);
@@ -751,22 +747,18 @@ int launch_m2l_sym(const void *op, const T *M, T *Lout, int level, T *part, int6
   else if (ng > 1 && (int64_t)ng * count > part_elems) ng = (int)(part_elems / count);
   if (ng < 1) ng = 1;
   sy::m2l_sym_kernel<T><<<dim3((unsigned)tiles, ng), sy::THREADS, sy::SMEM_BYTES, s>>>(
-      M, o->Bsteps, o->steps, o->nsteps, o->orbits, ng > 1 ? part : Lout, level, o->cl, boxes, nboxes, nsets);
+      M, o->Bsteps, o->steps, o->nsteps, o->orbits, Lout, part, level, o->cl, boxes, nboxes, nsets);
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess || ng == 1) return bbfmm_set_cuda_error(e, "m2l_sym", __FILE__, __LINE__);
-  if (boxes) {
-    sy::sym_sum_boxes_kernel<T><<<nboxes, 256, 0, s>>>(count, ng, (int)P, boxes, part, Lout);
-  } else {
-    const int64_t sg = (count + 255) / 256;
-    sy::sym_sum_parts_kernel<T><<<(unsigned)(sg < 148 * 16 ? sg : 148 * 16), 256, 0, s>>>(count, ng, part, Lout);
-  }
+  if (!boxes) return launch_sum_parts<T>(count, ng, part, Lout, s);
+  sy::sym_sum_boxes_kernel<T><<<nboxes, 256, 0, s>>>(count, ng, (int)P, boxes, part, Lout);
   return bbfmm_set_cuda_error(cudaGetLastError(), "m2l_sym parts", __FILE__, __LINE__);
 }
 
 #define SYM_INST(T)                                                                                                   \
   template int sym_prepare<T>(int, int, const T *, const T *, const T *, const T *, T *, T *, void **, cudaStream_t);    \
   template int sym_rotate<T>(const void *, bool, int64_t, const T *, T *, cudaStream_t);                              \
-  template int launch_m2l_sym<T>(const void *, const T *, T *, int, T *, int64_t, cudaStream_t, int, int, const int4 *, int);
+  template int launch_m2l_sym<T>(const void *, const T *, T *, int, double *, int64_t, cudaStream_t, int, int, const int4 *, int);
 SYM_INST(double)
 SYM_INST(float)
 

@@ -486,14 +486,14 @@ int Solver<T>::m2l_fp(const T *Ml, int level, int j0, int j1, int ni, bool folde
     return launch_m2l_sym<T>(symops, Ml, Lbuf, level, Lpart, Lpart_elems, stream, nsets, m2l_groups(level), boxes, nboxes);
   if (sizeof(T) == 8 && r == 256)
     return launch_m2l_dmma(r, (const double *)Ml, (const double *)Ecol, (double *)Lbuf, level, j0, j1, ni, offs,
-                           (double *)Lpart, Lpart_elems, stream, nsets, tune.m2l_groups[level], boxes, nboxes);
+                           Lpart, Lpart_elems, stream, nsets, tune.m2l_groups[level], boxes, nboxes);
   // FP32 at r = 256 writes all r outputs; in the rank mode (ni = rk()) the outputs i >= rank
   // of the zero-padded operators come out as zeros, so only other partial ranges are refused
   if (ni != r && ni != rk())
     return bbfmm_set_error(BBFMM_ERR_UNSUPPORTED, "partial output range needs the FP64 r = 256 path");
   if constexpr (sizeof(T) == 4)
-    return launch_m2l_simt(r, Ml, Ert, Lbuf, level, j0, j1, offs, stream, nsets, m2l_groups(level), Lpart, Lpart_elems,
-                           boxes, nboxes);
+    return launch_m2l_simt(r, Ml, Ert, Lbuf, level, j0, j1, offs, stream, nsets, m2l_groups(level), (float *)Lpart,
+                           Lpart_elems, boxes, nboxes);
   return bbfmm_set_error(BBFMM_ERR_UNSUPPORTED, "M2L rank must be 32 or 256 (n = 4 or 8)");
 }
 
@@ -603,7 +603,7 @@ int Solver<T>::m2l_post(int l) {
         if (masked) BBFMM_CUDA_OK(cudaMemsetAsync(Lbuf, 0, sizeof(T) * (size_t)cells(l) * r, stream));
         TRY(launch_m2l_tc(r, Msplit, Mcells(), Moff[l] / r, tcops, (double *)Lbuf, l, offs, stream, nsets,
                           tc_products, rk(), (const double *)Ml, (const double *)Ert, presplit ? Lsplit : nullptr,
-                          region_tcboxes[l], region_ntcboxes[l], region_tcgeom[l], (double *)Lpart, Lpart_elems,
+                          region_tcboxes[l], region_ntcboxes[l], region_tcgeom[l], Lpart, Lpart_elems,
                           tc_groups(l)));
         mark(ST_M2L, tc_groups(l) > 1 ? 2 : 1);
       } else if (lead > 0) {
@@ -613,7 +613,7 @@ int Solver<T>::m2l_post(int l) {
         mark(ST_M2L, 2);
       } else {
         TRY(launch_m2l_tc(r, Msplit, Mcells(), Moff[l] / r, tcops, (double *)Lbuf, l, offs, stream, nsets,
-                          tc_products, rk(), nullptr, nullptr, nullptr, nullptr, 0, 0x111, (double *)Lpart, Lpart_elems,
+                          tc_products, rk(), nullptr, nullptr, nullptr, nullptr, 0, 0x111, Lpart, Lpart_elems,
                           tc_groups(l)));
         mark(ST_M2L, tc_groups(l) > 1 ? 2 : 1);
       }
@@ -691,7 +691,7 @@ int Solver<T>::time_m2l(int level, int reps, float *ms) {
       else if (part == 0) rc = launch_m2l_tc(r, Msplit, Mcells(), Moff[level] / r, tcops, (double *)Lbuf, level, offs,
                                              stream, nsets, tc_products, rk(), fused ? (const double *)Ml : nullptr,
                                              fused ? (const double *)Ert : nullptr, presplit ? Lsplit : nullptr, nullptr,
-                                             0, 0x111, (double *)Lpart, Lpart_elems, tc_groups(level));
+                                             0, 0x111, Lpart, Lpart_elems, tc_groups(level));
       else rc = lead > 0 && !fused ? m2l_fp(Ml, level, 0, lead, lead_rows) : BBFMM_OK;
     }
     cudaEventRecord(b, stream);
@@ -1071,7 +1071,7 @@ int Solver<T>::autotune(const void *q_dev, int io_double) {
     if (sym_on()) cand.push_back({1, 0});
     // the DMMA and the SIMT M2L both split their offsets over groups
     for (int g : {1, 3, 7, 21})
-      if (dmma_part_elems(l, nsets, g, r) * (int64_t)sizeof(T) <= ((int64_t)1 << 30)) cand.push_back({1, g});
+      if (dmma_part_elems(l, nsets, g, r) * (int64_t)sizeof(double) <= ((int64_t)1 << 30)) cand.push_back({1, g});
     float best = 3.4e38f;
     std::pair<int, int> pick = cand[0];
     if (cand.size() > 1) {
@@ -1211,7 +1211,7 @@ int Solver<T>::copy_m2l_morton(int level, T *host_out) {
     if (lead > 0 && !fused) TRY(m2l_fp(Ml, level, 0, lead, lead_rows));
     TRY(launch_m2l_tc(r, Msplit, Mcells(), Moff[level] / r, tcops, (double *)Lbuf, level, offs, stream, nsets,
                       tc_products, rk(), fused ? (const double *)Ml : nullptr, fused ? (const double *)Ert : nullptr, nullptr,
-                      nullptr, 0, 0x111, (double *)Lpart, Lpart_elems, tc_groups(level)));
+                      nullptr, 0, 0x111, Lpart, Lpart_elems, tc_groups(level)));
   } else {
     TRY(m2l_fp(Ml, level, 0, rk(), rk(), msym[level]));
   }

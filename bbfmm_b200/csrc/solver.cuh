@@ -73,7 +73,7 @@ template <typename T> int r32_pack(const T *Ecol, double *Bpack, cudaStream_t s)
 int r32_default_groups(int level, int nsets);
 template <typename T> int r32_pack_proj(const T *Bup, const T *Bdn, double *frag, cudaStream_t s);
 template <typename T> int launch_proj_r32(bool up, int64_t rows, const T *A, const double *frag, const T *cs, T scale, T *C, int level, int64_t row0, const int64_t *rowlist, cudaStream_t s);
-template <typename T> int launch_m2l_r32(const double *Bpack, const T *M, T *Lout, int level, const int4 *offs, T *part, int64_t part_elems, cudaStream_t s, int nsets = 1, int ngroups = 0, const int4 *boxes = nullptr, int nboxes = 0);
+template <typename T> int launch_m2l_r32(const double *Bpack, const T *M, T *Lout, int level, const int4 *offs, double *part, int64_t part_elems, cudaStream_t s, int nsets = 1, int ngroups = 0, const int4 *boxes = nullptr, int nboxes = 0);
 int launch_m2l_simt(int r, const float *M, const float *Ert, float *Lout, int level, int j0, int j1, const int4 *offs, cudaStream_t s, int nsets = 1, int ngroups = 1, float *part = nullptr, int64_t part_elems = 0, const int4 *boxes = nullptr, int nboxes = 0);
 void build_offset_table(int *out);
 constexpr int DMMA_PARTS = 21;  // most offset groups of the FP64 M2L (189 = 9 x 21)
@@ -91,9 +91,10 @@ template <typename T>
 int sym_rotate(const void *ops, bool to_given, int64_t cells, const T *src, T *dst, cudaStream_t s);
 int sym_default_groups(int level, int nsets);
 template <typename T>
-int launch_m2l_sym(const void *ops, const T *M, T *Lout, int level, T *part, int64_t part_elems, cudaStream_t s,
+int launch_m2l_sym(const void *ops, const T *M, T *Lout, int level, double *part, int64_t part_elems, cudaStream_t s,
                    int nsets = 1, int ngroups = 0, const int4 *boxes = nullptr, int nboxes = 0);
 int64_t dmma_part_elems(int level, int nsets, int groups, int r);
+template <typename T> int launch_sum_parts(int64_t count, int ng, const double *part, T *Lout, cudaStream_t s);
 template <typename T>
 int launch_proj_dmma(int64_t M, int K, int N, const T *A, const T *B, const T *cs, T scale, T *C, int level, int mapmode,
                      cudaStream_t s, int64_t row0 = 0, int lda = 0, const int64_t *rows = nullptr);
@@ -304,7 +305,7 @@ struct Solver {
   T *Mall = nullptr;
   std::vector<int64_t> Moff;  // offset (elements) of level l in Mall, cpg layout
   T *Lbuf = nullptr;
-  T *Lpart = nullptr;  // partial sums of the offset-group FP64 M2L
+  double *Lpart = nullptr;  // partial sums of the M2L's offset (or step) groups (FP32 ones on CUDA cores)
   int64_t Lpart_elems = 0;
   void *Msplit = nullptr;
   T *phis = nullptr;

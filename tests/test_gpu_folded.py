@@ -305,3 +305,32 @@ def test_operators_that_differ_by_their_rounding_are_folded(mode):
     form, err = _output_by_components(U, E2, mode)
     assert form == "folded"
     assert all(e < t for e, t in zip(err, BY_COMPONENT[mode])), err
+
+
+@pytest.mark.parametrize("n", [4, 8])
+@pytest.mark.parametrize("level", [2, 3])
+def test_fp32_sums_do_not_depend_on_the_groups(n, level):
+    """The 189 offsets split over 1 to 21 CTAs: partial sums stay in FP64, so that the FP32 output is
+    one rounding of the same sum (a value may fall to the other side of a tie of FP32, about one in
+    1e7; one in 1e3 is allowed) and as close to the oracle as that rounding."""
+    import torch
+    from bbfmm_b200 import Solver
+    x, q = uniform_inputs(3000, seed=n + level)
+    U, E = _ops(n, single=True)
+    s = Solver(n, 3, 1.0, mode="s", operators=(U, E))
+    s.set_particles(x)
+    out = []
+    for g in (1, 2, 7, 21):
+        t = s.tuning()
+        t["m2l_groups"][level] = g
+        s.set_tuning(t)
+        if not out:
+            s.solve(torch.as_tensor(q, dtype=s.dtype, device="cuda"))
+        out.append(s.m2l_output(level))
+    for o in out[1:]:
+        assert np.mean(o != out[0]) < 1e-3
+    if n == 4:  # the multipoles read back are the ones contracted
+        r = n ** 3 // 2
+        want = Oracle("d").m2l_sample(level, r, E.astype(float), s.multipoles(level).astype(float), np.arange(8 ** level))
+        assert rel_l2(out[-1].astype(float).ravel(), np.asarray(want).ravel()) < 2.0 ** -24
+    s.close()
