@@ -722,9 +722,17 @@ static int sym_groups(int64_t tiles) {
 }
 int sym_default_groups(int level, int nsets) { return sym_groups(sym_tiles(level, nsets)); }
 
+// The same for a list of blocks of a level of `cells` cells, whose slices are the level's: at most
+// 65,536 cells of them (16 groups at level 4, 2 at level 5, 134 MB).
+int sym_list_groups(int nboxes, int64_t cells) {
+  const int64_t most = 65536 / cells;
+  const int g = sym_groups(8 * (int64_t)((nboxes + 7) / 8));
+  return g < most ? g : (most > 1 ? (int)most : 1);
+}
+
 // Writes Lout (assign, rotated basis) for every cell of the level, or with a box list of 2 x 2 x 2
-// blocks of parent cells (set, x0, y0, z0) for their cells only. ngroups: step groups of a whole
-// level (0: the default); a list takes as many as its tiles want and the scratch holds.
+// blocks of parent cells (set, x0, y0, z0) for their cells only, in `ngroups` step groups (fewer where
+// the scratch holds fewer).
 template <typename T>
 int launch_m2l_sym(const void *op, const T *M, T *Lout, int level, double *part, int64_t part_elems, cudaStream_t s, int nsets,
                    int ngroups, const int4 *boxes, int nboxes) {
@@ -741,8 +749,7 @@ int launch_m2l_sym(const void *op, const T *M, T *Lout, int level, double *part,
   }
   const int64_t count = 8 * (int64_t)nsets * P * P * P * sy::R;
   const int64_t tiles = boxes ? 8 * (int64_t)((nboxes + 7) / 8) : sym_tiles(level, nsets);
-  int ng = boxes || ngroups <= 0 ? sym_groups(tiles) : ngroups;
-  if (ng > DMMA_PARTS) ng = DMMA_PARTS;
+  int ng = ngroups < DMMA_PARTS ? ngroups : DMMA_PARTS;
   if (!part) ng = 1;
   else if (ng > 1 && (int64_t)ng * count > part_elems) ng = (int)(part_elems / count);
   if (ng < 1) ng = 1;

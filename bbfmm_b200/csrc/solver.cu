@@ -224,17 +224,12 @@ int Solver<T>::share_operators(const Solver<T> &o) {
   return BBFMM_OK;
 }
 
-// Partial-sum scratch of the offset-group FP64 M2L for the current tuning.
+// Partial-sum scratch of the M2L's offset groups for the current choices.
 template <typename T>
 int Solver<T>::alloc_partials() {
   int64_t need = 0;
-  {  // every full M2L (FP64 DMMA or SIMT) may split its offsets
-    for (int l = BBFMM_MINLEV; l <= maxlev; ++l) {
-      const int g = tc_m2l(l) ? tc_groups(l) : m2l_groups(l);
-      const int64_t e = dmma_part_elems(l, nsets, g, r);
-      if (e > need) need = e;
-    }
-  }
+  for (int l = BBFMM_MINLEV; l <= maxlev; ++l)
+    need = std::max(need, part_doubles(l, m2l_form(l), wanted_groups(l, m2l_form(l), listed(l))));
   if (need <= Lpart_elems && (need == 0 || Lpart)) return BBFMM_OK;
   if (Lpart) cudaFree(Lpart);
   Lpart = nullptr;
@@ -479,21 +474,22 @@ int Solver<T>::upward(const void *q_dev, int q_is_double) {
 // r = 256 operators there in FP64 and on CUDA cores in FP32.
 template <typename T>
 int Solver<T>::m2l_fp(const T *Ml, int level, int j0, int j1, int ni, bool folded, const int4 *boxes, int nboxes) {
+  const int ng = launch_groups(
+      level, r == 32 ? BBFMM_B200_M2L_R32 : (folded ? BBFMM_B200_M2L_FOLDED : BBFMM_B200_M2L_DENSE), boxes != nullptr);
   if (r == 32)
-    return launch_m2l_r32<T>(B32, Ml, Lbuf, level, offs, Lpart, Lpart_elems, stream, nsets, m2l_groups(level), boxes,
-                             nboxes);
+    return launch_m2l_r32<T>(B32, Ml, Lbuf, level, offs, Lpart, Lpart_elems, stream, nsets, ng, boxes, nboxes);
   if (folded)
-    return launch_m2l_sym<T>(symops, Ml, Lbuf, level, Lpart, Lpart_elems, stream, nsets, m2l_groups(level), boxes, nboxes);
+    return launch_m2l_sym<T>(symops, Ml, Lbuf, level, Lpart, Lpart_elems, stream, nsets, ng, boxes, nboxes);
   if (sizeof(T) == 8 && r == 256)
     return launch_m2l_dmma(r, (const double *)Ml, (const double *)Ecol, (double *)Lbuf, level, j0, j1, ni, offs,
-                           Lpart, Lpart_elems, stream, nsets, tune.m2l_groups[level], boxes, nboxes);
+                           Lpart, Lpart_elems, stream, nsets, ng, boxes, nboxes);
   // FP32 at r = 256 writes all r outputs; in the rank mode (ni = rk()) the outputs i >= rank
   // of the zero-padded operators come out as zeros, so only other partial ranges are refused
   if (ni != r && ni != rk())
     return bbfmm_set_error(BBFMM_ERR_UNSUPPORTED, "partial output range needs the FP64 r = 256 path");
   if constexpr (sizeof(T) == 4)
-    return launch_m2l_simt(r, Ml, Ert, Lbuf, level, j0, j1, offs, stream, nsets, m2l_groups(level), (float *)Lpart,
-                           Lpart_elems, boxes, nboxes);
+    return launch_m2l_simt(r, Ml, Ert, Lbuf, level, j0, j1, offs, stream, nsets, ng, (float *)Lpart, 2 * Lpart_elems, boxes,
+                           nboxes);
   return bbfmm_set_error(BBFMM_ERR_UNSUPPORTED, "M2L rank must be 32 or 256 (n = 4 or 8)");
 }
 
@@ -588,6 +584,7 @@ template <typename T>
 int Solver<T>::m2l_post(int l) {
   {
     const T *Ml = Mall + Moff[l];
+    const int ng = launch_groups(l, m2l_form(l), listed(l));  // several: one more launch adds the partial sums
     bool presplit = false;  // the M2L kernel wrote the split rows of the down projection
     const bool split = tc_m2l(l) && !msym[l];
     if (split) {
@@ -603,9 +600,8 @@ int Solver<T>::m2l_post(int l) {
         if (masked) BBFMM_CUDA_OK(cudaMemsetAsync(Lbuf, 0, sizeof(T) * (size_t)cells(l) * r, stream));
         TRY(launch_m2l_tc(r, Msplit, Mcells(), Moff[l] / r, tcops, (double *)Lbuf, l, offs, stream, nsets,
                           tc_products, rk(), (const double *)Ml, (const double *)Ert, presplit ? Lsplit : nullptr,
-                          region_tcboxes[l], region_ntcboxes[l], region_tcgeom[l], Lpart, Lpart_elems,
-                          tc_groups(l)));
-        mark(ST_M2L, tc_groups(l) > 1 ? 2 : 1);
+                          region_tcboxes[l], region_ntcboxes[l], region_tcgeom[l], Lpart, Lpart_elems, ng));
+        mark(ST_M2L, ng > 1 ? 2 : 1);
       } else if (lead > 0) {
         TRY(m2l_fp(Ml, l, 0, lead, lead_rows));
         TRY(launch_m2l_tc(r, Msplit, Mcells(), Moff[l] / r, tcops, (double *)Lbuf, l, offs, stream, nsets,
@@ -613,21 +609,17 @@ int Solver<T>::m2l_post(int l) {
         mark(ST_M2L, 2);
       } else {
         TRY(launch_m2l_tc(r, Msplit, Mcells(), Moff[l] / r, tcops, (double *)Lbuf, l, offs, stream, nsets,
-                          tc_products, rk(), nullptr, nullptr, nullptr, nullptr, 0, 0x111, Lpart, Lpart_elems,
-                          tc_groups(l)));
-        mark(ST_M2L, tc_groups(l) > 1 ? 2 : 1);
+                          tc_products, rk(), nullptr, nullptr, nullptr, nullptr, 0, 0x111, Lpart, Lpart_elems, ng));
+        mark(ST_M2L, ng > 1 ? 2 : 1);
       }
     } else if (region_boxes[l]) {
-      // a target region: only the blocks above active cells run (one offset group), the rest
-      // of the output is zero
+      // a target region: only the blocks above active cells run, the rest of the output is zero
       BBFMM_CUDA_OK(cudaMemsetAsync(Lbuf, 0, sizeof(T) * (size_t)cells(l) * r, stream));
       TRY(m2l_fp(Ml, l, 0, rk(), rk(), msym[l], region_boxes[l], region_nboxes[l]));
-      mark(ST_M2L, 1);
+      mark(ST_M2L, ng > 1 ? 2 : 1);
     } else {
       TRY(m2l_fp(Ml, l, 0, rk(), rk(), msym[l]));
-      int g = m2l_groups(l);
-      if ((int64_t)g * cells(l) * r > Lpart_elems) g = 1;
-      mark(ST_M2L, g > 1 ? 2 : 1);  // groups add the partial sum
+      mark(ST_M2L, ng > 1 ? 2 : 1);
     }
     if (!(l == maxlev && chunked())) {  // chunked leaf level: in leaf_down
       TRY(proj_down(l, local_solve ? n_tgt[l] : cells(l), 0, F[l & 1], presplit, local_solve ? tgt_list[l] : nullptr));
@@ -691,7 +683,8 @@ int Solver<T>::time_m2l(int level, int reps, float *ms) {
       else if (part == 0) rc = launch_m2l_tc(r, Msplit, Mcells(), Moff[level] / r, tcops, (double *)Lbuf, level, offs,
                                              stream, nsets, tc_products, rk(), fused ? (const double *)Ml : nullptr,
                                              fused ? (const double *)Ert : nullptr, presplit ? Lsplit : nullptr, nullptr,
-                                             0, 0x111, Lpart, Lpart_elems, tc_groups(level));
+                                             0, 0x111, Lpart, Lpart_elems,
+                                             launch_groups(level, BBFMM_B200_M2L_TENSOR, false));
       else rc = lead > 0 && !fused ? m2l_fp(Ml, level, 0, lead, lead_rows) : BBFMM_OK;
     }
     cudaEventRecord(b, stream);
@@ -1211,7 +1204,7 @@ int Solver<T>::copy_m2l_morton(int level, T *host_out) {
     if (lead > 0 && !fused) TRY(m2l_fp(Ml, level, 0, lead, lead_rows));
     TRY(launch_m2l_tc(r, Msplit, Mcells(), Moff[level] / r, tcops, (double *)Lbuf, level, offs, stream, nsets,
                       tc_products, rk(), fused ? (const double *)Ml : nullptr, fused ? (const double *)Ert : nullptr, nullptr,
-                      nullptr, 0, 0x111, Lpart, Lpart_elems, tc_groups(level)));
+                      nullptr, 0, 0x111, Lpart, Lpart_elems, launch_groups(level, BBFMM_B200_M2L_TENSOR, false)));
   } else {
     TRY(m2l_fp(Ml, level, 0, rk(), rk(), msym[level]));
   }
@@ -1430,6 +1423,17 @@ int bbfmm_b200_m2l_form(const bbfmm_b200_solver *h, int level, int *form) {
   if (level < BBFMM_MINLEV || level > maxlev) return bbfmm_set_error(BBFMM_ERR_ARG, "level out of range");
   *form = h->f ? h->f->m2l_form(level) : h->d->m2l_form(level);
   return BBFMM_OK;
+}
+
+int bbfmm_b200_m2l_groups(const bbfmm_b200_solver *h, int level, int *groups) {
+  if (!h || !groups) return bbfmm_set_error(BBFMM_ERR_ARG, "null argument");
+  auto get = [&](const auto &sv) -> int {
+    if (level < BBFMM_MINLEV || level > sv.maxlev) return bbfmm_set_error(BBFMM_ERR_ARG, "level out of range");
+    if (!sv.pos4) return bbfmm_set_error(BBFMM_ERR_STATE, "particles not set");
+    *groups = sv.launch_groups(level, sv.m2l_form(level), sv.listed(level));
+    return BBFMM_OK;
+  };
+  return h->f ? get(*h->f) : get(*h->d);
 }
 
 int bbfmm_b200_time_m2l(bbfmm_b200_solver *h, int level, int reps, float *ms) {

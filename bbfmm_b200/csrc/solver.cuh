@@ -90,6 +90,7 @@ void sym_free(void *ops);
 template <typename T>
 int sym_rotate(const void *ops, bool to_given, int64_t cells, const T *src, T *dst, cudaStream_t s);
 int sym_default_groups(int level, int nsets);
+int sym_list_groups(int nboxes, int64_t cells);
 template <typename T>
 int launch_m2l_sym(const void *ops, const T *M, T *Lout, int level, double *part, int64_t part_elems, cudaStream_t s,
                    int nsets = 1, int ngroups = 0, const int4 *boxes = nullptr, int nboxes = 0);
@@ -248,13 +249,30 @@ struct Solver {
   void *msplit_hi(int l) const { return (char *)Msplit + 2 * Moff[l]; }
   void *msplit_lo(int l) const { return (char *)Msplit + 2 * (Moff[l] + Mcells() * r); }
   bool split_later[11] = {};
-  int m2l_groups(int l) const {  // offset (or step) groups of the level's FP64 / FP32 M2L
-    // (of a target region's short block lists: up to 8, the scratch of small levels only)
-    if (region_boxes[l] && sym_on() && cells(l) <= 4096) return 8;
+  // Offset (or step) groups of a level's M2L, the CTAs that share a target tile's sum: what the
+  // choices want for a form, over the whole level or a target region's list of blocks (by the level
+  // and the list alone, so that a region's sums do not depend on what was solved before; only the
+  // folded M2L splits a list), the doubles of scratch that takes, and what the scratch in hand allows.
+  int wanted_groups(int l, int form, bool listed) const {
+    if (form == BBFMM_B200_M2L_TENSOR) return tc_groups(l);
+    if (listed) return form == BBFMM_B200_M2L_FOLDED ? sym_list_groups(region_nboxes[l], cells(l)) : 1;
     if (tune.m2l_groups[l] > 0) return tune.m2l_groups[l];
-    return r == 32 ? r32_default_groups(l, nsets)
-                   : (sym_on() ? sym_default_groups(l, nsets) : dmma_default_groups(l, nsets));
+    return form == BBFMM_B200_M2L_R32      ? r32_default_groups(l, nsets)
+           : form == BBFMM_B200_M2L_FOLDED ? sym_default_groups(l, nsets)
+                                           : dmma_default_groups(l, nsets);
   }
+  int64_t part_doubles(int l, int form, int groups) const {
+    const int64_t e = dmma_part_elems(l, nsets, groups, r);
+    return simt(form) ? e / 2 : e;
+  }
+  int launch_groups(int l, int form, bool listed) const {
+    const int g = wanted_groups(l, form, listed);
+    if (part_doubles(l, form, g) <= Lpart_elems) return g;
+    const int64_t fit = form == BBFMM_B200_M2L_TENSOR ? 1 : Lpart_elems * (simt(form) ? 2 : 1) / (cells(l) * r);
+    return fit > 1 ? (int)fit : 1;
+  }
+  bool simt(int form) const { return sizeof(T) == 4 && form == BBFMM_B200_M2L_DENSE; }  // FP32 partial sums
+  bool listed(int l) const { return region_boxes[l] != nullptr; }
   int4 *offs = nullptr;
   void *tcops = nullptr;  // mixed mode: split operators for the tensor-core kernel
   // mixed mode, n = 8: projections with the leading PROJ_LEAD components in FP64 and the rest

@@ -265,6 +265,12 @@ class Solver:
         _lib.check(_lib.lib().bbfmm_b200_m2l_form(self.h, int(level), C.byref(form)))
         return _lib.M2L_FORMS[form.value]
 
+    def m2l_groups(self, level: int) -> int:
+        """CTAs that share the sum of one target tile in the level's M2L of the next solve."""
+        g = C.c_int()
+        _lib.check(_lib.lib().bbfmm_b200_m2l_groups(self.h, int(level), C.byref(g)))
+        return g.value
+
     def time_m2l(self, level: int, reps: int = 3):
         ms = (C.c_float * 2)()
         _lib.check(_lib.lib().bbfmm_b200_time_m2l(self.h, level, reps, ms))

@@ -166,6 +166,9 @@ BBFMM_B200_API int bbfmm_b200_copy_m2l(bbfmm_b200_solver *s, int level, void *ho
 #define BBFMM_B200_M2L_R32 2    /* n = 4, FP64 tensor path */
 #define BBFMM_B200_M2L_TENSOR 3 /* MIXED: split BF16 on the tensor cores */
 BBFMM_B200_API int bbfmm_b200_m2l_form(const bbfmm_b200_solver *s, int level, int *form);
+/* groups[0] = the groups that the level's M2L of the next solve splits its 189 offsets (FOLDED: its
+ * steps) into, one CTA per target tile and group, whose partial sums another launch adds. */
+BBFMM_B200_API int bbfmm_b200_m2l_groups(const bbfmm_b200_solver *s, int level, int *groups);
 
 /* Re-run the M2L of one level `reps` times (inputs of the last solve), each launch as the
  * solve makes it, between CUDA events on the solver's stream: ms[0] = mean time of the main

@@ -148,6 +148,7 @@ def test_handle_setters_reject_null_handles_and_bad_values():
     assert L.bbfmm_b200_set_tc_products(None, 0) == 1
     assert L.bbfmm_b200_set_leaf_slab(None, 64) == 1
     assert L.bbfmm_b200_m2l_form(None, 2, None) == 1
+    assert L.bbfmm_b200_m2l_groups(None, 2, None) == 1
     assert L.bbfmm_b200_solve(None, None, None) == 1
     assert L.bbfmm_b200_set_particles(None, 10, None) == 1
     assert L.bbfmm_b200_set_particles_device(None, 10, None) == 1

@@ -334,3 +334,35 @@ def test_fp32_sums_do_not_depend_on_the_groups(n, level):
         want = Oracle("d").m2l_sample(level, r, E.astype(float), s.multipoles(level).astype(float), np.arange(8 ** level))
         assert rel_l2(out[-1].astype(float).ravel(), np.asarray(want).ravel()) < 2.0 ** -24
     s.close()
+
+
+def test_a_regions_sums_do_not_depend_on_earlier_tunings():
+    """The folded M2L of a target region's block list: its step groups follow from the level and the
+    list, whatever scratch an earlier tuning of the same solver left, and the results are the same
+    bits; particles in the region agree with the unrestricted solve."""
+    import torch
+    from bbfmm_b200 import Solver
+    from bbfmm_b200.fmm import leaf_of_particles
+    x, q = uniform_inputs(20000, seed=8)
+    qd = torch.as_tensor(q, device="cuda")
+    active = np.zeros(64, bool)
+    active[[5, 40]] = True
+    inside = active[leaf_of_particles(x, 1.0, 2)[0]]
+    got, groups = [], []
+    for more in (False, True):
+        s = Solver(8, 4, 1.0, mode="d")
+        s.set_particles(x)
+        if more:
+            whole = s.solve(qd).cpu().numpy()
+            for g in (21, 0):
+                t = s.tuning()
+                t["m2l_groups"] = [g] * 11
+                s.set_tuning(t)
+        s.set_target_region(2, active)
+        got.append(s.solve(qd).cpu().numpy()[inside])
+        groups.append([s.m2l_groups(l) for l in (2, 3, 4)])
+        s.close()
+    assert groups[0] == groups[1]
+    assert groups[0][2] == 16  # a list of two blocks at level 4: 18 would fill the GPU, 16 slices is the bound
+    assert np.array_equal(got[0], got[1])
+    assert rel_l2(got[0], whole[inside]) < 1e-12
