@@ -1486,6 +1486,12 @@ int bbfmm_b200_set_kernel(bbfmm_b200_solver *h, int kernel) {
   return BBFMM_OK;
 }
 
+// The rank and the products choose forms and groups: scratch for them, where particles are set.
+static int choices_changed(bbfmm_b200_solver *h) {
+  if (h->f) return h->f->pos4 ? h->f->alloc_partials() : BBFMM_OK;
+  return h->d->pos4 ? h->d->alloc_partials() : BBFMM_OK;
+}
+
 int bbfmm_b200_set_rank(bbfmm_b200_solver *h, int rank) {
   if (!h) return bbfmm_set_error(BBFMM_ERR_ARG, "null handle");
   const int r = h->f ? h->f->r : h->d->r;
@@ -1493,7 +1499,7 @@ int bbfmm_b200_set_rank(bbfmm_b200_solver *h, int rank) {
     return bbfmm_set_error(BBFMM_ERR_ARG, "rank must be 0 or a multiple of 32 in [32, r]");
   if (h->f) h->f->rank_eff = rank;
   else h->d->rank_eff = rank;
-  return BBFMM_OK;
+  return choices_changed(h);
 }
 
 int bbfmm_b200_set_tc_products(bbfmm_b200_solver *h, int nprod) {
@@ -1501,7 +1507,7 @@ int bbfmm_b200_set_tc_products(bbfmm_b200_solver *h, int nprod) {
     return bbfmm_set_error(BBFMM_ERR_ARG, "products must be 0 (adaptive), 1 or 3");
   if (h->f) return bbfmm_set_error(BBFMM_ERR_UNSUPPORTED, "tensor-core products apply to the mixed mode");
   h->d->tc_products = nprod;
-  return BBFMM_OK;
+  return choices_changed(h);
 }
 
 int bbfmm_b200_autotune(bbfmm_b200_solver *h, const void *q_dev) {

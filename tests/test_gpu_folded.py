@@ -366,3 +366,27 @@ def test_a_regions_sums_do_not_depend_on_earlier_tunings():
     assert groups[0][2] == 16  # a list of two blocks at level 4: 18 would fill the GPU, 16 slices is the bound
     assert np.array_equal(got[0], got[1])
     assert rel_l2(got[0], whole[inside]) < 1e-12
+
+
+@pytest.mark.parametrize("mode,change", [("d", "rank"), ("mixed", "products")])
+def test_choices_after_the_particles_get_their_scratch(mode, change):
+    """The rank or the products set after the particles: the groups that they take before them."""
+    from bbfmm_b200 import Solver, _lib
+    x, _ = uniform_inputs(3000, seed=1)
+    lev = 3 if change == "rank" else 4  # depths at which the first choice's scratch is the smaller
+    groups = []
+    for late in (False, True):
+        s = Solver(8, lev, 1.0, mode=mode)
+        if change == "products":
+            s.set_tc_products(3)
+        if late:
+            s.set_particles(x)
+        if change == "rank":
+            _lib.check(_lib.lib().bbfmm_b200_set_rank(s.h, 160))
+        else:
+            s.set_tc_products(0)
+        if not late:
+            s.set_particles(x)
+        groups.append([s.m2l_groups(l) for l in range(2, lev + 1)])
+        s.close()
+    assert groups[0] == groups[1] and max(groups[0]) > 1
