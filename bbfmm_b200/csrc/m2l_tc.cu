@@ -1448,7 +1448,7 @@ int launch_m2l_tc(int r, const void *Msplit, int64_t ncell_total, int64_t cell_o
       return bbfmm_set_error(BBFMM_ERR_ARG, "box list longer than the level");
     if (boxes && nboxes == 0) return BBFMM_OK;
     const int64_t per_class = boxes ? (int64_t)((nboxes + spl - 1) / spl) : tc2_tiles(level, nsets) / 8;
-    const int64_t tiles2 = 16 * ((per_class + 1) / 2);  // pairs of a class's tiles
+    const int64_t tiles2 = tc2_ctas(per_class);
     // offset groups need the leading block inside the kernel (or none), so that every slice is a sum
     const int64_t ncell = 8 * (int64_t)nsets * P * P * P, count = ncell * r;
     const int ng = part && ngroups > 1 && (fuse || ilead == 0) && ngroups * count <= part_elems ? ngroups : 1;

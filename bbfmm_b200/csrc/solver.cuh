@@ -178,6 +178,15 @@ inline int64_t tc2_tiles(int level, int nsets) {
   const int P = 1 << (level - 1), spt = 1 << (8 - g.lb());
   return 8 * (int64_t)((nsets + spt - 1) / spt) * (P >> g.lx) * (P >> g.ly) * (P >> g.lz);
 }
+// CTAs of a launch over `per_class` tiles of each class: pairs of tiles, an odd count rounded up.
+inline int64_t tc2_ctas(int64_t per_class) { return 16 * ((per_class + 1) / 2); }
+// Offset groups of a whole level: as many as leave every CTA an SM of its own, nine at most. By the
+// CTAs and not by the tiles: 12 sets at level 3 (three tiles a class, 32 CTAs) 0.574 ms in six groups,
+// two waves, 0.481 ms in four; 96 sets at level 2 0.571 -> 0.423 ms.
+inline int tc2_groups(int level, int nsets) {
+  const int64_t g = 148 / tc2_ctas(tc2_tiles(level, nsets) / 8);
+  return g < 1 ? 1 : (g > 9 ? 9 : (int)g);
+}
 
 // Degree of homogeneity of a BBFMM_B200_KERNEL_* value (bbfmm.c:109-144), 0 for an unknown one.
 inline int kernel_homogen(int kernel) {
@@ -397,8 +406,7 @@ struct Solver {
   // leading block is another kernel's.
   int tc_groups(int l) const {
     if (!tc_two_box(tc_products, rk()) || (lead > 0 && !tc_fuses_lead(tcops, tc_products, rk()))) return 1;
-    const int64_t g = 148 / tc2_tiles(l, nsets);
-    return g < 1 ? 1 : (g > 9 ? 9 : (int)g);
+    return tc2_groups(l, nsets);
   }
   // S rows -> Mall (cpg); F rows <- Lbuf (Morton, assign). Row t is cell row0 + t, or
   // rowlist[t] when a row list is given.
