@@ -919,15 +919,18 @@ int Solver<T>::build_region_tiles() {
 // synchronisation: the item count sizes the launch).
 template <typename T>
 int Solver<T>::build_near_work() {
-  if (!near_work) TRY(dalloc((unsigned char **)&near_work, near_work_bytes(N, maxlev, nsets) + near_order_bytes(N)));
+  if (!near_work) TRY(dalloc((unsigned char **)&near_work, near_work_bytes(N, maxlev, nsets)));
   int flag = 0;
   TRY(near_work_build(N, leaf_start, maxlev, nsets, tune.p2p_threads, near_work, stream, &near_items, &flag,
                       region_mask, region_level));
   if (flag) return bbfmm_set_error(BBFMM_ERR_ARG, "leaf offsets must rise from 0 to N without decreasing");
   near_threads = tune.p2p_threads;
-  // longest items first, through scratch behind the list
-  return near_order(N, leaf_start, maxlev, nsets, near_threads, near_work, near_items,
-                    (char *)near_work + near_work_bytes(N, maxlev, nsets), stream);
+  if (near_items < 2) return BBFMM_OK;
+  unsigned char *scratch = nullptr;  // longest items first
+  TRY(dalloc(&scratch, near_order_bytes(near_items)));
+  const int rc = near_order(N, leaf_start, maxlev, nsets, near_threads, near_work, near_items, scratch, stream);
+  cudaFree(scratch);  // waits for the launches
+  return rc;
 }
 
 // pot[i] = sum_j q_j / r_ij and fld[i] = grad pot at x_i (FMM), caller's order, no target

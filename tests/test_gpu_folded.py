@@ -390,3 +390,22 @@ def test_choices_after_the_particles_get_their_scratch(mode, change):
         groups.append([s.m2l_groups(l) for l in range(2, lev + 1)])
         s.close()
     assert groups[0] == groups[1] and max(groups[0]) > 1
+
+
+def test_the_near_list_keeps_no_scratch():
+    """Device memory that a particle more costs at one depth: its FP32 position, charge and potential,
+    an index and 8 bytes of the list (32 bytes), and no scratch of the list's order (8 more)."""
+    import torch
+    from bbfmm_b200 import Solver
+    used = []
+    rng = np.random.default_rng(0)
+    for N in (1_000_000, 9_000_000):
+        s = Solver(4, 4, 1.0, mode="s")
+        x = torch.as_tensor(rng.random((N, 3)) - 0.5, dtype=torch.float32, device="cuda")
+        torch.cuda.synchronize()
+        free = torch.cuda.mem_get_info()[0]
+        s.set_particles(x)
+        used.append(free - torch.cuda.mem_get_info()[0])
+        s.close()
+        del x
+    assert 30 < (used[1] - used[0]) / 8e6 < 34
