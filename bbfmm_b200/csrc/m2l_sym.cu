@@ -316,14 +316,16 @@ __global__ void __launch_bounds__(256) sym_sum_boxes_kernel(int64_t count, int n
 // ---------------------------------------------------------------- set-up
 // C(m, n) = sum_k A(m, k) B(k, n) for a batch (blockIdx.z), element (i, j) of a matrix at
 // i * rs + j * cs; sums in FP64. 64 x 64 tiles, 4 x 4 values per thread; dimensions multiples of 64.
+// alist (optional): matrix alist[z] of A for product z.
 template <typename TA, typename TB, typename TC>
 __global__ void __launch_bounds__(256) gemm_kernel(int K, const TA *__restrict__ A, int64_t ars, int64_t acs, int64_t ab,
                                                    const TB *__restrict__ B, int64_t brs, int64_t bcs, int64_t bb,
-                                                   TC *__restrict__ C, int64_t crs, int64_t ccs, int64_t cb) {
+                                                   TC *__restrict__ C, int64_t crs, int64_t ccs, int64_t cb,
+                                                   const int *__restrict__ alist = nullptr) {
   __shared__ double sa[16][65], sb[16][65];
   const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
   const int m0 = blockIdx.x * 64, n0 = blockIdx.y * 64;
-  A += blockIdx.z * ab;
+  A += (alist ? alist[blockIdx.z] : (int)blockIdx.z) * ab;
   B += blockIdx.z * bb;
   C += blockIdx.z * cb;
   double acc[4][4] = {};
@@ -361,22 +363,22 @@ __device__ __forceinline__ int class_of(const Classes &cl, int i) {
 }
 
 // One thread per component pair e = i r + j. Eavg[o] (row-major) = mean over the eight sign choices s
-// of S_s E'_{s a} S_s for each orbit o (words ax | ay << 2 | az << 4), E' row-major per offset;
-// off[e] = the pair's largest distance of an image from the mean (NaN is kept), mx the largest |E'|,
-// over all orbits.
-__global__ void __launch_bounds__(256) average_kernel(const double *__restrict__ Ep, const int *__restrict__ kt,
+// of S_s E'_{s a} S_s for each orbit o (words ax | ay << 2 | az << 4), E' row-major, the matrix of an
+// offset at slot[its cell of the 7 x 7 x 7 grid]; off[e] = the pair's largest distance of an image from
+// the mean (NaN is kept), mx the largest |E'|, over the orbits of every launch.
+__global__ void __launch_bounds__(256) average_kernel(const double *__restrict__ Ep, const int *__restrict__ slot,
                                                       const int *__restrict__ orbits, int norb, Classes cl,
                                                       double *__restrict__ Eavg, double *__restrict__ off, double *mx) {
   const int e = blockIdx.x * blockDim.x + threadIdx.x;
   const int u = class_of(cl, e / R) ^ class_of(cl, e % R);
-  double most = 0.0, far = 0.0;
+  double most = 0.0, far = off[e];
   for (int o = 0; o < norb; ++o) {
     const int w = orbits[o], a[3] = {w & 3, (w >> 2) & 3, (w >> 4) & 3};
     double v[8], sum = 0.0;
 #pragma unroll
     for (int s = 0; s < 8; ++s) {
       const int x = s & 4 ? -a[0] : a[0], y = s & 2 ? -a[1] : a[1], z = s & 1 ? -a[2] : a[2];
-      const double t = Ep[(int64_t)kt[49 * (x + 3) + 7 * (y + 3) + z + 3] * R * R + e];
+      const double t = Ep[(int64_t)slot[49 * (x + 3) + 7 * (y + 3) + z + 3] * R * R + e];
       v[s] = __popc(s & u) & 1 ? -t : t;
       sum += v[s];
       most = fmax(most, fabs(t));
@@ -468,6 +470,20 @@ void sym_free(void *p) {
   delete o;
 }
 
+// q minus its parts along the orthonormal cols[from .. to).
+static void take_out(std::vector<double> &q, const std::vector<std::vector<double>> &cols, size_t from, size_t to) {
+  const int r = (int)q.size();
+  for (size_t e = from; e < to; ++e) {
+    const std::vector<double> &c = cols[e];
+    double t4[4] = {};
+    for (int i = 0; i < r; i += 4)
+      for (int k4 = 0; k4 < 4; ++k4) t4[k4] += c[i + k4] * q[i + k4];
+    const double t = (t4[0] + t4[1]) + (t4[2] + t4[3]);
+    if (t != 0.0)
+      for (int i = 0; i < r; ++i) q[i] -= t * c[i];
+  }
+}
+
 // Orthogonal Q (r x r) whose columns have a parity in each axis, class by class in the order of
 // the given components (the largest singular values first): for class p the rows of U folded over
 // the eight mirror images of a node with the class's signs span the class's part of U, and the
@@ -518,15 +534,8 @@ static bool sym_basis(int n, int r, const T *U, std::vector<double> &Q, int *cst
       }
       // against the class's earlier columns, then against every earlier one (the classes are
       // orthogonal to about 1e-13 as they are; after that to rounding)
-      for (int pass = 0; pass < 2; ++pass)
-        for (size_t e = pass == 0 ? cstart[p] : 0; e < cols.size(); ++e) {
-          const std::vector<double> &c = cols[e];
-          double t4[4] = {};
-          for (int i = 0; i < r; i += 4)
-            for (int k4 = 0; k4 < 4; ++k4) t4[k4] += c[i + k4] * q[i + k4];
-          const double t = (t4[0] + t4[1]) + (t4[2] + t4[3]);
-          for (int i = 0; i < r; ++i) q[i] -= t * c[i];
-        }
+      take_out(q, cols, cstart[p], cols.size());
+      take_out(q, cols, 0, cols.size());
       double nn = 0.0;
       for (int i = 0; i < r; ++i) nn += q[i] * q[i];
       nn = 1.0 / std::sqrt(nn);
@@ -539,22 +548,12 @@ static bool sym_basis(int n, int r, const T *U, std::vector<double> &Q, int *cst
   cstart[8] = (int)cols.size();
   if (cstart[8] != r) return false;
   const double none = 16.0 * std::numeric_limits<T>::epsilon();
-  std::vector<int> at;
   for (size_t j = 0; j < cols.size(); ++j) {  // cleared, then orthonormal again
     std::vector<double> &c = cols[j];
     for (int i = 0; i < r; ++i)
       if (std::fabs(c[i]) < none) c[i] = 0.0;
-    for (int pass = 0; pass < 2; ++pass) {
-      at.clear();  // the entries left (one or three, but every one of a basis given in another mix)
-      for (int i = 0; i < r; ++i)
-        if (c[i] != 0.0) at.push_back(i);
-      for (size_t e = 0; e < j; ++e) {
-        double t = 0.0;
-        for (int i : at) t += cols[e][i] * c[i];
-        if (t != 0.0)
-          for (int i = 0; i < r; ++i) c[i] -= t * cols[e][i];
-      }
-    }
+    take_out(c, cols, 0, j);
+    take_out(c, cols, 0, j);
     double nn = 0.0;
     for (int i = 0; i < r; ++i) nn += c[i] * c[i];
     nn = 1.0 / std::sqrt(nn);
@@ -612,6 +611,10 @@ int sym_prepare(int n, int r, const T *U, const T *Ecol, const T *Bup, const T *
     const int x = c / 49 - 3, y = (c / 7) % 7 - 3, z = c % 7 - 3;
     if (x < -1 || x > 1 || y < -1 || y > 1 || z < -1 || z > 1) kt[c] = k++;
   }
+  // the operators are rotated and averaged a few orbits at a time (chunks of at most 32 offsets): slot
+  // of each offset in its chunk, the offsets chunk by chunk, and where chunks begin among both
+  constexpr int CHUNK = 32;
+  std::vector<int> slot(343, 0), list, ofirst{0}, kfirst{0};
   for (int w = 0; w < 64; ++w) {
     const int a[3] = {w & 3, (w >> 2) & 3, (w >> 4) & 3};
     if (a[0] <= 1 && a[1] <= 1 && a[2] <= 1) continue;
@@ -628,13 +631,26 @@ int sym_prepare(int n, int r, const T *U, const T *Ecol, const T *Bup, const T *
           }
           steps.push_back(st);
         }
+    if ((int)list.size() - kfirst.back() + (1 << __builtin_popcount(nz)) > CHUNK) {
+      ofirst.push_back((int)orbits.size());
+      kfirst.push_back((int)list.size());
+    }
+    for (int s = 0; s < 8; ++s)
+      if ((s & ~nz) == 0) {
+        const int x = s & 4 ? -a[0] : a[0], y = s & 2 ? -a[1] : a[1], z = s & 1 ? -a[2] : a[2];
+        const int c = 49 * (x + 3) + 7 * (y + 3) + z + 3;
+        slot[c] = (int)list.size() - kfirst.back();
+        list.push_back(kt[c]);
+      }
     orbits.push_back(w);
   }
+  ofirst.push_back((int)orbits.size());
+  kfirst.push_back((int)list.size());
   o->nsteps = (int)steps.size();
   double *tmp = nullptr, *Ep = nullptr, *Eavg = nullptr, *chk = nullptr;  // chk: largest entry, flag, off, squares
-  int *ktd = nullptr;
+  int *listd = nullptr;  // the offsets, then the slots
   auto cleanup = [&](int rc) {
-    for (void *p : {(void *)tmp, (void *)Ep, (void *)Eavg, (void *)chk, (void *)ktd})
+    for (void *p : {(void *)tmp, (void *)Ep, (void *)Eavg, (void *)chk, (void *)listd})
       if (p) cudaFree(p);
     if (rc != BBFMM_OK || !*out) sym_free(o);
     return rc;
@@ -645,28 +661,33 @@ int sym_prepare(int n, int r, const T *U, const T *Ecol, const T *Bup, const T *
     cudaError_t e__ = (x);                                                                              \
     if (e__ != cudaSuccess) return cleanup(bbfmm_set_cuda_error(e__, #x, __FILE__, __LINE__));          \
   } while (0)
-  SYM_OK(cudaMalloc(&tmp, BBFMM_NUM_OFFSETS * rr * 8));
-  SYM_OK(cudaMalloc(&Ep, BBFMM_NUM_OFFSETS * rr * 8));
+  SYM_OK(cudaMalloc(&tmp, CHUNK * rr * 8));
+  SYM_OK(cudaMalloc(&Ep, CHUNK * rr * 8));
   SYM_OK(cudaMalloc(&Eavg, orbits.size() * rr * 8));
   SYM_OK(cudaMalloc(&chk, (2 + 3 * rr) * 8));
-  SYM_OK(cudaMalloc(&ktd, kt.size() * 4));
+  list.insert(list.end(), slot.begin(), slot.end());
+  SYM_OK(cudaMalloc(&listd, list.size() * 4));
   SYM_OK(cudaMalloc(&o->Q, rr * 8));
   SYM_OK(cudaMalloc(&o->orbits, orbits.size() * 4));
   SYM_OK(cudaMalloc(&o->steps, steps.size() * sizeof(sy::Step)));
   SYM_OK(cudaMalloc(&o->Bsteps, steps.size() * sy::B_DOUBLES * 8));
   SYM_OK(cudaMemcpyAsync(o->Q, Q.data(), rr * 8, cudaMemcpyHostToDevice, s));
-  SYM_OK(cudaMemcpyAsync(ktd, kt.data(), kt.size() * 4, cudaMemcpyHostToDevice, s));
+  SYM_OK(cudaMemcpyAsync(listd, list.data(), list.size() * 4, cudaMemcpyHostToDevice, s));
   SYM_OK(cudaMemcpyAsync(o->orbits, orbits.data(), orbits.size() * 4, cudaMemcpyHostToDevice, s));
   SYM_OK(cudaMemcpyAsync(o->steps, steps.data(), steps.size() * sizeof(sy::Step), cudaMemcpyHostToDevice, s));
-  SYM_OK(cudaMemsetAsync(chk, 0, 16, s));
-  const dim3 g316(r / 64, r / 64, BBFMM_NUM_OFFSETS);
-  // E'_k = Q^T (E_k Q), row-major; E_k(i, j) at i + j r
-  sy::gemm_kernel<T, double, double><<<g316, 256, 0, s>>>(r, Ecol, 1, r, (int64_t)rr, o->Q, r, 1, 0, tmp, r, 1, (int64_t)rr);
-  sy::gemm_kernel<double, double, double><<<g316, 256, 0, s>>>(r, o->Q, 1, r, 0, tmp, r, 1, (int64_t)rr, Ep, r, 1,
-                                                              (int64_t)rr);
+  SYM_OK(cudaMemsetAsync(chk, 0, (2 + rr) * 8, s));
   const unsigned grr = (unsigned)(rr / 256);
   double *off = chk + 2, *sq = off + rr, *sq2 = sq + rr;
-  sy::average_kernel<<<grr, 256, 0, s>>>(Ep, ktd, o->orbits, (int)orbits.size(), cl, Eavg, off, chk);
+  for (size_t c = 0; c + 1 < ofirst.size(); ++c) {
+    const int k0 = kfirst[c], nk = kfirst[c + 1] - k0, o0 = ofirst[c], no = ofirst[c + 1] - o0;
+    const dim3 g(r / 64, r / 64, nk);
+    // E'_k = Q^T (E_k Q), row-major; E_k(i, j) at i + j r
+    sy::gemm_kernel<T, double, double><<<g, 256, 0, s>>>(r, Ecol, 1, r, (int64_t)rr, o->Q, r, 1, 0, tmp, r, 1, (int64_t)rr,
+                                                         listd + k0);
+    sy::gemm_kernel<double, double, double><<<g, 256, 0, s>>>(r, o->Q, 1, r, 0, tmp, r, 1, (int64_t)rr, Ep, r, 1,
+                                                              (int64_t)rr);
+    sy::average_kernel<<<grr, 256, 0, s>>>(Ep, listd + BBFMM_NUM_OFFSETS, o->orbits + o0, no, cl, Eavg + o0 * rr, off, chk);
+  }
   sy::largest_kernel<T><<<grr, 256, 0, s>>>(Ecol, sq);
   sy::rotate_squares_kernel<<<grr, 256, 0, s>>>(o->Q, sq, 1, sq2);
   sy::rotate_squares_kernel<<<grr, 256, 0, s>>>(o->Q, sq2, 0, sq);
