@@ -14,6 +14,8 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include "smem_opt_in.h"
+
 #define BBFMM_MINLEV 2
 #define BBFMM_NUM_OFFSETS 316
 

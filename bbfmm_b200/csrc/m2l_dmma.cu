@@ -390,31 +390,19 @@ int launch_m2l_dmma(int r, const double *M, const double *Ecol, double *Lout, in
     return bbfmm_set_error(BBFMM_ERR_ARG, "box list longer than the level");
   if (boxes && nboxes == 0) return BBFMM_OK;
   if (j0 == 0 && j1 <= 64 && (ni == 32 || ni == 64)) {  // the FP64 leading block
-    static bool lattr = false;
-    if (!lattr) {
-      cudaFuncSetAttribute(dm::m2l_lead_kernel<32, 64>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                           dm::lead::Cfg<32, 64>::SMEM);
-      cudaFuncSetAttribute(dm::m2l_lead_kernel<64, 64>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                           dm::lead::Cfg<64, 64>::SMEM);
-      cudaFuncSetAttribute(dm::m2l_lead_kernel<32, 128>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                           dm::lead::Cfg<32, 128>::SMEM);
-      lattr = true;
-    }
-    if (ni == 32 && P >= 8)  // 128-target tiles (8x4x4 boxes)
+    if (ni == 32 && P >= 8) {  // 128-target tiles (8x4x4 boxes)
+      BBFMM_CUDA_OK((smem_opt_in<dm::m2l_lead_kernel<32, 128>>(dm::lead::Cfg<32, 128>::SMEM)));
       dm::m2l_lead_kernel<32, 128><<<grid / 2, 256, dm::lead::Cfg<32, 128>::SMEM, s>>>(M, Ecol, Lout, level, j1, offs);
-    else if (ni == 32)
+    } else if (ni == 32) {
+      BBFMM_CUDA_OK((smem_opt_in<dm::m2l_lead_kernel<32, 64>>(dm::lead::Cfg<32, 64>::SMEM)));
       dm::m2l_lead_kernel<32, 64><<<grid, 256, dm::lead::Cfg<32, 64>::SMEM, s>>>(M, Ecol, Lout, level, j1, offs);
-    else
+    } else {
+      BBFMM_CUDA_OK((smem_opt_in<dm::m2l_lead_kernel<64, 64>>(dm::lead::Cfg<64, 64>::SMEM)));
       dm::m2l_lead_kernel<64, 64><<<grid, 256, dm::lead::Cfg<64, 64>::SMEM, s>>>(M, Ecol, Lout, level, j1, offs);
+    }
     return bbfmm_set_cuda_error(cudaGetLastError(), "m2l_lead", __FILE__, __LINE__);
   }
-  static bool attr = false;
-  if (!attr) {
-    cudaError_t e =
-        cudaFuncSetAttribute(dm::m2l_dmma_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, dm::SMEM_BYTES);
-    if (e != cudaSuccess) return bbfmm_set_cuda_error(e, "m2l_dmma smem attribute", __FILE__, __LINE__);
-    attr = true;
-  }
+  BBFMM_CUDA_OK(smem_opt_in<dm::m2l_dmma_kernel>(dm::SMEM_BYTES));
   int ng = ngroups > 0 ? ngroups : dmma_default_groups(level, nsets);
   if (ng > DMMA_PARTS) ng = DMMA_PARTS;
   const int64_t count = 8 * (int64_t)nsets * P * P * P * r;

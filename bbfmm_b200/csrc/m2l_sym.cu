@@ -762,12 +762,7 @@ int launch_m2l_sym(const void *op, const T *M, T *Lout, int level, double *part,
   if (boxes && (nboxes < 0 || nboxes > nsets * P * P * P / 8))
     return bbfmm_set_error(BBFMM_ERR_ARG, "box list longer than the level");
   if (boxes && nboxes == 0) return BBFMM_OK;
-  static bool attr = false;
-  if (!attr) {
-    cudaError_t e = cudaFuncSetAttribute(sy::m2l_sym_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, sy::SMEM_BYTES);
-    if (e != cudaSuccess) return bbfmm_set_cuda_error(e, "m2l_sym smem attribute", __FILE__, __LINE__);
-    attr = true;
-  }
+  BBFMM_CUDA_OK(smem_opt_in<sy::m2l_sym_kernel<T>>(sy::SMEM_BYTES));
   const int64_t count = 8 * (int64_t)nsets * P * P * P * sy::R;
   const int64_t tiles = boxes ? 8 * (int64_t)((nboxes + 7) / 8) : sym_tiles(level, nsets);
   int ng = ngroups < DMMA_PARTS ? ngroups : DMMA_PARTS;

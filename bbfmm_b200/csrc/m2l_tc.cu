@@ -1307,13 +1307,7 @@ int launch_proj_down(const void *pv, const void *Asplit, const double *Lfp, int6
   int rc = map2d(&ahi, hi, rows, p->r, tc::BM);
   if (rc == BBFMM_OK) rc = map2d(&alo, lo, rows, p->r, tc::BM);
   if (rc != BBFMM_OK) return rc;
-  static bool attr = false;
-  if (!attr) {
-    cudaError_t e = cudaFuncSetAttribute(tc::proj_fused_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         tc::PD_SMEM);
-    if (e != cudaSuccess) return bbfmm_set_cuda_error(e, "proj_fused smem attribute", __FILE__, __LINE__);
-    attr = true;
-  }
+  BBFMM_CUDA_OK(smem_opt_in<tc::proj_fused_kernel<false>>(tc::PD_SMEM));
   const int64_t ntiles = ((rows + tc::BM - 1) / tc::BM) * (p->n3 / tc::BN);
   const int grid = (int)(ntiles < 148 ? ntiles : 148);
   tc::proj_fused_kernel<false><<<grid, tc::PD_THREADS, tc::PD_SMEM, s>>>(
@@ -1337,13 +1331,7 @@ int launch_proj_up(const void *pv, const void *Asplit, int64_t rows, double *M, 
   int rc = map2d(&ahi, hi, rows, p->n3, tc::BM);
   if (rc == BBFMM_OK) rc = map2d(&alo, lo, rows, p->n3, tc::BM);
   if (rc != BBFMM_OK) return rc;
-  static bool attr = false;
-  if (!attr) {
-    cudaError_t e = cudaFuncSetAttribute(tc::proj_fused_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         tc::PD_SMEM);
-    if (e != cudaSuccess) return bbfmm_set_cuda_error(e, "proj_fused smem attribute", __FILE__, __LINE__);
-    attr = true;
-  }
+  BBFMM_CUDA_OK(smem_opt_in<tc::proj_fused_kernel<true>>(tc::PD_SMEM));
   const int64_t ntiles = (rows + tc::BM - 1) / tc::BM;
   const int grid = (int)(ntiles < 148 ? ntiles : 148);
   tc::proj_fused_kernel<true><<<grid, tc::PD_THREADS, tc::PD_SMEM, s>>>(
@@ -1434,13 +1422,7 @@ int launch_m2l_tc(int r, const void *Msplit, int64_t ncell_total, int64_t cell_o
     if (rc != BBFMM_OK) return rc;
   }
   if (two) {
-    static bool attr2 = false;
-    if (!attr2) {
-      cudaError_t e =
-          cudaFuncSetAttribute(tc::m2l_tc2_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, tc::SMEM2_BYTES);
-      if (e != cudaSuccess) return bbfmm_set_cuda_error(e, "m2l_tc2 smem attribute", __FILE__, __LINE__);
-      attr2 = true;
-    }
+    BBFMM_CUDA_OK(smem_opt_in<tc::m2l_tc2_kernel>(tc::SMEM2_BYTES));
     const bool fuse = Mlead && Erow && tc_fuses_lead(ops, nprod, rank) && kfirst == 0 && ilead == 32;
     if (Lsplit && !fuse) return bbfmm_set_error(BBFMM_ERR_ARG, "split M2L output needs the fused leading block");
     const int spl = 1 << (8 - g2.lb());  // listed blocks per tile
@@ -1464,12 +1446,7 @@ int launch_m2l_tc(int r, const void *Msplit, int64_t ncell_total, int64_t cell_o
         todo, ng, part, count, Lacc, level, rank, (__nv_bfloat16 *)Lsplit, ncell, boxes, lgeom);
     return bbfmm_set_cuda_error(cudaGetLastError(), "m2l_tc2 parts", __FILE__, __LINE__);
   }
-  static bool attr = false;
-  if (!attr) {
-    cudaError_t e = cudaFuncSetAttribute(tc::m2l_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, tc::SMEM_BYTES);
-    if (e != cudaSuccess) return bbfmm_set_cuda_error(e, "m2l_tc smem attribute", __FILE__, __LINE__);
-    attr = true;
-  }
+  BBFMM_CUDA_OK(smem_opt_in<tc::m2l_tc_kernel>(tc::SMEM_BYTES));
   if (boxes) return bbfmm_set_error(BBFMM_ERR_UNSUPPORTED, "box lists are for the two-box tensor-core M2L");
   const int tiles = 8 * nsets * (P / tc::BOX_X) * (P / tc::BOX_Y) * (P / tc::BOX_Z);
   tc::m2l_tc_kernel<<<tiles, 192, tc::SMEM_BYTES, s>>>(mapAhi, mapAlo, mapBhi, mapBlo, Lacc, level, offs, kfirst,

@@ -674,12 +674,11 @@ static int grid_for(int64_t work, int per_block, int cap) {
 template <auto Kernel>
 static int resident_grid(int threads, int smem = 0) {
   static int blocks = 0;  // one cache per kernel
+  if (smem > 0) smem_opt_in<Kernel>(smem);  // dynamic plus static above 48 KB
   if (!blocks) {
     int dev = 0, sms = 148, per = 1;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    // dynamic plus static shared memory above 48 KB needs the opt-in
-    if (smem > 0) cudaFuncSetAttribute(Kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, Kernel, threads, smem);
     blocks = sms * (per > 0 ? per : 1);
   }
@@ -733,7 +732,7 @@ int launch_m2m(int n, const T *Sc, T *Sp, int level, const Tables &t, cudaStream
   if (n == 4) {
     m2m_kernel<T, 4><<<grid, 256, smem, s>>>(Sc, Sp, level, t, first, count);
   } else if (n == 8) {
-    cudaFuncSetAttribute(m2m_kernel<T, 8>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    BBFMM_CUDA_OK((smem_opt_in<m2m_kernel<T, 8>>((int)smem)));
     m2m_kernel<T, 8><<<grid, 256, smem, s>>>(Sc, Sp, level, t, first, count);
   } else return bbfmm_set_error(BBFMM_ERR_UNSUPPORTED, "order n must be 4 or 8");
   return bbfmm_set_cuda_error(cudaGetLastError(), "m2m", __FILE__, __LINE__);
@@ -752,7 +751,7 @@ int launch_l2l(int n, const T *Fp, T *Fc, int level, const Tables &t, cudaStream
   if (n == 4) {
     l2l_kernel<T, 4><<<grid, 256, smem, s>>>(Fp, Fc, level, t, first, count);
   } else if (n == 8) {
-    cudaFuncSetAttribute(l2l_kernel<T, 8>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    BBFMM_CUDA_OK((smem_opt_in<l2l_kernel<T, 8>>((int)smem)));
     l2l_kernel<T, 8><<<grid, 256, smem, s>>>(Fp, Fc, level, t, first, count);
   } else return bbfmm_set_error(BBFMM_ERR_UNSUPPORTED, "order n must be 4 or 8");
   return bbfmm_set_cuda_error(cudaGetLastError(), "l2l", __FILE__, __LINE__);

@@ -173,12 +173,7 @@ __global__ void __launch_bounds__(256) l2l_dmma_kernel(const double *__restrict_
 
 int launch_m2m_dmma(const double *Sc, double *Sp, const double *cw, int64_t first, int64_t count, cudaStream_t s) {
   if (count <= 0) return BBFMM_OK;
-  static bool attr = false;
-  if (!attr) {
-    cudaError_t e = cudaFuncSetAttribute(pd::m2m_dmma_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, pd::M2M_SMEM);
-    if (e != cudaSuccess) return bbfmm_set_cuda_error(e, "m2m_dmma smem attribute", __FILE__, __LINE__);
-    attr = true;
-  }
+  BBFMM_CUDA_OK(smem_opt_in<pd::m2m_dmma_kernel>(pd::M2M_SMEM));
   int64_t g = count < 148 * 3 * 4 ? count : 148 * 3 * 4;
   pd::m2m_dmma_kernel<<<(int)g, 256, pd::M2M_SMEM, s>>>(Sc, Sp, cw, first, count);
   return bbfmm_set_cuda_error(cudaGetLastError(), "m2m_dmma", __FILE__, __LINE__);

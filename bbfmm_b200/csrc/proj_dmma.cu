@@ -227,23 +227,10 @@ int launch_proj_narrow(int64_t M, int K, const double *A, const double *B, doubl
                        int mapmode, cudaStream_t s, int64_t row0, const int64_t *rows, void *Chi, void *Clo) {
   if (K % pj::nw::BK) return bbfmm_set_error(BBFMM_ERR_ARG, "narrow projection: K must be a multiple of 16");
   if (M <= 0) return BBFMM_OK;
-  static bool attr = false;  // 47 KB of dynamic shared memory
-  if (!attr) {
-    cudaError_t e = cudaFuncSetAttribute(pj::proj_narrow_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         pj::nw::SMEM_BYTES);
-    if (e != cudaSuccess) return bbfmm_set_cuda_error(e, "proj_narrow smem attribute", __FILE__, __LINE__);
-    attr = true;
-  }
+  BBFMM_CUDA_OK(smem_opt_in<pj::proj_narrow_kernel>(pj::nw::SMEM_BYTES));
   pj::proj_narrow_kernel<<<(unsigned)((M + pj::nw::BM - 1) / pj::nw::BM), 256, pj::nw::SMEM_BYTES, s>>>(
       M, K, A, B, C, ldc, level, mapmode, row0, rows, (__nv_bfloat16 *)Chi, (__nv_bfloat16 *)Clo);
   return bbfmm_set_cuda_error(cudaGetLastError(), "proj_narrow", __FILE__, __LINE__);
-}
-
-template <typename T, int BN>
-static int proj_dmma_attr() {  // dynamic shared memory above 48 KB needs the opt-in
-  return bbfmm_set_cuda_error(cudaFuncSetAttribute(pj::proj_dmma_kernel<T, BN>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                                   pj::smem_bytes<T>(BN)),
-                              "proj_dmma smem attribute", __FILE__, __LINE__);
 }
 
 template <typename T>
@@ -251,15 +238,16 @@ int launch_proj_dmma(int64_t M, int K, int N, const T *A, const T *B, const T *c
                      cudaStream_t s, int64_t row0, int lda, const int64_t *rows) {
   if (K % pj::BK || N % 256) return bbfmm_set_error(BBFMM_ERR_UNSUPPORTED, "projection: K % 16 and N % 256 must be 0");
   if (M <= 0) return BBFMM_OK;
-  static const int attr = proj_dmma_attr<T, 256>() | proj_dmma_attr<T, 64>();
-  if (attr) return BBFMM_ERR_CUDA;
   const unsigned mt = (unsigned)((M + pj::BM - 1) / pj::BM);
-  if ((int64_t)mt * (N / 256) < 148)
+  if ((int64_t)mt * (N / 256) < 148) {
+    BBFMM_CUDA_OK((smem_opt_in<pj::proj_dmma_kernel<T, 64>>(pj::smem_bytes<T>(64))));
     pj::proj_dmma_kernel<T, 64><<<dim3(mt, (unsigned)(N / 64)), 256, pj::smem_bytes<T>(64), s>>>(
         M, K, N, A, B, cs, scale, C, level, mapmode, row0, lda > 0 ? lda : K, rows);
-  else
+  } else {
+    BBFMM_CUDA_OK((smem_opt_in<pj::proj_dmma_kernel<T, 256>>(pj::smem_bytes<T>(256))));
     pj::proj_dmma_kernel<T, 256><<<dim3(mt, (unsigned)(N / 256)), 256, pj::smem_bytes<T>(256), s>>>(
         M, K, N, A, B, cs, scale, C, level, mapmode, row0, lda > 0 ? lda : K, rows);
+  }
   return bbfmm_set_cuda_error(cudaGetLastError(), "proj_dmma", __FILE__, __LINE__);
 }
 template int launch_proj_dmma<double>(int64_t, int, int, const double *, const double *, const double *, double, double *,
