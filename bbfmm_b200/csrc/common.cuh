@@ -108,6 +108,9 @@ struct Tables {
   const double *tkz_d, *cw_d, *kw_d;
   const float *tkz_f, *cw_f, *kw_f;
 };
+// Stable radix sort of (key, index) pairs on the device (tree.cu).
+size_t sort_scratch_ints(int N);
+int sort_pairs(int N, int bits, int *&k0, int *&i0, int *&k1, int *&i1, int *scratch, cudaStream_t s);
 // Leaves above `cap` particles of a pass's rows (device lists, launch_heavy): P2M and L2P run one
 // warp per leaf, and these as chunks of at most cap particles, one warp each.
 struct HeavyLeaves {

@@ -227,10 +227,33 @@ static int scan_exclusive(int64_t n, int *data, int *sums, cudaStream_t s) {
   return bbfmm_set_cuda_error(cudaGetLastError(), "tree scan", __FILE__, __LINE__);
 }
 
+// Ints of scratch that sort_pairs takes besides the pairs.
+static int64_t sort_blocks(int N) { return ((int64_t)N + tr::TILE - 1) / tr::TILE; }
+size_t sort_scratch_ints(int N) {
+  const int64_t nh = tr::DIGITS * sort_blocks(N);
+  return (size_t)(nh + (nh + tr::TILE - 1) / tr::TILE + 2);
+}
+
+// Stable order of the pairs (k0, i0) by the low `bits` bits of the keys, four at a time, through
+// (k1, i1); returns with the sorted pairs in k0 and i0 (the pointers swapped on odd passes).
+int sort_pairs(int N, int bits, int *&k0, int *&i0, int *&k1, int *&i1, int *scratch, cudaStream_t s) {
+  const int nb = (int)sort_blocks(N);
+  const int64_t nh = (int64_t)tr::DIGITS * nb;
+  for (int shift = 0; shift < bits; shift += 4) {
+    tr::radix_hist_kernel<<<nb, tr::THREADS, 0, s>>>(N, k0, shift, scratch);
+    const int rc = scan_exclusive(nh, scratch, scratch + nh, s);
+    if (rc != BBFMM_OK) return rc;
+    tr::radix_scatter_kernel<<<nb, tr::THREADS, 0, s>>>(N, k0, i0, shift, scratch, k1, i1);
+    BBFMM_CUDA_OK(cudaGetLastError());
+    std::swap(k0, k1);
+    std::swap(i0, i1);
+  }
+  return BBFMM_OK;
+}
+
 // perm (N = sum of counts) and leaf_start (nseg 8^maxlev + 1) on the device for the stacked
 // sets whose particles are xyz[off[j] .. off[j] + count[j]) (device, [..][3]; off and count on
-// the host). Scratch: 4 N + 16 ceil(N / 4096) + ceil(that / 4096) + 1 + 2 nseg + 1 ints,
-// allocated here.
+// the host). Scratch: 4 N + sort_scratch_ints(N) + 2 nseg + 1 ints, allocated here.
 template <typename T>
 int build_tree_device_sets(int nseg, const int *off_h, const int *count_h, const T *xyz, T L, int maxlev, int *perm,
                            int *leaf_start, cudaStream_t s) {
@@ -255,15 +278,12 @@ int build_tree_device_sets(int nseg, const int *off_h, const int *count_h, const
   T celeng = L;
   for (int l = 1; l <= maxlev; ++l) celeng *= (T)0.5;
   const T L0half = L / 2, iLm = 1 / celeng;  // the host routine's values, bit for bit
-  const int nb = (int)((N + tr::TILE - 1) / tr::TILE);
-  const int64_t nh = (int64_t)tr::DIGITS * nb;
-  const int64_t nsum = (nh + tr::TILE - 1) / tr::TILE + 1;
   int *buf = nullptr;
-  const size_t words = 4 * (size_t)N + nh + nsum + 1 + seg.size();
+  const size_t ns = sort_scratch_ints(N), words = 4 * (size_t)N + ns + seg.size();
   cudaError_t e = cudaMalloc(&buf, words * sizeof(int));
   if (e != cudaSuccess) return bbfmm_set_cuda_error(e, "tree build scratch", __FILE__, __LINE__);
   int *k0 = buf, *i0 = buf + N, *k1 = buf + 2 * (size_t)N, *i1 = buf + 3 * (size_t)N;
-  int *hist = buf + 4 * (size_t)N, *sums = hist + nh, *seg_d = sums + nsum + 1;
+  int *scratch = buf + 4 * (size_t)N, *seg_d = scratch + ns;
   int rc = BBFMM_OK;
   const int zero = 0;
   e = cudaMemcpyAsync(seg_d, seg.data(), sizeof(int) * seg.size(), cudaMemcpyHostToDevice, s);
@@ -275,15 +295,7 @@ int build_tree_device_sets(int nseg, const int *off_h, const int *count_h, const
   }
   int bits = 3 * maxlev;  // keys < nseg 8^maxlev
   while (((int64_t)1 << bits) < nleaf) ++bits;
-  for (int shift = 0; e == cudaSuccess && rc == BBFMM_OK && shift < bits; shift += 4) {
-    tr::radix_hist_kernel<<<nb, tr::THREADS, 0, s>>>(N, k0, shift, hist);
-    rc = scan_exclusive(nh, hist, sums, s);
-    if (rc != BBFMM_OK) break;
-    tr::radix_scatter_kernel<<<nb, tr::THREADS, 0, s>>>(N, k0, i0, shift, hist, k1, i1);
-    e = cudaGetLastError();
-    std::swap(k0, k1);
-    std::swap(i0, i1);
-  }
+  if (e == cudaSuccess) rc = sort_pairs(N, bits, k0, i0, k1, i1, scratch, s);
   if (e == cudaSuccess && rc == BBFMM_OK) {
     e = cudaMemcpyAsync(perm, i0, sizeof(int) * N, cudaMemcpyDeviceToDevice, s);
     if (e == cudaSuccess) {
