@@ -1408,6 +1408,7 @@ int launch_m2l_tc(int r, const void *Msplit, int64_t ncell_total, int64_t cell_o
   // with a full-width leading strip its K-steps are skipped; otherwise every K-step runs
   const int kfirst = ops->lead_rows >= r ? ops->lead / 16 : 0;
   const int ilead = ops->lead > 0 ? ops->lead_rows : 0;
+  if (kfirst * 16 >= rank) return BBFMM_OK;  // the strip holds every component: nothing to add to it
   // B boxes of the first `rank` operator rows (the effective rank); the lo box keeps its
   // split_rows rows (box maps built here when they differ from the prepared ones)
   CUtensorMap mapBhi = two ? ops->mapBhi_two : ops->mapBhi, mapBlo = ops->mapBlo;

@@ -60,3 +60,20 @@ def test_mixed_repeatable():
     b = s.solve(torch.as_tensor(q, device="cuda")).cpu().numpy()
     assert np.array_equal(a, b)
     s.close()
+
+
+@pytest.mark.parametrize("lead,rank", [(64, 64), (48, 32), (64, 96)])
+def test_leading_strip_as_wide_as_the_rank(lead, rank):
+    """A full-width FP64 strip that holds every component of a rank cut leaves the tensor cores no
+    product (their accumulators are never written): the M2L is the strip alone, and the solve that of
+    the FP64 mode at this rank."""
+    import torch
+    from bbfmm_b200 import Solver
+    x, q = uniform_inputs(20000, seed=lead + rank)
+    out = []
+    for mode, kw in (("mixed", dict(lead=lead, lead_rows=256)), ("d", {})):
+        s = Solver(8, 4, 1.0, mode=mode, rank=rank, **kw)
+        s.set_particles(x)
+        out.append(s.solve(torch.as_tensor(q, device="cuda")).cpu().numpy())
+        s.close()
+    assert rel_l2(out[0], out[1]) < 3e-7
