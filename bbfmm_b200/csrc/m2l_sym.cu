@@ -552,8 +552,7 @@ static bool sym_basis(int n, int r, const T *U, std::vector<double> &Q, int *cst
     std::vector<double> &c = cols[j];
     for (int i = 0; i < r; ++i)
       if (std::fabs(c[i]) < none) c[i] = 0.0;
-    take_out(c, cols, 0, j);
-    take_out(c, cols, 0, j);
+    take_out(c, cols, 0, j);  // once: what was cleared is below 32 roundings
     double nn = 0.0;
     for (int i = 0; i < r; ++i) nn += c[i] * c[i];
     nn = 1.0 / std::sqrt(nn);
