@@ -335,7 +335,7 @@ int Solver<T>::set_particles_global(int nsets_, int N_, const int *perm_h, const
   if (N > 0) BBFMM_CUDA_OK(cudaMemcpy(perm, perm_h, sizeof(int) * N, cudaMemcpyHostToDevice));
   BBFMM_CUDA_OK(cudaMemcpy(leaf_start, leaf_start_h, sizeof(int) * (nl + 1), cudaMemcpyHostToDevice));
   BBFMM_CUDA_OK(cudaDeviceSynchronize());
-  TRY(build_near_work());  // refuses offsets out of order
+  TRY(build_near_work(true));  // refuses offsets out of order
   TRY(build_heavy());
   if (N > 0) {
     T *xyz_d = nullptr;
@@ -395,7 +395,7 @@ int Solver<T>::set_particles_sets_device(int nsets_, const int *off_h, const int
   TRY(dalloc(&pos4, 4 * (size_t)(N > 0 ? N : 1)));
   TRY(dalloc(&phis, N > 0 ? N : 1));
   TRY(build_tree_device_sets<T>(nsets, off_h, count_h, xyz_d, (T)L, maxlev, perm, leaf_start, stream));
-  TRY(build_near_work());  // refuses offsets out of order
+  TRY(build_near_work(true));  // refuses offsets out of order
   TRY(build_heavy());
   if (N > 0) TRY((launch_gather<T, T>(N, perm, xyz_d, nullptr, pos4, stream)));
   TRY(alloc_work());
@@ -918,7 +918,7 @@ int Solver<T>::build_region_tiles() {
 // The near-field work list of the current tree for tune.p2p_threads threads per CTA (one
 // synchronisation: the item count sizes the launch).
 template <typename T>
-int Solver<T>::build_near_work() {
+int Solver<T>::build_near_work(bool positions_free) {
   if (!near_work) TRY(dalloc((unsigned char **)&near_work, near_work_bytes(N, maxlev, nsets)));
   int flag = 0;
   TRY(near_work_build(N, leaf_start, maxlev, nsets, tune.p2p_threads, near_work, stream, &near_items, &flag,
@@ -926,10 +926,12 @@ int Solver<T>::build_near_work() {
   if (flag) return bbfmm_set_error(BBFMM_ERR_ARG, "leaf offsets must rise from 0 to N without decreasing");
   near_threads = tune.p2p_threads;
   if (near_items < 2) return BBFMM_OK;
-  unsigned char *scratch = nullptr;  // longest items first
-  TRY(dalloc(&scratch, near_order_bytes(near_items)));
-  const int rc = near_order(N, leaf_start, maxlev, nsets, near_threads, near_work, near_items, scratch, stream);
-  cudaFree(scratch);  // waits for the launches
+  // longest items first, through the positions' memory while it is free, else a scratch of the call
+  unsigned char *scratch = nullptr;
+  const bool own = !positions_free || near_order_bytes(near_items) > 4 * sizeof(T) * (size_t)N;
+  if (own) TRY(dalloc(&scratch, near_order_bytes(near_items)));
+  const int rc = near_order(N, leaf_start, maxlev, nsets, near_threads, near_work, near_items, own ? (void *)scratch : pos4, stream);
+  if (own) cudaFree(scratch);  // waits for the launches
   return rc;
 }
 

@@ -372,7 +372,8 @@ struct Solver {
   int share_operators(const Solver<T> &from);  // borrow tables and operators (same n, mode, lead)
   int alloc_partials();                          // Lpart for the current tuning
   int near(T *pot, T *fld);                      // P2P (add) into sorted pot (and field)
-  int build_near_work();                         // the work list for tune.p2p_threads
+  // the work list for tune.p2p_threads; positions_free: pos4 holds nothing yet
+  int build_near_work(bool positions_free = false);
   int set_target_region(int level, const unsigned char *active_host);  // level < 0 clears
   int set_m2l_first(int level);                                        // m2l_first, then the runs
   HeavyLeaves heavy_up, heavy_down;  // of the rows that P2M and L2P run over
