@@ -35,9 +35,9 @@ METRIC = "FMM solves/s at N=4,194,304, n=8, depth 7 (1 GPU; err <= 1.2x FP64 req
 # DRAM bytes of one m2l_tc2_kernel launch per cell of its level, from an ncu capture of the
 # level-6 launch of a depth-6 solve in the form the solve makes it (split rows of the down
 # projection written; profiles/m2l_tc2_n8_level6_traffic.md); the traffic scales with the
-# number of cells (multipoles in, FP64 output and split rows out): 885.2 MB read + 299.2 MB
+# number of cells (multipoles in, FP64 output and split rows out): 927.8 MB read + 298.4 MB
 # written for 262,144 cells.
-TC_DRAM_BYTES_PER_CELL = (885159936 + 299155712) / 262144
+TC_DRAM_BYTES_PER_CELL = (927820800 + 298434560) / 262144
 SMS, MAX_SM_MHZ = 148, 1965.0
 # FP64 tensor (DMMA) peak: 128 FP64 flops per clock per SM (profiles/m2l_lead_n8_level5.md)
 DMMA_TFLOPS = SMS * 128 * MAX_SM_MHZ * 1e6 / 1e12
