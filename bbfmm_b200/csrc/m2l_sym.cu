@@ -24,11 +24,11 @@
 // read without bank conflicts, and double-buffered with one barrier a step.
 //
 // Bound by the FP64 tensor path (37 TFLOP/s measured) and the latency of a step with three warps per
-// scheduler: the path is busy about half of the time. Offsets and validity come from small shared
-// tables, because finding eight sources by integer arithmetic was the larger part of a step's
-// instructions. M2L of 262,144 particles, depth 5: unfolded FP64 57.6 ms, folded 16.1 ms, with the
-// tables 12.8 ms. Warps that multiply first and form tiles afterwards (13.8 ms) and twice the warps
-// with half the targets each (15.8 ms) were slower.
+// scheduler: the path is busy 50% of the time at level 5 (512 tiles, two groups, 10.9 ms). Offsets and
+// validity come from small shared tables, because finding eight sources by integer arithmetic was the
+// larger part of a step's instructions. M2L of 262,144 particles, depth 5: unfolded FP64 57.6 ms, folded
+// 16.1 ms, with the tables 12.8 ms. Warps that multiply first and form tiles afterwards (13.8 ms) and
+// twice the warps with half the targets each (15.8 ms) were slower.
 #include <cmath>
 #include <limits>
 #include <vector>

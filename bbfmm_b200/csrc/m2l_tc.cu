@@ -382,9 +382,9 @@ __global__ void __launch_bounds__(192, 1)
 // the CTA's half of B_hi for each chunk of 64 components, and after the first chunk's a stage with
 // A_lo and the halves of B_hi and B_lo for the TC_SPLIT_ROWS three-product outputs.
 // Bound by the tensor pipe, which the FP64 leading block's DMMA shares: at 4,194,304 particles, depth 7
-// the M2L takes 59.5 ms (67.4 ms with single CTAs of 64-byte rows and four leading-block warps); in
-// timing-only builds 46.8 ms without the leading block and 26.7 ms with it alone, at 1.4 PFLOP/s of
-// executed products under the power cap.
+// the M2L takes 57 to 59 ms with the clock (67.4 ms with single CTAs of 64-byte rows and four
+// leading-block warps); in timing-only builds 46.8 ms without the leading block and 26.7 ms with it
+// alone, at 1.4 PFLOP/s of executed products under the power cap.
 // With Mlead and Erow given (leading block i < 32, j < 16), the eight epilogue warps, idle
 // while the tensor cores run the mainloop of a CTA, compute that block in FP64 for the
 // 32 rows each later reads from tensor memory (with four warps of 64 rows, one half after the

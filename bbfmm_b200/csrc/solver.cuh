@@ -76,7 +76,7 @@ template <typename T> int launch_proj_r32(bool up, int64_t rows, const T *A, con
 template <typename T> int launch_m2l_r32(const double *Bpack, const T *M, T *Lout, int level, const int4 *offs, double *part, int64_t part_elems, cudaStream_t s, int nsets = 1, int ngroups = 0, const int4 *boxes = nullptr, int nboxes = 0);
 int launch_m2l_simt(int r, const float *M, const float *Ert, float *Lout, int level, int j0, int j1, const int4 *offs, cudaStream_t s, int nsets = 1, int ngroups = 1, float *part = nullptr, int64_t part_elems = 0, const int4 *boxes = nullptr, int nboxes = 0);
 void build_offset_table(int *out);
-constexpr int DMMA_PARTS = 21;  // most offset groups of the FP64 M2L (189 = 9 x 21)
+constexpr int DMMA_PARTS = 21;  // most offset groups of an FP64 / FP32 M2L (189 = 9 x 21)
 int launch_m2l_dmma(int r, const double *M, const double *Ecol, double *Lout, int level, int j0, int j1, int ni,
                     const int4 *offs, double *part, int64_t part_elems, cudaStream_t s, int nsets = 1,
                     int ngroups = 0, const int4 *boxes = nullptr, int nboxes = 0);
@@ -201,7 +201,7 @@ struct Tuning {
   // 0: default (the tensor-core split M2L where the mode has it, from level 4, and at levels
   // 2-3 for stacked sets), 1: FP64/SIMT M2L, 2: the tensor-core M2L wherever it tiles the level
   int m2l_kind[11] = {};
-  int m2l_groups[11] = {};  // offset groups of the FP64 DMMA M2L (0: dmma_default_groups)
+  int m2l_groups[11] = {};  // offset (or step) groups of the FP64 / FP32 M2L (0: the form's default)
   int p2p_threads = 128;    // threads per block of the near-field kernel
 };
 
