@@ -331,17 +331,12 @@ __global__ void __launch_bounds__(256) m2l_lead_kernel(const double *__restrict_
 // Lout[e] = sum_g part[g][e], in a fixed order, in FP64 whatever T is.
 template <typename T>
 __global__ void sum_parts_kernel(int64_t count, int ng, const double *__restrict__ part, T *__restrict__ Lout) {
-  const int64_t e = 2 * (blockIdx.x * (int64_t)blockDim.x + threadIdx.x);  // pairs: count is even
+  const int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   if (e >= count) return;
-  double a = 0.0, b = 0.0;
+  double a = 0.0;
 #pragma unroll 4
-  for (int g = 0; g < ng; ++g) {
-    const double2 v = *reinterpret_cast<const double2 *>(part + g * count + e);
-    a += v.x;
-    b += v.y;
-  }
+  for (int g = 0; g < ng; ++g) a += part[g * count + e];
   Lout[e] = (T)a;
-  Lout[e + 1] = (T)b;
 }
 
 }  // namespace dm
@@ -349,7 +344,7 @@ __global__ void sum_parts_kernel(int64_t count, int ng, const double *__restrict
 // The partial sums of a whole level's offset (or step) groups added up: `count` values a group.
 template <typename T>
 int launch_sum_parts(int64_t count, int ng, const double *part, T *Lout, cudaStream_t s) {
-  dm::sum_parts_kernel<T><<<(unsigned)((count + 511) / 512), 256, 0, s>>>(count, ng, part, Lout);
+  dm::sum_parts_kernel<T><<<(unsigned)((count + 255) / 256), 256, 0, s>>>(count, ng, part, Lout);
   return bbfmm_set_cuda_error(cudaGetLastError(), "M2L parts", __FILE__, __LINE__);
 }
 template int launch_sum_parts<double>(int64_t, int, const double *, double *, cudaStream_t);

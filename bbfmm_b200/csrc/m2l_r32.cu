@@ -47,11 +47,12 @@ __device__ __forceinline__ double get8(const Eight<float> &e, int k) {
 }
 
 // Grid: x = 8 classes x tiles of 16 blocks (class fastest: the resident CTAs share one source
-// region), y = groups of the 189 offsets; several write their sums to slices of part, in FP64 whatever T is.
-template <typename T>
+// region), y = groups of the 189 offsets, each with its own slice of Lout (TO: double with several
+// groups, whatever T is, else T).
+template <typename T, typename TO>
 __global__ void __launch_bounds__(THREADS, 2)
-    m2l_r32_kernel(const T *__restrict__ M, const double *__restrict__ Bpack, T *__restrict__ Lout,
-                   double *__restrict__ part, int level, const int4 *__restrict__ offs, const int4 *__restrict__ boxes, int nblocks, int nsets) {
+    m2l_r32_kernel(const T *__restrict__ M, const double *__restrict__ Bpack, TO *__restrict__ Lout, int level,
+                   const int4 *__restrict__ offs, const int4 *__restrict__ boxes, int nblocks, int nsets) {
   __shared__ __align__(16) double Bs[STAGES][B_DOUBLES];
   const int P = 1 << (level - 1), P3 = P * P * P;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -84,7 +85,7 @@ __global__ void __launch_bounds__(THREADS, 2)
     sb[m] = o.x * 8 * P3;
   }
   const int o0 = (189 * blockIdx.y) / gridDim.y, o1 = (189 * (blockIdx.y + 1)) / gridDim.y;
-  part += (int64_t)blockIdx.y * 8 * nsets * P3 * R;
+  Lout += (int64_t)blockIdx.y * 8 * nsets * P3 * R;
 
   auto load_b = [&](int o) {
     if (o < o1) {
@@ -144,16 +145,11 @@ __global__ void __launch_bounds__(THREADS, 2)
 #pragma unroll
   for (int m = 0; m < 2; ++m) {
     if (!live[m]) continue;
-    const int64_t at = (int64_t)(sb[m] + c * P3 + (z0[m] * P + y0[m]) * P + x0[m]) * R + 2 * (lane & 3);
+    TO *dst = Lout + (int64_t)(sb[m] + c * P3 + (z0[m] * P + y0[m]) * P + x0[m]) * R + 2 * (lane & 3);
 #pragma unroll
     for (int f = 0; f < 4; ++f) {
-      if (gridDim.y > 1) {
-        part[at + 8 * f] = acc[m][f][0];
-        part[at + 8 * f + 1] = acc[m][f][1];
-      } else {
-        Lout[at + 8 * f] = (T)acc[m][f][0];
-        Lout[at + 8 * f + 1] = (T)acc[m][f][1];
-      }
+      dst[8 * f] = (TO)acc[m][f][0];
+      dst[8 * f + 1] = (TO)acc[m][f][1];
     }
   }
 }
@@ -297,8 +293,11 @@ int launch_m2l_r32(const double *Bpack, const T *M, T *Lout, int level, const in
   if (ng < 1) ng = 1;
   const int64_t nb = boxes ? nboxes : all;
   const int64_t tiles = 8 * ((nb + r32::BLOCKS - 1) / r32::BLOCKS);
-  r32::m2l_r32_kernel<T><<<dim3((unsigned)tiles, ng), r32::THREADS, 0, s>>>(M, Bpack, Lout, part, level, offs, boxes,
-                                                                         (int)nb, nsets);
+  const dim3 grid((unsigned)tiles, ng);
+  if (ng > 1)
+    r32::m2l_r32_kernel<T, double><<<grid, r32::THREADS, 0, s>>>(M, Bpack, part, level, offs, boxes, (int)nb, nsets);
+  else
+    r32::m2l_r32_kernel<T, T><<<grid, r32::THREADS, 0, s>>>(M, Bpack, Lout, level, offs, boxes, (int)nb, nsets);
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess || ng == 1) return bbfmm_set_cuda_error(e, "m2l_r32", __FILE__, __LINE__);
   return launch_sum_parts<T>(count, ng, part, Lout, s);

@@ -70,11 +70,11 @@ __device__ __forceinline__ void dmma(double &d0, double &d1, double a, double b)
                : "d"(a), "d"(b));
 }
 
-template <typename T>
+// TO: double where several step groups write their sums to slices, whatever T is, else T.
+template <typename T, typename TO>
 __global__ void __launch_bounds__(THREADS, 1)
     m2l_sym_kernel(const T *__restrict__ M, const double *__restrict__ Bsteps, const Step *__restrict__ steps, int nsteps,
-                   const int *__restrict__ orbits, T *__restrict__ Lout, double *__restrict__ part, int level,
-                   const __grid_constant__ Classes cl,
+                   const int *__restrict__ orbits, TO *__restrict__ Lout, int level, const __grid_constant__ Classes cl,
                    const int4 *__restrict__ boxes, int nboxes, int nsets) {
   extern __shared__ __align__(16) double smem[];
   double *const Bs = smem + 2 * A_DOUBLES;  // A tiles of two steps, then B tiles of two
@@ -127,7 +127,7 @@ __global__ void __launch_bounds__(THREADS, 1)
   __syncthreads();
   const int og = blockIdx.y, ng = gridDim.y;
   const int s0 = (int)((int64_t)nsteps * og / ng), s1 = (int)((int64_t)nsteps * (og + 1) / ng);
-  part += (int64_t)og * 8 * nsets * P3 * R;  // used with several groups: FP64 whatever T is
+  Lout += (int64_t)og * 8 * nsets * P3 * R;
 
   // the two elements of the A tiles this thread forms: component tid % 12 of targets tid / 12 and
   // 32 + tid / 12 (a warp's loads are runs of 12 consecutive components); target t is cell t & 7 of
@@ -284,14 +284,9 @@ __global__ void __launch_bounds__(THREADS, 1)
     for (int f = 0; f < FW; ++f) {
       const int c0 = cl.cstart[fc[f]], n = cl.cstart[fc[f] + 1] - c0;
       const int col = cl.fcol[warp * FW + f] + 2 * (lane & 3);
-      const int64_t at = cell * R + c0 + col;
-      if (ng > 1) {
-        if (col < n) part[at] = acc[m][f][0];
-        if (col + 1 < n) part[at + 1] = acc[m][f][1];
-      } else {
-        if (col < n) Lout[at] = (T)acc[m][f][0];
-        if (col + 1 < n) Lout[at + 1] = (T)acc[m][f][1];
-      }
+      TO *dst = Lout + cell * R + c0 + col;
+      if (col < n) dst[0] = (TO)acc[m][f][0];
+      if (col + 1 < n) dst[1] = (TO)acc[m][f][1];
     }
   }
 }
@@ -761,15 +756,22 @@ int launch_m2l_sym(const void *op, const T *M, T *Lout, int level, double *part,
   if (boxes && (nboxes < 0 || nboxes > nsets * P * P * P / 8))
     return bbfmm_set_error(BBFMM_ERR_ARG, "box list longer than the level");
   if (boxes && nboxes == 0) return BBFMM_OK;
-  BBFMM_CUDA_OK(smem_opt_in<sy::m2l_sym_kernel<T>>(sy::SMEM_BYTES));
   const int64_t count = 8 * (int64_t)nsets * P * P * P * sy::R;
   const int64_t tiles = boxes ? 8 * (int64_t)((nboxes + 7) / 8) : sym_tiles(level, nsets);
   int ng = ngroups < DMMA_PARTS ? ngroups : DMMA_PARTS;
   if (!part) ng = 1;
   else if (ng > 1 && (int64_t)ng * count > part_elems) ng = (int)(part_elems / count);
   if (ng < 1) ng = 1;
-  sy::m2l_sym_kernel<T><<<dim3((unsigned)tiles, ng), sy::THREADS, sy::SMEM_BYTES, s>>>(
-      M, o->Bsteps, o->steps, o->nsteps, o->orbits, Lout, part, level, o->cl, boxes, nboxes, nsets);
+  const dim3 grid((unsigned)tiles, ng);
+  if (ng > 1) {
+    BBFMM_CUDA_OK((smem_opt_in<sy::m2l_sym_kernel<T, double>>(sy::SMEM_BYTES)));
+    sy::m2l_sym_kernel<T, double><<<grid, sy::THREADS, sy::SMEM_BYTES, s>>>(M, o->Bsteps, o->steps, o->nsteps, o->orbits, part,
+                                                                          level, o->cl, boxes, nboxes, nsets);
+  } else {
+    BBFMM_CUDA_OK((smem_opt_in<sy::m2l_sym_kernel<T, T>>(sy::SMEM_BYTES)));
+    sy::m2l_sym_kernel<T, T><<<grid, sy::THREADS, sy::SMEM_BYTES, s>>>(M, o->Bsteps, o->steps, o->nsteps, o->orbits, Lout,
+                                                                     level, o->cl, boxes, nboxes, nsets);
+  }
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess || ng == 1) return bbfmm_set_cuda_error(e, "m2l_sym", __FILE__, __LINE__);
   if (!boxes) return launch_sum_parts<T>(count, ng, part, Lout, s);
